@@ -55,25 +55,11 @@ using namespace vgbd;
 #ifndef VGB_BATCH_LEAN_OOL
 #define VGB_BATCH_LEAN_OOL 1
 #endif
-// 1: k_batch_direct traces a tile's camera rays and shadow rays as warp packets (binary layout).
-// Off: on the 256-frame trajectory the packets took 1.45 s against 1.17 s for one traversal per
-// lane (same results; 64 registers each).
-#ifndef VGB_BATCH_PACKET
-#define VGB_BATCH_PACKET 0
-#endif
 // >= 0: the shared-memory carveout (percent of the maximum) requested for the traversal and
 // shading kernels, which use no shared memory; the rest of the SM's 256 KB is L1.  -1 leaves the
 // driver's choice, which measured the same as 0 on the path-traced frame (100 lost 12 %).
 #ifndef VGB_L1_CARVEOUT
 #define VGB_L1_CARVEOUT -1
-#endif
-// > 0: before each continuation bounce, k_bin_rays sorts the live-path queue into this many
-// bins by the rays' vertical direction component, and k_trace takes its items bin by bin (the
-// hit records keep the queue order, so k_shade reads them unchanged).  Up to 8.  Off: on the
-// path-traced frame 4 bins cut the closest-hit time by under 2 % and the binning pass cost more
-// (3469 and 3485 Mrays/s with 4 and 8 bins against 3639).
-#ifndef VGB_TRACE_BINS
-#define VGB_TRACE_BINS 0
 #endif
 #ifndef VGB_SHADOW_MINB
 #define VGB_SHADOW_MINB 5
@@ -163,6 +149,7 @@ namespace {
 // ------------------------------------------------------------------ device data
 struct DevScene {
     const uint4* nodes;    // binary (4 words per node) or compressed 8-wide (5 words per node)
+    const uint4* wide;     // wide nodes of the binary layout (8 words per node)
     const float4* tris;
     const uint32_t* idx;   // 3 per triangle, caller order
     const float4* vpos;    // xyz
@@ -180,6 +167,10 @@ struct DevScene {
     uint32_t tex_mono;                // every texel has the same value in all bands
     float albedo_value[VGB_MAX_BANDS];
 };
+
+// The node array the traversal of layout L reads.
+template <int L>
+__device__ __forceinline__ const uint4* bvh_nodes(const DevScene& s) { return L == 4 ? s.wide : s.nodes; }
 
 struct DevState {
     // per-pixel path state
@@ -205,7 +196,6 @@ struct DevState {
     uint32_t* sq_slot[VGB_MAX_LIGHTS];
     float* sq_con[VGB_MAX_LIGHTS];   // [B][P]
     float4* hit;         // [P] closest-hit record per queue item: (t, id bits, w(v1), w(v2))
-    uint32_t* binq;      // [VGB_TRACE_BINS][P] queue items binned by ray direction (null: off)
     // adaptive sampling: per pixel the sums of the path-radiance magnitude and of its square,
     // and the sample index at which the pixel stopped (0 while it samples on)
     float* as1;
@@ -221,8 +211,8 @@ struct DevState {
 // the error word and the batch kernels' work counter.
 enum {
     C_PQ0 = 0, C_PQ1 = 1, C_SQ = 2, C_FTRACE = 2 + VGB_MAX_LIGHTS, C_FSHADOW = 3 + VGB_MAX_LIGHTS,
-    C_ERR = 3 + 2 * VGB_MAX_LIGHTS, C_BATCH = 4 + 2 * VGB_MAX_LIGHTS, C_BIN = 5 + 2 * VGB_MAX_LIGHTS,
-    C_COUNT = C_BIN + 8
+    C_ERR = 3 + 2 * VGB_MAX_LIGHTS, C_BATCH = 4 + 2 * VGB_MAX_LIGHTS,
+    C_COUNT
 };
 // counters cleared at the start of every bounce: the shadow queues and the persistent item counters
 constexpr int kBounceResetWords = 1 + 2 * VGB_MAX_LIGHTS;
@@ -766,27 +756,15 @@ __global__ void __launch_bounds__(VGB_TRACE_BLOCK, (L == 8 ? VGB_TRACE8_MINB : V
             if (!camera_ray(fp, item, sample, slot, ro, rd)) continue;
             if (fp.opt.adaptive_sampling && sample != 0 && st.anum[slot]) continue;  // pixel has stopped
         }
-        uint32_t qi = item;  // the queue position this ray's hit record goes to
         if (!B0) {
-#if VGB_TRACE_BINS > 0
-            if (st.binq) {
-                uint32_t first = 0;
-#pragma unroll
-                for (int b = 0; b < VGB_TRACE_BINS; ++b) {
-                    const uint32_t c = st.counters[C_BIN + b];
-                    if (item >= first && item - first < c) qi = st.binq[b * P + (item - first)];
-                    first += c;
-                }
-            }
-#endif
-            slot = in_queue[qi];
+            slot = in_queue[item];
             ro = F3{st.org[slot], st.org[P + slot], st.org[2 * P + slot]};
             rd = F3{st.dir[slot], st.dir[P + slot], st.dir[2 * P + slot]};
         }
         HitOut h;
         h.U = h.V = h.W = 0.f; h.det = 1.f;
         const WRay wr = make_wray(ro, rd);
-        traverse_any_layout<L, false, COUNT>(s.nodes, s.tris, wr, 0.f, h, err, cnt, s.iter_cap);
+        traverse_any_layout<L, false, COUNT>(bvh_nodes<L>(s), s.tris, wr, 0.f, h, err, cnt, s.iter_cap);
         nclosest++;
         float w0 = 0.f, w1 = 0.f;
         if (h.id != VGB_NO_HIT) {
@@ -794,7 +772,7 @@ __global__ void __launch_bounds__(VGB_TRACE_BLOCK, (L == 8 ? VGB_TRACE8_MINB : V
             w0 = h.V * rcp;
             w1 = h.W * rcp;
         }
-        st.hit[qi] = make_float4(h.t, __uint_as_float(h.id), w0, w1);
+        st.hit[item] = make_float4(h.t, __uint_as_float(h.id), w0, w1);
     }
     if (err) atomicOr(&st.counters[C_ERR], err);
     warp_reduce_add(&st.stats[2], nclosest);
@@ -806,40 +784,11 @@ __global__ void __launch_bounds__(VGB_TRACE_BLOCK, (L == 8 ? VGB_TRACE8_MINB : V
     }
 }
 
-#if VGB_TRACE_BINS > 0
-// The live-path queue `in_q` binned by the vertical component of each ray's direction (bins of
-// equal width over [-1, 1]), so that a warp of k_trace takes rays of similar traversal length:
-// on terrain the near-horizontal rays cross far more of the tree than the steep ones.  Each bin
-// lists queue positions; the appends are warp-aggregated per bin.  Sum of the bins = the queue.
-__global__ void __launch_bounds__(256) k_bin_rays(DevState st, uint32_t in_q) {
-    const size_t P = st.P;
-    const uint32_t n = st.counters[in_q];
-    const uint32_t* in_queue = st.pq[in_q];
-    const int lane = threadIdx.x & 31;
-    const uint32_t stride = gridDim.x * blockDim.x;
-    for (uint32_t base = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); base < n; base += stride) {
-        const uint32_t item = base + lane;
-        const bool valid = item < n;
-        const unsigned vmask = __ballot_sync(0xffffffffu, valid);
-        if (!valid) continue;
-        const float dz = st.dir[2 * P + in_queue[item]];
-        const float x = fminf(fmaxf((dz + 1.0f) * (0.5f * VGB_TRACE_BINS), 0.0f), (float)(VGB_TRACE_BINS - 1));
-        const uint32_t b = (uint32_t)x;
-        const unsigned grp = __match_any_sync(vmask, b);
-        const int leader = __ffs(grp) - 1;
-        uint32_t pos = 0;
-        if (lane == leader) pos = atomicAdd(&st.counters[C_BIN + b], (uint32_t)__popc(grp));
-        pos = __shfl_sync(grp, pos, leader) + (uint32_t)__popc(grp & ((1u << lane) - 1u));
-        st.binq[b * P + pos] = item;
-    }
-}
-#endif
-
-// ------------------------------------------------------------------ persistent traversal (binary layout)
-// k_trace_p / k_shadow_p replace the grid-stride loops of k_trace / k_shadow for the binary BVH.
+// ------------------------------------------------------------------ persistent traversal (wide nodes)
+// k_trace_p / k_shadow_p replace the grid-stride loops of k_trace / k_shadow for the wide BVH.
 // They launch one wave of resident blocks; each warp claims chunks of kWarpChunk consecutive queue
 // items from a launch-wide counter and hands them to its lanes as lanes become free, and every
-// lane advances its ray by at most `budget` inner-node visits between hand-outs (traverse_resume).
+// lane advances its ray by at most `budget` inner-node visits between hand-outs (traverse4 with RESUME).
 // A lane whose ray finished thus starts the next ray while its neighbours are still traversing,
 // instead of idling until the warp's slowest ray is done, which is what left bounce-1 rays at
 // half-empty warps.  Rays, their order within a warp and every test are those of the grid-stride
@@ -890,7 +839,7 @@ __global__ void __launch_bounds__(256, VGB_TRACEP_MINB) k_trace_p(const DevScene
     const size_t P = st.P;
     const uint32_t n_items = (bounce == 0) ? n_items_bounce0 : st.counters[in_q];
     const uint32_t* in_queue = st.pq[in_q];
-    const float4* nodes = reinterpret_cast<const float4*>(s.nodes);
+    const uint4* nodes = s.wide;
     const int lane = threadIdx.x & 31;
     uint32_t err = 0, nclosest = 0;
     Counters cnt{0, 0};
@@ -898,10 +847,10 @@ __global__ void __launch_bounds__(256, VGB_TRACEP_MINB) k_trace_p(const DevScene
     bool live = false;
     uint32_t item = 0;
     WRay wr;
-    SlabRay q;
+    WideRay q;
     TravState ts;
     HitOut h;
-    int stack[kStackSize];
+    int stack[kStackWide];
     while (true) {
         const unsigned idle = __ballot_sync(kFullMask, !live);
         if ((wi.left || !wi.done) && (__popc(idle) >= refill || idle == kFullMask)) {
@@ -921,8 +870,8 @@ __global__ void __launch_bounds__(256, VGB_TRACEP_MINB) k_trace_p(const DevScene
                 if (ok) {
                     item = it;
                     wr = make_wray(ro, rd);
-                    q = make_slab(wr);
-                    ts = trav_start(0.f, false, h);
+                    q = make_wide(wr);
+                    ts = trav_start(0.f, false, h, stack);
                     live = true;
                     nclosest++;
                 }
@@ -932,7 +881,7 @@ __global__ void __launch_bounds__(256, VGB_TRACEP_MINB) k_trace_p(const DevScene
             if (wi.done && wi.left == 0) break;
             continue;
         }
-        if (live && traverse_resume<COUNT>(nodes, s.tris, wr, q, 0.f, false, stack, ts, h, err, cnt, s.iter_cap, budget)) {
+        if (live && traverse4<COUNT, true>(nodes, s.tris, wr, q, 0.f, false, stack, ts, h, err, cnt, s.iter_cap, budget)) {
             float w0 = 0.f, w1 = 0.f;
             if (h.id != VGB_NO_HIT) {
                 const float rcp = 1.0f / h.det;
@@ -958,7 +907,7 @@ __global__ void __launch_bounds__(256, VGB_SHADOWP_MINB) k_shadow_p(const DevSce
                                                    int budget, uint32_t refill) {
     const size_t P = st.P;
     const uint32_t n = st.counters[C_SQ + light];
-    const float4* nodes = reinterpret_cast<const float4*>(s.nodes);
+    const uint4* nodes = s.wide;
     const int lane = threadIdx.x & 31;
     uint32_t err = 0, nsh = 0;
     Counters cnt{0, 0};
@@ -967,10 +916,10 @@ __global__ void __launch_bounds__(256, VGB_SHADOWP_MINB) k_shadow_p(const DevSce
     uint32_t item = 0;
     float tmax = 0.f;
     WRay wr;
-    SlabRay q;
+    WideRay q;
     TravState ts;
     HitOut h;
-    int stack[kStackSize];
+    int stack[kStackWide];
     while (true) {
         const unsigned idle = __ballot_sync(kFullMask, !live);
         if ((wi.left || !wi.done) && (__popc(idle) >= refill || idle == kFullMask)) {
@@ -981,8 +930,8 @@ __global__ void __launch_bounds__(256, VGB_SHADOWP_MINB) k_shadow_p(const DevSce
                 const F3 d{st.sq_dir[light][it], st.sq_dir[light][P + it], st.sq_dir[light][2 * P + it]};
                 tmax = st.sq_tmax[light][it];
                 wr = make_wray(o, d);
-                q = make_slab(wr);
-                ts = trav_start(tmax, true, h);
+                q = make_wide(wr);
+                ts = trav_start(tmax, true, h, stack);
                 live = true;
                 nsh++;
             }
@@ -991,7 +940,7 @@ __global__ void __launch_bounds__(256, VGB_SHADOWP_MINB) k_shadow_p(const DevSce
             if (wi.done && wi.left == 0) break;
             continue;
         }
-        if (live && traverse_resume<COUNT>(nodes, s.tris, wr, q, tmax, true, stack, ts, h, err, cnt, s.iter_cap, budget)) {
+        if (live && traverse4<COUNT, true>(nodes, s.tris, wr, q, tmax, true, stack, ts, h, err, cnt, s.iter_cap, budget)) {
             if (h.id == VGB_NO_HIT) {
                 const uint32_t slot = st.sq_slot[light][item];
 #pragma unroll
@@ -1239,7 +1188,7 @@ __global__ void __launch_bounds__(VGB_SHADOW_BLOCK, (L == 8 ? VGB_SHADOW8_MINB :
         const float tmax = st.sq_tmax[light][i];
         WRay wr = make_wray(o, d);
         HitOut h;
-        traverse_any_layout<L, true, COUNT>(s.nodes, s.tris, wr, tmax, h, err, cnt, s.iter_cap);
+        traverse_any_layout<L, true, COUNT>(bvh_nodes<L>(s), s.tris, wr, tmax, h, err, cnt, s.iter_cap);
         nsh++;
         if (h.id == VGB_NO_HIT) {
             const uint32_t slot = st.sq_slot[light][i];
@@ -1401,7 +1350,7 @@ __global__ void __launch_bounds__(VGB_RAYS_BLOCK) k_trace_batch(const DevScene s
         WRay wr = make_wray(o, d);
         HitOut h;
         h.U = h.V = h.W = 0.f; h.det = 1.f;
-        traverse_any_layout<L, ANY, COUNT>(s.nodes, s.tris, wr, tmax ? tmax[i] : __int_as_float(0x7f800000), h, err, cnt, s.iter_cap);
+        traverse_any_layout<L, ANY, COUNT>(bvh_nodes<L>(s), s.tris, wr, tmax ? tmax[i] : __int_as_float(0x7f800000), h, err, cnt, s.iter_cap);
         tri[i] = h.id;
         if (tout) tout[i] = h.t;
         if (bary) {
@@ -1452,6 +1401,8 @@ struct vgb_context {
     std::vector<uint32_t> h_idx;
     // BVH
     uint4* d_nodes = nullptr;
+    uint4* d_wide = nullptr;        // binary layout: its wide nodes, which the traversal reads
+    uint32_t nwide = 0;
     float4* d_tris = nullptr;
     uint32_t nnodes = 0;
     uint32_t bvh_layout = 2;
@@ -1548,8 +1499,8 @@ void free_scene(vgb_context* ctx) {
     ctx->nmotion = 0;
 }
 void free_bvh(vgb_context* ctx) {
-    dfree(ctx->d_nodes); dfree(ctx->d_tris); dfree(ctx->d_parent); dfree(ctx->d_refit);
-    ctx->d_nodes = nullptr; ctx->d_tris = nullptr; ctx->d_parent = nullptr; ctx->d_refit = nullptr;
+    dfree(ctx->d_nodes); dfree(ctx->d_wide); dfree(ctx->d_tris); dfree(ctx->d_parent); dfree(ctx->d_refit);
+    ctx->d_nodes = ctx->d_wide = nullptr; ctx->nwide = 0; ctx->d_tris = nullptr; ctx->d_parent = nullptr; ctx->d_refit = nullptr;
     ctx->bvh_ready = false; ctx->nnodes = 0;
 }
 void free_scratch(vgb_context* ctx) {
@@ -1610,8 +1561,6 @@ vgb_status ensure_scratch(vgb_context* ctx, size_t P, size_t n_items, uint32_t B
     AL(st.pq[0], P * u); AL(st.pq[1], P * u);
     AL(st.hit, n_items * sizeof(float4));
     AL(st.as1, P * f); AL(st.as2, P * f); AL(st.anum, P * u);
-    st.binq = nullptr;
-    if (VGB_TRACE_BINS > 0) AL(st.binq, VGB_TRACE_BINS * P * u);
     for (uint32_t l = 0; l < VGB_MAX_LIGHTS; ++l) {
         if (l < L) {
             AL(st.sq_org[l], 3 * P * f); AL(st.sq_dir[l], 3 * P * f); AL(st.sq_tmax[l], P * f);
@@ -1630,7 +1579,7 @@ vgb_status ensure_scratch(vgb_context* ctx, size_t P, size_t n_items, uint32_t B
 
 DevScene dev_scene(const vgb_context* ctx) {
     DevScene s;
-    s.nodes = ctx->d_nodes; s.tris = ctx->d_tris; s.idx = ctx->d_idx; s.vpos = ctx->d_vpos; s.vnrm = ctx->d_vnrm;
+    s.nodes = ctx->d_nodes; s.wide = ctx->d_wide; s.tris = ctx->d_tris; s.idx = ctx->d_idx; s.vpos = ctx->d_vpos; s.vnrm = ctx->d_vnrm;
     s.vuv = ctx->d_vuv; s.valb = ctx->d_valb; s.tex = ctx->d_tex; s.tw = ctx->tw; s.th = ctx->th;
     s.nmap = ctx->d_nmap; s.nw = ctx->nw; s.nh = ctx->nh;
     s.motion = ctx->d_motion; s.nmotion = ctx->nmotion;
@@ -1704,8 +1653,8 @@ void launch_render(vgb_context* ctx, const FrameParams& fp, const FilmOut& film,
     const int gs = grid_for(ctx, n0, VGB_SHADE_GRID * 256 / VGB_SHADE_BLOCK, VGB_SHADE_BLOCK);
     const int go = grid_for(ctx, n0, VGB_SHADOW_GRID * 256 / VGB_SHADOW_BLOCK, VGB_SHADOW_BLOCK);
     const int gp = grid_for(ctx, (size_t)fp.cam.width * fp.cam.height, VGB_END_GRID);
-    // persistent traversal (binary layout): one resident wave, lanes refilled from the queue
-    const bool persist = L == 2 && ctx->trav_persistent;
+    // persistent traversal (wide nodes): one resident wave, lanes refilled from the queue
+    const bool persist = L == 4 && ctx->trav_persistent;
     const int gtp = persist ? resident_grid(ctx, k_trace_p<COUNT>) : 0;
     const int gop = persist ? resident_grid(ctx, k_shadow_p<NB, COUNT>) : 0;
     const int budget = (int)ctx->trav_budget;
@@ -1727,13 +1676,6 @@ void launch_render(vgb_context* ctx, const FrameParams& fp, const FilmOut& film,
             // reset the output path queue, the shadow queues and the persistent item counters
             cudaMemsetAsync(&st.counters[(q ^ 1u)], 0, sizeof(uint32_t), ctx->stream);
             cudaMemsetAsync(&st.counters[C_SQ], 0, sizeof(uint32_t) * kBounceResetWords, ctx->stream);
-#if VGB_TRACE_BINS > 0
-            if (b != 0 && st.binq && !persist) {
-                cudaMemsetAsync(&st.counters[C_BIN], 0, sizeof(uint32_t) * VGB_TRACE_BINS, ctx->stream);
-                k_bin_rays<<<gs, 256, 0, ctx->stream>>>(st, q);
-                launches++;
-            }
-#endif
             {
                 Prof p(ctx, 0, prof);
                 if (persist) k_trace_p<COUNT><<<gtp, 256, 0, ctx->stream>>>(s, st, fp, b, smp, q, n0, budget, refill);
@@ -1776,7 +1718,7 @@ template <bool COUNT>
 void dispatch_render(vgb_context* ctx, const FrameParams& fp, const FilmOut& film, const DevState& st, bool prof,
                      uint32_t& launches) {
     if (ctx->bvh_layout == 8) dispatch_render_l<8, COUNT>(ctx, fp, film, st, prof, launches);
-    else dispatch_render_l<2, COUNT>(ctx, fp, film, st, prof, launches);
+    else dispatch_render_l<4, COUNT>(ctx, fp, film, st, prof, launches);
 }
 
 }  // namespace
@@ -2197,6 +2139,26 @@ VGB_API vgb_status vgb_scene_upload(vgb_context* ctx, const float* pos, uint32_t
     return vgb::status_of_exception(ctx ? &ctx->err : nullptr);
 }
 
+// The wide nodes of the context's binary BVH.
+static vgb_status build_wide(vgb_context* ctx) {
+    uint32_t* work = nullptr;
+    vgb_status s = dalloc(ctx, &work, vgb::wide_work_words(ctx->nnodes) * sizeof(uint32_t));
+    if (s != VGB_OK) return s;
+    const uint32_t* nodes = reinterpret_cast<const uint32_t*>(ctx->d_nodes);
+    cudaError_t e = (cudaError_t)vgb::launch_wide_fold(ctx->stream, ctx->num_sms, nodes, ctx->nnodes, work, &ctx->nwide);
+    if (e == cudaSuccess) s = dalloc(ctx, &ctx->d_wide, (size_t)ctx->nwide * 128);
+    if (e == cudaSuccess && s == VGB_OK)
+        e = (cudaError_t)vgb::launch_wide_emit(ctx->stream, ctx->num_sms, nodes, ctx->nnodes, work, ctx->nwide, ctx->d_wide);
+    const cudaError_t e2 = cudaStreamSynchronize(ctx->stream);
+    dfree(work);
+    if (s != VGB_OK) return s;
+    CK(e);
+    CK(e2);
+    ctx->stats.bvh_nodes = ctx->nwide;
+    ctx->stats.bvh_node_bytes = 128;
+    return VGB_OK;
+}
+
 VGB_API vgb_status vgb_bvh_build(vgb_context* ctx, const vgb_bvh_options* opts) try {
     if (!ctx) return VGB_ERR_INVALID_ARGUMENT;
     if (ctx->ntris == 0) return fail(ctx, VGB_ERR_NOT_READY, "bvh_build: no scene uploaded");
@@ -2236,9 +2198,8 @@ VGB_API vgb_status vgb_bvh_build(vgb_context* ctx, const vgb_bvh_options* opts) 
         ctx->nnodes = nn;
         ctx->bvh_layout = 2;
         ctx->bvh_leaf = leaf; ctx->bvh_threads = 0;
+        if ((s = build_wide(ctx)) != VGB_OK) return s;
         ctx->bvh_ready = true;
-        ctx->stats.bvh_nodes = nn;
-        ctx->stats.bvh_node_bytes = 64;
         ctx->stats.tri_record_bytes = 48;
         return VGB_OK;
     }
@@ -2274,9 +2235,10 @@ VGB_API vgb_status vgb_bvh_build(vgb_context* ctx, const vgb_bvh_options* opts) 
     ctx->nnodes = bvh.num_nodes;
     ctx->bvh_layout = layout;
     ctx->bvh_leaf = leaf; ctx->bvh_threads = threads;
-    ctx->bvh_ready = true;
     ctx->stats.bvh_nodes = bvh.num_nodes;
-    ctx->stats.bvh_node_bytes = layout == 8 ? 80 : 64;
+    ctx->stats.bvh_node_bytes = 80;
+    if (layout == 2 && (s = build_wide(ctx)) != VGB_OK) return s;
+    ctx->bvh_ready = true;
     ctx->stats.tri_record_bytes = 48;
     return VGB_OK;
 } catch (...) {
@@ -2501,6 +2463,8 @@ VGB_API vgb_status vgb_scene_update_positions(vgb_context* ctx, const float* pos
                                              ctx->d_refit);
             if (rc == -2) return fail(ctx, VGB_ERR_CUDA, "scene_update_positions: refit walk exceeded the tree depth");
             CK((cudaError_t)rc);
+            CK((cudaError_t)vgb::launch_wide_refit(ctx->stream, ctx->num_sms, reinterpret_cast<const uint32_t*>(ctx->d_nodes),
+                                                   ctx->nwide, ctx->d_wide));
         } else {
             vgb_bvh_options o{};
             o.max_leaf_size = ctx->bvh_leaf; o.threads = ctx->bvh_threads; o.layout = ctx->bvh_layout;
@@ -3350,18 +3314,17 @@ VGB_API vgb_status vgb_trace_rays(vgb_context* ctx, const float* org, const floa
     CK(cudaMemsetAsync(ctx->d_stats, 0, sizeof(uint64_t) * 8, ctx->stream));
     CK(cudaEventRecord(ctx->ev0, ctx->stream));
     const int g = grid_for(ctx, n, VGB_RAYS_GRID * 256 / VGB_RAYS_BLOCK, VGB_RAYS_BLOCK);
-    auto launch = [&](auto lc) {
+    auto launch = [&](auto lc, auto any) {
         constexpr int L = decltype(lc)::value;
-        if (any_hit) {
-            if (ctx->count_pass) k_trace_batch<L, true, true><<<g, VGB_RAYS_BLOCK, 0, ctx->stream>>>(sc, dorg, ddir, dtmax, n, dtri, dt, db, ctx->d_counters, ctx->d_stats);
-            else k_trace_batch<L, true, false><<<g, VGB_RAYS_BLOCK, 0, ctx->stream>>>(sc, dorg, ddir, dtmax, n, dtri, dt, db, ctx->d_counters, ctx->d_stats);
-        } else {
-            if (ctx->count_pass) k_trace_batch<L, false, true><<<g, VGB_RAYS_BLOCK, 0, ctx->stream>>>(sc, dorg, ddir, dtmax, n, dtri, dt, db, ctx->d_counters, ctx->d_stats);
-            else k_trace_batch<L, false, false><<<g, VGB_RAYS_BLOCK, 0, ctx->stream>>>(sc, dorg, ddir, dtmax, n, dtri, dt, db, ctx->d_counters, ctx->d_stats);
-        }
+        constexpr bool ANY = decltype(any)::value;
+        if (ctx->count_pass) k_trace_batch<L, ANY, true><<<g, VGB_RAYS_BLOCK, 0, ctx->stream>>>(sc, dorg, ddir, dtmax, n, dtri, dt, db, ctx->d_counters, ctx->d_stats);
+        else k_trace_batch<L, ANY, false><<<g, VGB_RAYS_BLOCK, 0, ctx->stream>>>(sc, dorg, ddir, dtmax, n, dtri, dt, db, ctx->d_counters, ctx->d_stats);
     };
-    if (ctx->bvh_layout == 8) launch(std::integral_constant<int, 8>{});
-    else launch(std::integral_constant<int, 2>{});
+    // An occlusion query reports the occluder that its walk meets first: it stays on the binary
+    // nodes, whose order callers have seen; the closest hit is the same whatever the nodes.
+    const bool l8 = ctx->bvh_layout == 8;
+    if (any_hit) { if (l8) launch(std::integral_constant<int, 8>{}, std::true_type{}); else launch(std::integral_constant<int, 2>{}, std::true_type{}); }
+    else { if (l8) launch(std::integral_constant<int, 8>{}, std::false_type{}); else launch(std::integral_constant<int, 4>{}, std::false_type{}); }
     CK(cudaGetLastError());
     CK(cudaEventRecord(ctx->ev1, ctx->stream));
     if (!on_device) {
@@ -3548,7 +3511,7 @@ template <int L>
 __device__ __noinline__ void trace_ool(const DevScene& s, WRay r, float tmax, bool any, HitOut& h, uint32_t& err) {
     Counters c{0, 0};
     if (L == 8) traverse8_rt<false>(s.nodes, s.tris, r, tmax, any, h, err, c, s.iter_cap);
-    else traverse_rt<false>(reinterpret_cast<const float4*>(s.nodes), s.tris, r, tmax, any, h, err, c, s.iter_cap);
+    else traverse4_rt<false>(s.wide, s.tris, r, tmax, any, h, err, c, s.iter_cap);
 }
 
 // ====================================================================== batched trajectory
@@ -3814,15 +3777,11 @@ template <int NB, int L, bool SUMS>
 __global__ void __launch_bounds__(256, VGB_BATCH_LEAN_MINB) k_batch_direct(const DevScene s, const DevFrame* __restrict__ frames,
                                                               const __grid_constant__ BatchParams bp, uint32_t* counter,
                                                               uint32_t* errw, uint64_t* stats) {
-    // The warp's lanes stay converged through every traversal (lanes outside the frame or whose
-    // ray missed carry flags), so the binary layout can trace the tile's rays as warp packets.
-    constexpr bool PACKET = L == 2 && VGB_BATCH_PACKET;
     const int lane = threadIdx.x & 31;
     const uint32_t nb = bp.nb;
     const vgb_pt_options& opt = bp.opt;
     const uint32_t k0 = (uint32_t)opt.seed, k1 = (uint32_t)(opt.seed >> 32);
     const uint32_t n_items = (bp.total_tiles + bp.tile_stride - 1) / bp.tile_stride;
-    const float4* nodes2 = reinterpret_cast<const float4*>(s.nodes);
     uint32_t err = 0, nclosest = 0, nshadow = 0;
     while (true) {
         uint32_t base = 0;
@@ -3854,14 +3813,12 @@ __global__ void __launch_bounds__(256, VGB_BATCH_LEAN_MINB) k_batch_direct(const
                 HitOut h;
                 h.U = h.V = h.W = 0.f; h.det = 1.f;
                 h.id = VGB_NO_HIT;
-                if (PACKET) {
-                    traverse_packet<false>(nodes2, s.tris, make_wray(ro, rd), 0.f, valid, h, err, s.iter_cap);
-                } else if (valid) {
+                if (valid) {
                     if (VGB_BATCH_LEAN_OOL) {
                         trace_ool<L>(s, make_wray(ro, rd), 0.f, false, h, err);
                     } else {
                         Counters c{0, 0};
-                        traverse_any_layout<L, false, false>(s.nodes, s.tris, make_wray(ro, rd), 0.f, h, err, c,
+                        traverse_any_layout<L, false, false>(bvh_nodes<L>(s), s.tris, make_wray(ro, rd), 0.f, h, err, c,
                                                              s.iter_cap);
                     }
                 }
@@ -3922,15 +3879,12 @@ __global__ void __launch_bounds__(256, VGB_BATCH_LEAN_MINB) k_batch_direct(const
                     const bool shadow = lit && lpdf > 0;
                     HitOut hs;
                     hs.id = VGB_NO_HIT;
-                    if (PACKET) {
-                        if (__any_sync(0xffffffffu, shadow))
-                            traverse_packet<true>(nodes2, s.tris, make_wray(Pp, Ld), dist, shadow, hs, err, s.iter_cap);
-                    } else if (shadow) {
+                    if (shadow) {
                         if (VGB_BATCH_LEAN_OOL) {
                             trace_ool<L>(s, make_wray(Pp, Ld), dist, true, hs, err);
                         } else {
                             Counters c{0, 0};
-                            traverse_any_layout<L, true, false>(s.nodes, s.tris, make_wray(Pp, Ld), dist, hs, err, c,
+                            traverse_any_layout<L, true, false>(bvh_nodes<L>(s), s.tris, make_wray(Pp, Ld), dist, hs, err, c,
                                                                 s.iter_cap);
                         }
                     }
@@ -4051,9 +4005,9 @@ cudaError_t launch_batch_any(vgb_context* ctx, const DevFrame* d_frames, const B
         if (bp.nb <= 4) return launch_batch<4, 8>(ctx, d_frames, bp, threads, bps);
         return launch_batch<8, 8>(ctx, d_frames, bp, threads, bps);
     }
-    if (bp.nb <= 1) return launch_batch<1, 2>(ctx, d_frames, bp, threads, bps);
-    if (bp.nb <= 4) return launch_batch<4, 2>(ctx, d_frames, bp, threads, bps);
-    return launch_batch<8, 2>(ctx, d_frames, bp, threads, bps);
+    if (bp.nb <= 1) return launch_batch<1, 4>(ctx, d_frames, bp, threads, bps);
+    if (bp.nb <= 4) return launch_batch<4, 4>(ctx, d_frames, bp, threads, bps);
+    return launch_batch<8, 4>(ctx, d_frames, bp, threads, bps);
 }
 
 }  // namespace
@@ -4709,9 +4663,9 @@ void launch_adjoint_batch(vgb_context* ctx, const DevView* views, const AdjBatch
 template <typename F>
 void dispatch_nb_layout(vgb_context* ctx, F&& f) {
     const bool l8 = ctx->bvh_layout == 8;
-    if (ctx->nbands <= 1) { if (l8) f(std::integral_constant<int, 1>{}, std::integral_constant<int, 8>{}); else f(std::integral_constant<int, 1>{}, std::integral_constant<int, 2>{}); }
-    else if (ctx->nbands <= 4) { if (l8) f(std::integral_constant<int, 4>{}, std::integral_constant<int, 8>{}); else f(std::integral_constant<int, 4>{}, std::integral_constant<int, 2>{}); }
-    else { if (l8) f(std::integral_constant<int, 8>{}, std::integral_constant<int, 8>{}); else f(std::integral_constant<int, 8>{}, std::integral_constant<int, 2>{}); }
+    if (ctx->nbands <= 1) { if (l8) f(std::integral_constant<int, 1>{}, std::integral_constant<int, 8>{}); else f(std::integral_constant<int, 1>{}, std::integral_constant<int, 4>{}); }
+    else if (ctx->nbands <= 4) { if (l8) f(std::integral_constant<int, 4>{}, std::integral_constant<int, 8>{}); else f(std::integral_constant<int, 4>{}, std::integral_constant<int, 4>{}); }
+    else { if (l8) f(std::integral_constant<int, 8>{}, std::integral_constant<int, 8>{}); else f(std::integral_constant<int, 8>{}, std::integral_constant<int, 4>{}); }
 }
 
 // Position-gradient scratch: vertex-normal gradients, normal sums and (for z-only callers)

@@ -19,18 +19,7 @@ constexpr uint32_t kSlotMain = 0u, kSlotRR = 0xFEu, kSlotJitter = 0xFFu;
 // device error word bits
 constexpr uint32_t kErrStack = 1u, kErrIter = 2u;
 
-constexpr int kStackSize = 64;
-// 1: the wavefront traversal kernels postpone leaves speculatively (traverse_spec_rt).
-#ifndef VGB_TRAV_SPECULATIVE
-#define VGB_TRAV_SPECULATIVE 0
-#endif
-// 1: traverse_rt keeps each pushed child's entry distance on the stack and, for closest-hit
-// rays, drops a popped entry whose box starts beyond the current closest hit without fetching it
-// (the box test re-evaluated with the new bound; results unchanged).  Off: on the path-traced
-// frame the closest-hit launches took 82.2 against 81.5 ms per frame with it.
-#ifndef VGB_TRAV_CULL
-#define VGB_TRAV_CULL 0
-#endif
+constexpr int kStackSize = 64;   // binary layout
 constexpr uint32_t kIterCap = 1u << 22;  // default traversal steps per ray before giving up
 
 // ------------------------------------------------------------------ Philox-4x32-10
@@ -202,9 +191,6 @@ __device__ __forceinline__ void traverse_rt(const float4* __restrict__ nodes, co
                                             const WRay& r, float tmax, const bool any, HitOut& h, uint32_t& err,
                                             Counters& cnt, uint32_t cap) {
     int stack[kStackSize];
-#if VGB_TRAV_CULL
-    float stack_tn[kStackSize];   // entry distance of each stacked child's box
-#endif
     int sp = 0;
     int node = 0;
     float best = any ? tmax : __int_as_float(0x7f800000);
@@ -212,25 +198,6 @@ __device__ __forceinline__ void traverse_rt(const float4* __restrict__ nodes, co
     h.id = VGB_NO_HIT;
     uint32_t iter = 0;
     const SlabRay q = make_slab(r);
-    // The next stacked node, or false when the stack is empty.  With culling, a closest-hit
-    // ray skips entries whose box test, re-run against the current closest hit, would fail: the
-    // test passes iff tn <= min(tf, best) * widen, and tn <= tf * widen held when it was pushed.
-    auto pop = [&](int& nd) -> bool {
-#if VGB_TRAV_CULL
-        const float bound = best * (1.0f + 0x1p-20f);
-        while (sp > 0) {
-            --sp;
-            if (!any && stack_tn[sp] > bound) continue;
-            nd = stack[sp];
-            return true;
-        }
-        return false;
-#else
-        if (sp == 0) return false;
-        nd = stack[--sp];
-        return true;
-#endif
-    };
     while (true) {
         while (node >= 0) {
             if (++iter > cap) { err |= kErrIter; return; }
@@ -246,14 +213,8 @@ __device__ __forceinline__ void traverse_rt(const float4* __restrict__ nodes, co
             const int ch0 = __float_as_int(n3.x), ch1 = __float_as_int(n3.y);
             if (h0 && h1) {
                 int nearc = ch0, farc = ch1;
-                float tfar = tn1;
-                if (tn1 < tn0) { nearc = ch1; farc = ch0; tfar = tn0; }
+                if (tn1 < tn0) { nearc = ch1; farc = ch0; }
                 if (sp >= kStackSize) { err |= kErrStack; return; }
-#if VGB_TRAV_CULL
-                stack_tn[sp] = tfar;
-#else
-                (void)tfar;
-#endif
                 stack[sp++] = farc;
                 node = nearc;
             } else if (h0) {
@@ -261,7 +222,8 @@ __device__ __forceinline__ void traverse_rt(const float4* __restrict__ nodes, co
             } else if (h1) {
                 node = ch1;
             } else {
-                if (!pop(node)) return;
+                if (sp == 0) return;
+                node = stack[--sp];
             }
         }
         // leaf
@@ -283,70 +245,152 @@ __device__ __forceinline__ void traverse_rt(const float4* __restrict__ nodes, co
                 }
             }
         }
-        if (!pop(node)) return;
+        if (sp == 0) return;
+        node = stack[--sp];
     }
 }
 
-// Resumable form of traverse_rt for the persistent traversal kernels: the state of one ray's
-// traversal between calls (the stack itself lives in the caller's per-thread array).
-struct TravState {
-    int node;       // next node (>= 0 inner; < 0 a leaf to test)
-    int sp;         // stack depth
-    float best;     // closest-hit t so far (tmax for occlusion rays)
-    uint32_t iter;  // inner nodes visited
-};
+// ------------------------------------------------------------------ wide traversal (4 children per node)
+// The layout the render, batch, adjoint and closest-hit ray kernels walk: the binary tree with
+// up to three inner nodes folded into one 128-byte node (one cache line; WideNode in
+// vgb_internal.h), so a ray follows half as many dependent node fetches.  A child's box is its
+// centre c and half extent h: with m = (c - o) / d, the entry and exit of an axis are m - h / |d|
+// and m + h / |d|, which needs no per-axis minimum and maximum, and the four operations run two
+// lanes wide (f32x2).  The binary traversal was bound by the latency of its chain of node fetches
+// and by the ALU pipe that executes minimum, maximum and select (47 % busy against 17 % of the
+// FMA pipe at camera rays).
+// Nodes visited per ray 24.3 -> 12.3 (8.4M triangles, camera and bounce rays);
+// whole calls: 512^2 x 16 spp over 2.1M triangles 7.96 -> 7.32 ms, 2048^2 x 4 spp over 8.4M 14.1 ->
+// 13.5 ms, fused adjoint of 12 asteroid views 9.0 -> 7.8 ms.  Folding three nodes beat the same
+// box test on the binary nodes (7.91 against 7.38 ms of device time at 512^2, 13.38 against 13.15
+// at 2048^2); walking the children of occlusion rays unsorted lost (2.94 -> 3.16 ms at 512^2).
+//
+// Conservative: m carries a relative error below 4 * 2^-24, so a plane distance m -+ h / |d| is
+// off by at most that part of |distance| + h / |d|; the builder enlarges h (wide_half_extent) by
+// far more than the second part, and the exit distance is widened by 2^-18 for the first, which
+// also covers the rounding of the triangle test's own distance and edge functions.  No box that
+// holds a triangle the test accepts is culled, so the closest hit does not depend on the layout.
+constexpr int kStackWide = 192;             // up to three pushes per level of a 64-level binary tree
+constexpr int kWideEmpty = (int)0x80000000; // link of an empty child slot; the stack's bottom entry
 
-__device__ __forceinline__ TravState trav_start(float tmax, bool any, HitOut& h) {
-    h.t = __int_as_float(0x7f800000);
-    h.id = VGB_NO_HIT;
-    h.U = h.V = h.W = 0.f;
-    h.det = 1.f;
-    return TravState{0, 0, any ? tmax : __int_as_float(0x7f800000), 0u};
+typedef unsigned long long u64;
+__device__ __forceinline__ u64 pk2(float lo, float hi) {
+    u64 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ void up2(u64 v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+__device__ __forceinline__ u64 add2(u64 a, u64 b) {
+    u64 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ u64 mul2(u64 a, u64 b) {
+    u64 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ u64 fma2(u64 a, u64 b, u64 c) {
+    u64 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+// 32 bytes (a 32-byte aligned address) in one load.
+__device__ __forceinline__ void ldg32(const void* p, u64& a, u64& b, u64& c, u64& d) {
+    asm("ld.global.nc.v4.b64 {%0, %1, %2, %3}, [%4];" : "=l"(a), "=l"(b), "=l"(c), "=l"(d) : "l"(p));
 }
 
-// Continues the traversal of ray r for at most `budget` inner-node visits.  Returns true when the
-// ray is finished (h holds its answer), false when it stopped early; the next call resumes where it
-// stopped.  Node order, box and triangle tests are traverse_rt's, so the answer is the same.
-template <bool COUNT>
-__device__ __forceinline__ bool traverse_resume(const float4* __restrict__ nodes, const float4* __restrict__ tris,
-                                                const WRay& r, const SlabRay& q, float tmax, const bool any,
-                                                int* stack, TravState& ts, HitOut& h, uint32_t& err, Counters& cnt,
-                                                uint32_t cap, int budget) {
+// Per-ray constants: minus the origin, 1/d and +-1/|d|, the x and y axes as a pair, z twice.
+struct WideRay { u64 noxy, nozz, ixy, izz, axy, azz, nxy, nzz; };
+__device__ __forceinline__ WideRay make_wide(const WRay& r) {
+    WideRay q;
+    const float ax = fabsf(r.ix), ay = fabsf(r.iy), az = fabsf(r.iz);
+    q.noxy = pk2(-r.o.x, -r.o.y); q.nozz = pk2(-r.o.z, -r.o.z);
+    q.ixy = pk2(r.ix, r.iy); q.izz = pk2(r.iz, r.iz);
+    q.axy = pk2(ax, ay); q.azz = pk2(az, az);
+    q.nxy = pk2(-ax, -ay); q.nzz = pk2(-az, -az);
+    return q;
+}
+
+// State of one ray's traversal between calls (the stack lives in the caller's per-thread array).
+struct TravState {
+    int node;       // next node (>= 0 inner; < 0 a leaf to test; kWideEmpty: finished)
+    int sp;         // stack entries, the bottom one included
+    float best;     // closest-hit t so far (tmax for occlusion rays)
+    uint32_t iter;  // nodes visited
+};
+
+__device__ __forceinline__ TravState trav_start(float tmax, bool any, HitOut& h, int* stack) {
+    h.t = __int_as_float(0x7f800000);
+    h.id = VGB_NO_HIT;
+    stack[0] = kWideEmpty;
+    return TravState{0, 1, any ? tmax : __int_as_float(0x7f800000), 0u};
+}
+
+// Closest hit (any = false; ties in t go to the smaller id) or occlusion (any = true, any hit
+// with t <= tmax).  RESUME: stops after `budget` nodes; returns true when the ray is finished (h
+// holds its answer), false when the next call is to continue from ts.
+template <bool COUNT, bool RESUME>
+__device__ __forceinline__ bool traverse4(const uint4* __restrict__ nodes, const float4* __restrict__ tris,
+                                          const WRay& r, const WideRay& q, float tmax, const bool any, int* stack,
+                                          TravState& ts, HitOut& h, uint32_t& err, Counters& cnt, uint32_t cap,
+                                          int budget) {
+    const u64 widen = pk2(1.0f + 0x1p-18f, 1.0f + 0x1p-18f);
+    const float inf = __int_as_float(0x7f800000);
     int node = ts.node, sp = ts.sp;
     float best = ts.best;
     uint32_t iter = ts.iter;
     while (true) {
         while (node >= 0) {
-            if (budget-- <= 0) {
+            if (RESUME && budget-- <= 0) {
                 ts.node = node; ts.sp = sp; ts.best = best; ts.iter = iter;
                 return false;
             }
             if (++iter > cap) { err |= kErrIter; return true; }
-            const float4 n0 = __ldg(&nodes[4 * node + 0]);
-            const float4 n1 = __ldg(&nodes[4 * node + 1]);
-            const float4 n2 = __ldg(&nodes[4 * node + 2]);
-            const float4 n3 = __ldg(&nodes[4 * node + 3]);
+            if (sp > kStackWide - 3) { err |= kErrStack; return true; }
+            const char* p = reinterpret_cast<const char*>(nodes) + (size_t)(uint32_t)node * 128u;
+            u64 c0, h0, c1, h1, c2, h2, c3, h3, cz01, cz23, hz01, hz23;
+            ldg32(p, c0, h0, c1, h1);
+            ldg32(p + 32, c2, h2, c3, h3);
+            ldg32(p + 64, cz01, cz23, hz01, hz23);
+            const int4 link = __ldg(reinterpret_cast<const int4*>(p + 96));
             if (COUNT) cnt.nodes++;
-            float tn0, tf0, tn1, tf1;
-            slab(q, n0.x, n0.y, n0.z, n0.w, n2.x, n2.y, best, tn0, tf0);
-            slab(q, n1.x, n1.y, n1.z, n1.w, n2.z, n2.w, best, tn1, tf1);
-            const bool h0 = tn0 <= tf0, h1 = tn1 <= tf1;
-            const int ch0 = __float_as_int(n3.x), ch1 = __float_as_int(n3.y);
-            if (h0 && h1) {
-                int nearc = ch0, farc = ch1;
-                if (tn1 < tn0) { nearc = ch1; farc = ch0; }
-                if (sp >= kStackSize) { err |= kErrStack; return true; }
-                stack[sp++] = farc;
-                node = nearc;
-            } else if (h0) {
-                node = ch0;
-            } else if (h1) {
-                node = ch1;
-            } else {
-                if (sp == 0) return true;
-                node = stack[--sp];
+            float tn[4], tf[4];
+            {
+                const u64 m01 = mul2(add2(cz01, q.nozz), q.izz), m23 = mul2(add2(cz23, q.nozz), q.izz);
+                up2(fma2(hz01, q.nzz, m01), tn[0], tn[1]);
+                up2(fma2(hz23, q.nzz, m23), tn[2], tn[3]);
+                up2(fma2(hz01, q.azz, m01), tf[0], tf[1]);
+                up2(fma2(hz23, q.azz, m23), tf[2], tf[3]);
             }
+            const u64 cc[4] = {c0, c1, c2, c3}, hh[4] = {h0, h1, h2, h3};
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const u64 m = mul2(add2(cc[k], q.noxy), q.ixy);
+                float nx, ny, fx, fy;
+                up2(fma2(hh[k], q.nxy, m), nx, ny);
+                up2(fma2(hh[k], q.axy, m), fx, fy);
+                tn[k] = fmax3(nx, ny, fmaxf(tn[k], 0.0f));
+                tf[k] = fmin3(fx, fy, fminf(tf[k], best));
+            }
+            up2(mul2(pk2(tf[0], tf[1]), widen), tf[0], tf[1]);
+            up2(mul2(pk2(tf[2], tf[3]), widen), tf[2], tf[3]);
+            const bool b0 = tn[0] <= tf[0], b1 = tn[1] <= tf[1], b2 = tn[2] <= tf[2], b3 = tn[3] <= tf[3];
+            const int l0 = b0 ? link.x : kWideEmpty, l1 = b1 ? link.y : kWideEmpty;
+            const int l2 = b2 ? link.z : kWideEmpty, l3 = b3 ? link.w : kWideEmpty;
+            // near to far: each pair by its entry distances, then the pairs by their nearer one
+            const float t0 = b0 ? tn[0] : inf, t1 = b1 ? tn[1] : inf, t2 = b2 ? tn[2] : inf, t3 = b3 ? tn[3] : inf;
+            const bool s01 = t1 < t0, s23 = t3 < t2;
+            const int a0 = s01 ? l1 : l0, a1 = s01 ? l0 : l1, e0 = s23 ? l3 : l2, e1 = s23 ? l2 : l3;
+            const bool sw = fminf(t2, t3) < fminf(t0, t1);
+            const int n0 = sw ? e0 : a0, n1 = sw ? e1 : a1, f0 = sw ? a0 : e0, f1 = sw ? a1 : e1;
+            if (f1 != kWideEmpty) stack[sp++] = f1;
+            if (f0 != kWideEmpty) stack[sp++] = f0;
+            if (n1 != kWideEmpty) stack[sp++] = n1;
+            node = n0;
+            if (node == kWideEmpty) node = stack[--sp];
         }
+        if (node == kWideEmpty) return true;
         const uint32_t x = ~(uint32_t)node;
         const uint32_t start = x >> 3, cntl = (x & 7u) + 1u;
         for (uint32_t k = 0; k < cntl; ++k) {
@@ -365,184 +409,17 @@ __device__ __forceinline__ bool traverse_resume(const float4* __restrict__ nodes
                 }
             }
         }
-        if (sp == 0) return true;
         node = stack[--sp];
     }
 }
 
-// Warp-packet traversal of the binary BVH for coherent rays (a warp's 8x4 pixel tile of camera
-// rays, or their shadow rays towards one light).  Every lane of the warp calls it together; a
-// lane with active = false only takes part.  The warp walks one node sequence: each node is
-// fetched once for all lanes (the same address, one broadcast load), every active lane tests
-// both child boxes against its own ray and current best distance, and a child is entered when
-// any lane's ray overlaps it, the one more lanes reach first.  Leaves are tested by every active
-// lane.  A lane thus tests a superset of the triangles its own traversal would test, with the
-// same conservative box test and the same acceptance rule (closest t, ties to the smaller id;
-// any hit within tmax), so its answer is the same as traverse_rt's: the closest hit does not
-// depend on which boxes are opened, and an occlusion test only reports whether some triangle
-// lies within tmax.  The warp's node stack (kStackSize = 64 entries) is spread over the lanes'
-// registers: entry i is held by lane i % 32 in its register s0 (i < 32) or s1.
-template <bool ANY>
-__device__ __forceinline__ void traverse_packet(const float4* __restrict__ nodes, const float4* __restrict__ tris,
-                                                const WRay& r, float tmax, bool active, HitOut& h, uint32_t& err,
-                                                uint32_t cap) {
-    static_assert(kStackSize == 64, "two stack registers per lane");
-    const unsigned full = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
-    h.t = __int_as_float(0x7f800000);
-    h.id = VGB_NO_HIT;
-    float best = ANY ? tmax : __int_as_float(0x7f800000);
-    bool live = active;
-    const SlabRay q = make_slab(r);
-    int sp = 0, node = 0, s0 = 0, s1 = 0;
-    uint32_t iter = 0;
-    if (!__any_sync(full, live)) return;
-    while (true) {
-        while (node >= 0) {
-            if (++iter > cap) { if (live) err |= kErrIter; return; }
-            const float4 n0 = __ldg(&nodes[4 * node + 0]);
-            const float4 n1 = __ldg(&nodes[4 * node + 1]);
-            const float4 n2 = __ldg(&nodes[4 * node + 2]);
-            const float4 n3 = __ldg(&nodes[4 * node + 3]);
-            bool h0 = false, h1 = false, near0 = false;
-            if (live) {
-                float tn0, tf0, tn1, tf1;
-                slab(q, n0.x, n0.y, n0.z, n0.w, n2.x, n2.y, best, tn0, tf0);
-                slab(q, n1.x, n1.y, n1.z, n1.w, n2.z, n2.w, best, tn1, tf1);
-                h0 = tn0 <= tf0;
-                h1 = tn1 <= tf1;
-                near0 = h0 && (!h1 || tn0 <= tn1);
-            }
-            const unsigned m0 = __ballot_sync(full, h0), m1 = __ballot_sync(full, h1);
-            const int ch0 = __float_as_int(n3.x), ch1 = __float_as_int(n3.y);
-            if (m0 && m1) {
-                const unsigned nm = __ballot_sync(full, near0);
-                const bool first0 = 2 * __popc(nm) >= __popc(m0 | m1);
-                if (sp >= kStackSize) { if (live) err |= kErrStack; return; }
-                if (lane == (sp & 31)) {
-                    if (sp < 32) s0 = first0 ? ch1 : ch0;
-                    else s1 = first0 ? ch1 : ch0;
-                }
-                ++sp;
-                node = first0 ? ch0 : ch1;
-            } else if (m0) {
-                node = ch0;
-            } else if (m1) {
-                node = ch1;
-            } else {
-                if (sp == 0) return;
-                --sp;
-                node = __shfl_sync(full, sp < 32 ? s0 : s1, sp & 31);
-            }
-        }
-        const uint32_t x = ~(uint32_t)node;
-        const uint32_t start = x >> 3, cntl = (x & 7u) + 1u;
-        for (uint32_t k = 0; k < cntl; ++k) {
-            const float4 t0 = __ldg(&tris[3 * (start + k) + 0]);
-            const float4 t1 = __ldg(&tris[3 * (start + k) + 1]);
-            const float4 t2 = __ldg(&tris[3 * (start + k) + 2]);
-            float tt, U, V, W, det;
-            if (live && wt_test(r, ld3(t0), ld3(t1), ld3(t2), tt, U, V, W, det)) {
-                const uint32_t id = __float_as_uint(t0.w);
-                if (ANY) {
-                    if (tt <= tmax) { h.t = tt; h.id = id; live = false; }
-                } else if (tt < h.t || (tt == h.t && id < h.id)) {
-                    h.t = tt; h.id = id; h.U = U; h.V = V; h.W = W; h.det = det;
-                    best = tt;
-                }
-            }
-        }
-        if (ANY && !__any_sync(full, live)) return;
-        if (sp == 0) return;
-        --sp;
-        node = __shfl_sync(full, sp < 32 ? s0 : s1, sp & 31);
-    }
-}
-
-// traverse_rt with speculative leaf postponing (Aila and Laine, HPG 2009, "speculative
-// while-while"): a lane that reaches a leaf while others are still among inner nodes keeps the
-// leaf aside and goes on to the next inner node; the warp tests leaves once every converged lane
-// holds one.  The set of leaves tested and the acceptance rule are traverse_rt's, only their
-// order changes, so the answer is the same (the closest hit does not depend on the order).
 template <bool COUNT>
-__device__ __forceinline__ void traverse_spec_rt(const float4* __restrict__ nodes, const float4* __restrict__ tris,
-                                                 const WRay& r, float tmax, const bool any, HitOut& h,
-                                                 uint32_t& err, Counters& cnt, uint32_t cap) {
-    constexpr int kDone = 0x7fffffff;   // beyond every node index: traversal finished
-    int stack[kStackSize];
-    int sp = 0;
-    int node = 0, leaf = kDone;          // leaf < 0: a postponed leaf
-    float best = any ? tmax : __int_as_float(0x7f800000);
-    h.t = __int_as_float(0x7f800000);
-    h.id = VGB_NO_HIT;
-    uint32_t iter = 0;
-    const SlabRay q = make_slab(r);
-    while (node != kDone || leaf < 0) {
-        while (node >= 0 && node != kDone) {
-            if (++iter > cap) { err |= kErrIter; return; }
-            const float4 n0 = __ldg(&nodes[4 * node + 0]);
-            const float4 n1 = __ldg(&nodes[4 * node + 1]);
-            const float4 n2 = __ldg(&nodes[4 * node + 2]);
-            const float4 n3 = __ldg(&nodes[4 * node + 3]);
-            if (COUNT) cnt.nodes++;
-            float tn0, tf0, tn1, tf1;
-            slab(q, n0.x, n0.y, n0.z, n0.w, n2.x, n2.y, best, tn0, tf0);
-            slab(q, n1.x, n1.y, n1.z, n1.w, n2.z, n2.w, best, tn1, tf1);
-            const bool h0 = tn0 <= tf0, h1 = tn1 <= tf1;
-            const int ch0 = __float_as_int(n3.x), ch1 = __float_as_int(n3.y);
-            if (h0 && h1) {
-                int nearc = ch0, farc = ch1;
-                if (tn1 < tn0) { nearc = ch1; farc = ch0; }
-                if (sp >= kStackSize) { err |= kErrStack; return; }
-                stack[sp++] = farc;
-                node = nearc;
-            } else if (h0) {
-                node = ch0;
-            } else if (h1) {
-                node = ch1;
-            } else {
-                node = sp ? stack[--sp] : kDone;
-            }
-            if (node < 0 && leaf >= 0) {   // postpone the first leaf, keep descending
-                leaf = node;
-                node = sp ? stack[--sp] : kDone;
-            }
-            if (!__any_sync(__activemask(), leaf >= 0)) break;
-        }
-        while (leaf < 0) {
-            const uint32_t x = ~(uint32_t)leaf;
-            const uint32_t start = x >> 3, cntl = (x & 7u) + 1u;
-            for (uint32_t k = 0; k < cntl; ++k) {
-                const float4 t0 = __ldg(&tris[3 * (start + k) + 0]);
-                const float4 t1 = __ldg(&tris[3 * (start + k) + 1]);
-                const float4 t2 = __ldg(&tris[3 * (start + k) + 2]);
-                if (COUNT) cnt.tris++;
-                float tt, U, V, W, det;
-                if (wt_test(r, ld3(t0), ld3(t1), ld3(t2), tt, U, V, W, det)) {
-                    const uint32_t id = __float_as_uint(t0.w);
-                    if (any) {
-                        if (tt <= tmax) { h.t = tt; h.id = id; return; }
-                    } else if (tt < h.t || (tt == h.t && id < h.id)) {
-                        h.t = tt; h.id = id; h.U = U; h.V = V; h.W = W; h.det = det;
-                        best = tt;
-                    }
-                }
-            }
-            leaf = node;                   // the current node may be a leaf too
-            if (node < 0) node = sp ? stack[--sp] : kDone;
-        }
-    }
-}
-
-template <bool ANY, bool COUNT>
-__device__ __forceinline__ void traverse(const float4* __restrict__ nodes, const float4* __restrict__ tris,
-                                         const WRay& r, float tmax, HitOut& h, uint32_t& err, Counters& cnt,
-                                         uint32_t cap) {
-#if VGB_TRAV_SPECULATIVE
-    traverse_spec_rt<COUNT>(nodes, tris, r, tmax, ANY, h, err, cnt, cap);
-#else
-    traverse_rt<COUNT>(nodes, tris, r, tmax, ANY, h, err, cnt, cap);
-#endif
+__device__ __forceinline__ void traverse4_rt(const uint4* __restrict__ nodes, const float4* __restrict__ tris,
+                                             const WRay& r, float tmax, const bool any, HitOut& h, uint32_t& err,
+                                             Counters& cnt, uint32_t cap) {
+    int stack[kStackWide];
+    TravState ts = trav_start(tmax, any, h, stack);
+    traverse4<COUNT, false>(nodes, tris, r, make_wide(r), tmax, any, stack, ts, h, err, cnt, cap, 0);
 }
 
 // ------------------------------------------------------------------ compressed 8-wide traversal
@@ -685,14 +562,15 @@ __device__ __forceinline__ void traverse8(const uint4* __restrict__ nodes, const
     traverse8_rt<COUNT>(nodes, tris, r, tmax, ANY, h, err, cnt, cap);
 }
 
-// Dispatch on the node layout (2: binary, 8: compressed 8-wide).  `cap`: traversal steps per
-// ray before the ray gives up and sets kErrIter.
+// Dispatch on the node layout (2: binary, 4: wide, 8: compressed 8-wide).  `cap`: traversal steps
+// per ray before the ray gives up and sets kErrIter.
 template <int LAYOUT, bool ANY, bool COUNT>
 __device__ __forceinline__ void traverse_any_layout(const uint4* __restrict__ nodes, const float4* __restrict__ tris,
                                                     const WRay& r, float tmax, HitOut& h, uint32_t& err, Counters& cnt,
                                                     uint32_t cap) {
     if (LAYOUT == 8) traverse8<ANY, COUNT>(nodes, tris, r, tmax, h, err, cnt, cap);
-    else traverse<ANY, COUNT>(reinterpret_cast<const float4*>(nodes), tris, r, tmax, h, err, cnt, cap);
+    else if (LAYOUT == 4) traverse4_rt<COUNT>(nodes, tris, r, tmax, ANY, h, err, cnt, cap);
+    else traverse_rt<COUNT>(reinterpret_cast<const float4*>(nodes), tris, r, tmax, ANY, h, err, cnt, cap);
 }
 
 }  // namespace vgbd

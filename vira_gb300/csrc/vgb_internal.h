@@ -8,6 +8,14 @@
 // A leaf holds 1..8 consecutive triangle records.  The root is node 0; a scene whose root
 // is a leaf gets one inner node whose two children are that leaf.
 //
+// Device BVH (wide): up to three binary inner nodes folded into one node of four children, 128
+// bytes (a cache line), made on the device from the binary nodes (vgb_mesh.cu, launch_wide_*):
+//   bytes 0..63    per child: (centre x, centre y, half extent x, half extent y)
+//   bytes 64..95   centre z of the four children, half extent z of the four children
+//   bytes 96..111  four links: >= 0 wide node index, < 0 leaf as above, 0x80000000 empty slot
+//   bytes 112..127 four sources: (binary node << 1) | side whose box the child carries (refits)
+// The half extents are enlarged (wide_half_extent); an empty slot has half extent -1.
+//
 // Device BVH (compressed 8-wide): one node is five 16-byte words, see vgb_host.cpp.
 //
 // Triangle record (watertight test input), three 16-byte words in leaf order:
@@ -190,6 +198,14 @@ int launch_lbvh_emit(void* stream, int sms, const void* vpos, const uint32_t* id
 // Returns nonzero on a CUDA error, -2 when an upward walk exceeded its bound.
 int launch_refit(void* stream, int sms, const void* vpos /* float4 */, const uint32_t* idx, uint32_t ntris,
                  void* tris /* float4 */, uint32_t* nodes, uint32_t nnodes, const uint32_t* parent, uint32_t* counts);
+// The wide nodes of a binary BVH: fold writes the node roots and their children into `work`
+// (wide_work_words) and returns the number of wide nodes; emit writes them (128 bytes each);
+// refit rewrites the boxes of emitted nodes from the binary ones.  Return a CUDA error or 0.
+size_t wide_work_words(uint32_t nnodes);
+int launch_wide_fold(void* stream, int sms, const uint32_t* nodes, uint32_t nnodes, uint32_t* work, uint32_t* nwide_out);
+int launch_wide_emit(void* stream, int sms, const uint32_t* nodes, uint32_t nnodes, const uint32_t* work,
+                     uint32_t nwide, void* wide);
+int launch_wide_refit(void* stream, int sms, const uint32_t* nodes, uint32_t nwide, void* wide);
 
 
 // ---- DEM Quipu (vgb_quipu.cpp host side, vgb_mesh.cu device decode)

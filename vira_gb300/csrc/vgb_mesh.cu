@@ -482,9 +482,163 @@ __global__ void k_refit_nodes(const float4* __restrict__ tris, uint32_t* nodes, 
     }
 }
 
+// ------------------------------------------------------------------ wide nodes (4 children)
+// The enlarged half extent of a child box [lo, hi] of one axis about the centre c: the exact one
+// (both differences are rounded up by the factor) plus a part of the box's largest half extent and
+// of its distance from the frame's origin, which covers the rounding of the box test (2^-22 of
+// the half extent) and of the triangle test's vertex differences and edge functions (a few parts
+// in 2^24 of the coordinates and of the triangle's size, in any axis).
+__device__ __forceinline__ float wide_half_extent(float lo, float hi, float c, float slack) {
+    return fmaxf(hi - c, c - lo) * (1.0f + 0x1p-18f) + slack;
+}
+
+__device__ __forceinline__ void put_wide_child(float* w, int k, const RBox& b) {
+    const float cx = 0.5f * b.lx + 0.5f * b.hx, cy = 0.5f * b.ly + 0.5f * b.hy, cz = 0.5f * b.lz + 0.5f * b.hz;
+    const float ex = b.hx - cx, ey = b.hy - cy, ez = b.hz - cz;
+    const float slack = 0x1p-21f * (fmaxf(fmaxf(fabsf(cx), fabsf(cy)), fabsf(cz)) + fmaxf(fmaxf(ex, ey), ez)) + 1e-12f;
+    const bool ok = isfinite(b.lx) && isfinite(b.hx) && isfinite(b.ly) && isfinite(b.hy) && isfinite(b.lz) && isfinite(b.hz);
+    // a box with an infinite or undefined bound is never culled
+    w[4 * k] = ok ? cx : 0.f;
+    w[4 * k + 1] = ok ? cy : 0.f;
+    w[16 + k] = ok ? cz : 0.f;
+    w[4 * k + 2] = ok ? wide_half_extent(b.lx, b.hx, cx, slack) : 3e38f;
+    w[4 * k + 3] = ok ? wide_half_extent(b.ly, b.hy, cy, slack) : 3e38f;
+    w[20 + k] = ok ? wide_half_extent(b.lz, b.hz, cz, slack) : 3e38f;
+}
+
+// One level of the fold: the roots queue[begin, end) each open the inner child of the largest
+// surface until they have four children or only leaves, and queue the inner children as roots.
+__global__ void k_wide_fold(const uint32_t* __restrict__ nodes, uint32_t* queue, uint32_t begin, uint32_t end,
+                            uint4* __restrict__ src, uint32_t* __restrict__ is_root, uint32_t* tail) {
+    for (uint32_t i = begin + blockIdx.x * blockDim.x + threadIdx.x; i < end; i += gridDim.x * blockDim.x) {
+        const uint32_t root = queue[i];
+        is_root[root] = 1u;
+        uint32_t e[4] = {root << 1, (root << 1) | 1u, vgb::kNoParent, vgb::kNoParent};
+        int n = 2;
+        while (n < 4) {
+            int best = -1;
+            float area = -1.f;
+            for (int k = 0; k < n; ++k) {
+                if ((int32_t)nodes[16 * (size_t)(e[k] >> 1) + 12 + (e[k] & 1u)] < 0) continue;
+                const RBox b = get_box(nodes, e[k] >> 1, (int)(e[k] & 1u));
+                const float x = b.hx - b.lx, y = b.hy - b.ly, z = b.hz - b.lz;
+                const float a = x * y + y * z + z * x;
+                if (best < 0 || a > area) { area = a; best = k; }
+            }
+            if (best < 0) break;
+            const uint32_t m = nodes[16 * (size_t)(e[best] >> 1) + 12 + (e[best] & 1u)];
+            for (int k = n; k > best + 1; --k) e[k] = e[k - 1];   // keep the tree's order: siblings stay adjacent
+            e[best] = m << 1;
+            e[best + 1] = (m << 1) | 1u;
+            ++n;
+        }
+        src[i] = make_uint4(e[0], e[1], e[2], e[3]);
+        uint32_t inner[4];
+        int c = 0;
+        for (int k = 0; k < n; ++k) {
+            const int32_t link = (int32_t)nodes[16 * (size_t)(e[k] >> 1) + 12 + (e[k] & 1u)];
+            if (link >= 0) inner[c++] = (uint32_t)link;
+        }
+        if (c) {
+            const uint32_t at = atomicAdd(tail, (uint32_t)c);
+            for (int k = 0; k < c; ++k) queue[at + k] = inner[k];
+        }
+    }
+}
+
+// Wide nodes in the order of their roots among the binary nodes (rank: exclusive scan of is_root),
+// so the memory order of the tree is the binary tree's.
+__global__ void k_wide_emit(const uint32_t* __restrict__ nodes, const uint32_t* __restrict__ queue,
+                            const uint4* __restrict__ src, const uint32_t* __restrict__ rank, uint32_t nwide,
+                            float* __restrict__ wide) {
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nwide; i += gridDim.x * blockDim.x) {
+        float* w = wide + 32 * (size_t)rank[queue[i]];
+        const uint4 s4 = src[i];
+        const uint32_t e[4] = {s4.x, s4.y, s4.z, s4.w};
+        for (int k = 0; k < 4; ++k) {
+            uint32_t link = 0x80000000u;
+            if (e[k] == vgb::kNoParent) {
+                w[4 * k] = w[4 * k + 1] = w[16 + k] = 0.f;
+                w[4 * k + 2] = w[4 * k + 3] = w[20 + k] = -1.f;
+            } else {
+                put_wide_child(w, k, get_box(nodes, e[k] >> 1, (int)(e[k] & 1u)));
+                link = nodes[16 * (size_t)(e[k] >> 1) + 12 + (e[k] & 1u)];
+                if ((int32_t)link >= 0) link = rank[link];
+            }
+            w[24 + k] = __uint_as_float(link);
+            w[28 + k] = __uint_as_float(e[k]);
+        }
+    }
+}
+
+__global__ void k_wide_refit(const uint32_t* __restrict__ nodes, uint32_t nwide, float* __restrict__ wide) {
+    for (size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x; q < 4 * (size_t)nwide;
+         q += (size_t)gridDim.x * blockDim.x) {
+        float* w = wide + 32 * (q >> 2);
+        const int k = (int)(q & 3);
+        const uint32_t e = __float_as_uint(w[28 + k]);
+        if (e != vgb::kNoParent) put_wide_child(w, k, get_box(nodes, e >> 1, (int)(e & 1u)));
+    }
+}
+
 }  // namespace
 
 namespace vgb {
+
+// work: queue of roots [nnodes], sources [4 nnodes], root flags and their scan [nnodes + 1 each],
+// the queue's tail, scan scratch
+size_t wide_work_words(uint32_t nnodes) {
+    return 7 * (size_t)nnodes + 8 + scan_temp_words((size_t)nnodes + 1);
+}
+
+namespace {
+struct WideWork { uint4* src; uint32_t *queue, *flag, *rank, *tail, *tmp; };
+WideWork wide_work(uint32_t* work, uint32_t nnodes) {
+    WideWork w;
+    const size_t n = nnodes;
+    w.src = reinterpret_cast<uint4*>(work);
+    w.queue = work + 4 * n;
+    w.flag = w.queue + n;
+    w.rank = w.flag + n + 1;
+    w.tail = w.rank + n + 1;
+    w.tmp = w.tail + 1;
+    return w;
+}
+}  // namespace
+
+int launch_wide_fold(void* stream, int sms, const uint32_t* nodes, uint32_t nnodes, uint32_t* work, uint32_t* nwide_out) {
+    cudaStream_t s = (cudaStream_t)stream;
+    const WideWork w = wide_work(work, nnodes);
+    const uint32_t one = 1;
+    cudaMemsetAsync(w.queue, 0, sizeof(uint32_t), s);   // the binary root
+    cudaMemsetAsync(w.flag, 0, ((size_t)nnodes + 1) * sizeof(uint32_t), s);
+    cudaMemcpyAsync(w.tail, &one, sizeof(uint32_t), cudaMemcpyHostToDevice, s);
+    uint32_t begin = 0, end = 1;
+    while (begin < end) {   // one level of wide nodes per pass; every binary node is a root at most once
+        k_wide_fold<<<grid(end - begin, sms), 256, 0, s>>>(nodes, w.queue, begin, end, w.src, w.flag, w.tail);
+        uint32_t tail = 0;
+        cudaMemcpyAsync(&tail, w.tail, sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
+        const cudaError_t e = cudaStreamSynchronize(s);
+        if (e != cudaSuccess) return (int)e;
+        begin = end;
+        end = tail;
+    }
+    scan(s, w.flag, w.rank, (size_t)nnodes + 1, w.tmp);
+    *nwide_out = end;
+    return (int)cudaGetLastError();
+}
+
+int launch_wide_emit(void* stream, int sms, const uint32_t* nodes, uint32_t nnodes, const uint32_t* work,
+                     uint32_t nwide, void* wide) {
+    const WideWork w = wide_work(const_cast<uint32_t*>(work), nnodes);
+    k_wide_emit<<<grid(nwide, sms), 256, 0, (cudaStream_t)stream>>>(nodes, w.queue, w.src, w.rank, nwide, (float*)wide);
+    return (int)cudaGetLastError();
+}
+
+int launch_wide_refit(void* stream, int sms, const uint32_t* nodes, uint32_t nwide, void* wide) {
+    k_wide_refit<<<grid(4 * (size_t)nwide, sms), 256, 0, (cudaStream_t)stream>>>(nodes, nwide, (float*)wide);
+    return (int)cudaGetLastError();
+}
 
 int launch_refit(void* stream, int sms, const void* vpos, const uint32_t* idx, uint32_t ntris, void* tris,
                  uint32_t* nodes, uint32_t nnodes, const uint32_t* parent, uint32_t* counts) {
