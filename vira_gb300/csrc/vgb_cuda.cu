@@ -71,6 +71,21 @@ using namespace vgbd;
 #ifndef VGB_SHADOW8_MINB
 #define VGB_SHADOW8_MINB 5
 #endif
+// k_front: 64-thread blocks resident per SM; 12 / 16 / 20 gave 2.86 / 2.76 / 2.80 ms at 512^2 x 16 spp
+// and 12.0 / 11.5 / 11.6 at 2048^2 x 4 spp.
+#ifndef VGB_FRONT_MINB
+#define VGB_FRONT_MINB 16
+#endif
+// Grids of the wavefront kernels after k_front, in 256-thread blocks per SM: their queues hold the
+// few paths that hit a second time (8 / 20 / 60: 2.756 / 2.760 / 2.791 ms at 512^2 x 16 spp).
+#ifndef VGB_LATE_GRID
+#define VGB_LATE_GRID 20
+#endif
+// State slots (pixels times samples in flight) of a chunk of a frame's samples: 2^22 took 12.5 ms for
+// 2048^2 x 4 spp, 2^23 11.5 (fewer launches over short queues); about 0.4 KB each at 8 bands.
+#ifndef VGB_CHUNK_SLOTS
+#define VGB_CHUNK_SLOTS (1u << 23)
+#endif
 // Grids of the wavefront kernels (grid-stride loops over the bounce's items), in blocks per SM;
 // 0 launches one 256-thread block per 256 items.  Many waves of short blocks let the block
 // scheduler even out rays of uneven cost: on the path-traced frame (2048^2 items) the closest-hit
@@ -201,6 +216,8 @@ struct DevState {
     float* as1;
     float* as2;
     uint32_t* anum;
+    float* pfh;          // [7][P] first-hit passes per sample slot (k_front; null unless requested)
+    float* acc;          // per-pixel sums between the chunks of a frame's samples (k_fold)
     uint32_t* counters;  // see C_* below
     uint64_t* stats;     // [0] nodes, [1] tris, [2] closest rays, [3] shadow rays
     size_t P;            // plane stride
@@ -210,12 +227,14 @@ struct DevState {
 // the persistent closest-hit and occlusion launches (reset with the shadow queues each bounce),
 // the error word and the batch kernels' work counter.
 enum {
-    C_PQ0 = 0, C_PQ1 = 1, C_SQ = 2, C_FTRACE = 2 + VGB_MAX_LIGHTS, C_FSHADOW = 3 + VGB_MAX_LIGHTS,
+    C_PQ0 = 0, C_SQ = 1, C_FTRACE = 1 + VGB_MAX_LIGHTS, C_FSHADOW = 2 + VGB_MAX_LIGHTS, C_PQ1 = 2 + 2 * VGB_MAX_LIGHTS,
     C_ERR = 3 + 2 * VGB_MAX_LIGHTS, C_BATCH = 4 + 2 * VGB_MAX_LIGHTS,
     C_COUNT
 };
-// counters cleared at the start of every bounce: the shadow queues and the persistent item counters
-constexpr int kBounceResetWords = 1 + 2 * VGB_MAX_LIGHTS;
+// Counters cleared at the start of every bounce: the shadow queues, the persistent item counters and
+// the output path queue's, which lie on either side of them (one memset).
+constexpr int kBounceResetWords = 2 + 2 * VGB_MAX_LIGHTS;
+__host__ __device__ __forceinline__ uint32_t path_count(uint32_t q) { return q ? C_PQ1 : C_PQ0; }
 
 struct FrameParams {
     vgb_camera cam;
@@ -227,6 +246,7 @@ struct FrameParams {
     uint32_t aux;   // AUX_* bits: the per-pixel sums the requested film planes need
     // first-hit film planes k_shade writes directly (null when not requested)
     float *vel_g, *vel_c, *tsz;
+    uint32_t npix;   // pixels of the frame: a state slot is (sample in flight) * npix + pixel
 };
 
 // Per-pixel sums kept over the samples only when a requested film plane reads them (the total
@@ -238,6 +258,9 @@ enum : uint32_t { AUX_ALB = 1u, AUX_NRM = 2u, AUX_DIR = 4u, AUX_DEP = 8u, AUX_TR
 // (0 nothing, 1 bounce-0 radiance, 2 a later bounce's), bit 2 set while the path radiance has
 // not been written this sample (it reads as 0).
 constexpr uint32_t kPendMask = 3u, kPradEmpty = 4u;
+// k_front's notes for k_fold in the same word: the camera ray hit, the path's second ray was traced,
+// and from bit 8 the shadow rays traced.
+constexpr uint32_t kPendHit = 8u, kPendRay1 = 16u, kPendShadow = 8u;
 
 struct FilmOut {
     float *total, *direct, *indirect, *power, *albedo, *normal, *depth, *alpha;
@@ -736,6 +759,17 @@ __device__ __noinline__ void first_hit_passes(const DevScene& s, const vgb_camer
     }
 }
 
+// Out-of-line traversal for the kernels that trace both ray kinds in one large body (k_front,
+// k_batch, the adjoint replay): one copy of the loop, called for closest-hit and occlusion rays, keeps
+// those kernels' instruction footprint small (instruction fetch was their leading stall; the
+// batch kernel ran 12 % and the adjoint 28 % faster than with both loops inlined).
+template <int L>
+__device__ __noinline__ void trace_ool(const DevScene& s, WRay r, float tmax, bool any, HitOut& h, uint32_t& err) {
+    Counters c{0, 0};
+    if (L == 8) traverse8_rt<false>(s.nodes, s.tris, r, tmax, any, h, err, c, s.iter_cap);
+    else traverse4_rt<false>(s.wide, s.tris, r, tmax, any, h, err, c, s.iter_cap);
+}
+
 // ------------------------------------------------------------------ k_trace (closest hit)
 // Scene::intersect for every live path: camera rays at bounce 0, queued continuation rays
 // after.  Writes one 16-byte hit record per queue item; kept lean so that enough warps are
@@ -745,7 +779,7 @@ template <int L, bool COUNT, bool B0>
 __global__ void __launch_bounds__(VGB_TRACE_BLOCK, (L == 8 ? VGB_TRACE8_MINB : VGB_TRACE_MINB) * 256 / VGB_TRACE_BLOCK) k_trace(const DevScene s, DevState st, const __grid_constant__ FrameParams fp,
                                                uint32_t bounce, uint32_t sample, uint32_t in_q, uint32_t n_items_bounce0) {
     const size_t P = st.P;
-    const uint32_t n_items = (B0) ? n_items_bounce0 : st.counters[in_q];
+    const uint32_t n_items = (B0) ? n_items_bounce0 : st.counters[path_count(in_q)];
     const uint32_t* in_queue = st.pq[in_q];
     uint32_t err = 0, nclosest = 0;
     Counters cnt{0, 0};
@@ -837,7 +871,7 @@ __global__ void __launch_bounds__(256, VGB_TRACEP_MINB) k_trace_p(const DevScene
                                                  uint32_t bounce, uint32_t sample, uint32_t in_q,
                                                  uint32_t n_items_bounce0, int budget, uint32_t refill) {
     const size_t P = st.P;
-    const uint32_t n_items = (bounce == 0) ? n_items_bounce0 : st.counters[in_q];
+    const uint32_t n_items = (bounce == 0) ? n_items_bounce0 : st.counters[path_count(in_q)];
     const uint32_t* in_queue = st.pq[in_q];
     const uint4* nodes = s.wide;
     const int lane = threadIdx.x & 31;
@@ -983,8 +1017,8 @@ __global__ void __launch_bounds__(VGB_SHADE_BLOCK, VGB_SHADE_MINB * 256 / VGB_SH
     const size_t P = st.P;
     const int lane = threadIdx.x & 31;
     const uint32_t stride = gridDim.x * blockDim.x;
-    const uint32_t n_items = (B0) ? n_items_bounce0 : st.counters[in_q];
-    uint32_t* out_count = &st.counters[(in_q ^ 1u)];
+    const uint32_t n_items = (B0) ? n_items_bounce0 : st.counters[path_count(in_q)];
+    uint32_t* out_count = &st.counters[path_count(in_q ^ 1u)];
     uint32_t* out_q = st.pq[in_q ^ 1u];
     const uint32_t* in_queue = st.pq[in_q];
     uint32_t nhits = 0;
@@ -998,9 +1032,11 @@ __global__ void __launch_bounds__(VGB_SHADE_BLOCK, VGB_SHADE_MINB * 256 / VGB_SH
         for (int k = 0; k < NB; ++k) thr[k] = 1.f;
         const uint32_t aux = fp.aux;
         uint32_t pendv = 0u;  // this item's fold state, written once below
+        uint32_t pix = 0, smp = sample, note = 0;
         if (active) {
             if (B0) {
                 active = camera_ray(fp, item, sample, slot, ro, rd);
+                pix = slot;
                 if (active && fp.opt.adaptive_sampling) {
                     if (sample == 0) { st.as1[slot] = 0.f; st.as2[slot] = 0.f; st.anum[slot] = 0u; }
                     else if (st.anum[slot]) active = false;  // the pixel has stopped sampling
@@ -1030,7 +1066,11 @@ __global__ void __launch_bounds__(VGB_SHADE_BLOCK, VGB_SHADE_MINB * 256 / VGB_SH
                 // the incoming ray stays in the path state; it is read below only for a miss.
                 // Fold the previous bounce's radiance into the path now, so that the path
                 // radiance is not live through the shading.
+                const uint32_t sl = slot / fp.npix;
+                pix = slot - sl * fp.npix;
+                smp = sample + sl;
                 const uint32_t pend = st.pend[slot];
+                note = pend & ~(kPendMask | kPradEmpty);
                 if (pend & kPendMask) {
 #pragma unroll
                     for (int k = 0; k < NB; ++k) {
@@ -1114,7 +1154,7 @@ __global__ void __launch_bounds__(VGB_SHADE_BLOCK, VGB_SHADE_MINB * 256 / VGB_SH
                         st.brad[k * P + slot] = (B0 && fp.opt.has_ambient) ? 0.f + thr[k] * (fp.opt.ambient[k] * alb[k]) : 0.f;
                 }
                 pendv = (pendv & kPradEmpty) | ((B0) ? 1u : 2u);
-                r0 = philox(U4{slot, sample, fp.opt.frame, (bounce << 8) | kSlotMain}, k0, k1);
+                r0 = philox(U4{pix, smp, fp.opt.frame, (bounce << 8) | kSlotMain}, k0, k1);
             }
         }
         // ---- NEE: one shadow ray per light, appended to that light's queue (warp ballot)
@@ -1127,7 +1167,7 @@ __global__ void __launch_bounds__(VGB_SHADE_BLOCK, VGB_SHADE_MINB * 256 / VGB_SH
                 float ru1, ru2;
                 if (l == 0) { ru1 = u01(r0.x); ru2 = u01(r0.y); }
                 else {
-                    U4 rl = philox(U4{slot, sample, fp.opt.frame, (bounce << 8) | (1u + l)}, k0, k1);
+                    U4 rl = philox(U4{pix, smp, fp.opt.frame, (bounce << 8) | (1u + l)}, k0, k1);
                     ru1 = u01(rl.x); ru2 = u01(rl.y);
                 }
                 pred = nee_light<NB>(fp.lights[l], Pp, N, alb, thr, nb, fp.opt.deterministic_light != 0, ru1, ru2, Ld,
@@ -1148,14 +1188,14 @@ __global__ void __launch_bounds__(VGB_SHADE_BLOCK, VGB_SHADE_MINB * 256 / VGB_SH
         bool new_ray = false;
         if (lit && bounce < fp.opt.bounces) {
             F3 nd;
-            cont = continue_path<NB>(fp.lights, fp.nlights, fp.opt, nb, Pp, N, tg, bt, nf, alb, thr, r0, slot, sample,
+            cont = continue_path<NB>(fp.lights, fp.nlights, fp.opt, nb, Pp, N, tg, bt, nf, alb, thr, r0, pix, smp,
                                      fp.opt.frame, bounce, nd, new_ray);
             if (new_ray) { ro = Pp; rd = nd; }
             // pdf 0: the reference keeps the incoming ray and throughput
         }
         // ---- write path state and append live paths
         if (active) {
-            st.pend[slot] = pendv;
+            st.pend[slot] = pendv | note;
             if (cont) {
 #pragma unroll
                 for (int k = 0; k < NB; ++k)
@@ -1206,13 +1246,41 @@ __global__ void __launch_bounds__(VGB_SHADOW_BLOCK, (L == 8 ? VGB_SHADOW8_MINB :
 }
 
 // ------------------------------------------------------------------ k_end_sample
+// A pixel's film values from its sums over the samples: unidirectional (cpu_path_tracer.ipp:229-240)
+// and RenderPasses::updateImages (passes.ipp:82-128).  dir(k), alb(k): the direct and albedo sums.
+template <int NB, typename Dir, typename Alb>
+__device__ __forceinline__ void film_pixel(const FrameParams& fp, const FilmOut& f, size_t p, const float* tot, float sf,
+                                           float dep, uint32_t count, uint32_t tri, F3 nsum, Dir&& dir, Alb&& alb) {
+    const size_t FP = fp.npix;   // plane stride of the caller's film
+#pragma unroll
+    for (int k = 0; k < NB; ++k) {
+        if (k < (int)fp.nb) {
+            const float total = tot[k] / sf;
+            if (f.total) f.total[k * FP + p] = total;
+            if (f.direct || f.indirect) {
+                const float direct = dir(k) / sf;
+                if (f.direct) f.direct[k * FP + p] = direct;
+                if (f.indirect) f.indirect[k * FP + p] = total - direct;
+            }
+            if (f.albedo) f.albedo[k * FP + p] = alb(k) / sf;
+            if (f.power) f.power[k * FP + p] = (fp.cam.power_scale[k] * f.omega[p]) * total;
+        }
+    }
+    if (f.normal) {
+        const F3 n = normalize(nsum);
+        f.normal[p] = n.x; f.normal[FP + p] = n.y; f.normal[2 * FP + p] = n.z;
+    }
+    if (f.depth) f.depth[p] = (count == 0) ? __int_as_float(0x7f800000) : dep / (float)count;
+    if (f.alpha) f.alpha[p] = (float)count / sf;
+    if (f.tri) f.tri[p] = tri;
+}
+
 template <int NB, bool ADAPTIVE>
 __global__ void __launch_bounds__(256) k_end_sample(DevState st, const __grid_constant__ FrameParams fp, uint32_t smp,
                                                     uint32_t last, FilmOut f) {
     const size_t P = st.P;                       // plane stride of the scratch state
     const uint32_t nb = fp.nb;
     const uint32_t npix = fp.cam.width * fp.cam.height;
-    const size_t FP = npix;                      // plane stride of the caller's film
     const float sf_all = (float)fp.opt.samples;
     const bool adaptive = ADAPTIVE;
     for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < npix; p += gridDim.x * blockDim.x) {
@@ -1268,30 +1336,260 @@ __global__ void __launch_bounds__(256) k_end_sample(DevState st, const __grid_co
             for (int k = 0; k < NB; ++k) tot[k] = (k < (int)nb) ? st.arad[k * P + p] : 0.f;
         }
         if (!last) continue;
-        // unidirectional (cpu_path_tracer.ipp:229-240) + RenderPasses::updateImages (passes.ipp:82-128);
         // a pixel that stopped early divides by the index of its last sample, as the reference does
         const float sf = stopped ? (float)stopped : sf_all;
-        const uint32_t count = (fp.aux & AUX_DEP) ? st.acnt[p] : 0u;
+        film_pixel<NB>(fp, f, p, tot, sf, (fp.aux & AUX_DEP) ? st.adep[p] : 0.f, (fp.aux & AUX_DEP) ? st.acnt[p] : 0u,
+                       (fp.aux & AUX_TRI) ? st.atri[p] : VGB_NO_HIT,
+                       f.normal ? F3{st.anrm[p], st.anrm[P + p], st.anrm[2 * P + p]} : F3{0.f, 0.f, 0.f},
+                       [&](int k) { return want_dir ? st.adir[k * P + p] : 0.f; },
+                       [&](int k) { return st.aalb[k * P + p]; });
+    }
+}
+
+// ------------------------------------------------------------------ k_front (camera ray to second hit)
+// One thread per (pixel, sample) of a chunk of a frame's samples, a warp per (8x4-pixel tile,
+// sample): the camera ray, its surface, the shadow ray of every light, the continuation and the
+// continuation's closest hit, with the path in registers throughout.  What the sample adds to the
+// film goes to the planes of its slot (sample in flight * npix + pixel), which k_fold sums in sample
+// order; only a path whose second ray hit writes a path state and joins the queue, and the wavefront
+// kernels take it from there at bounce 1.
+//
+// Against starting the path with k_trace, k_shade, k_shadow and k_trace a sample at a time this moves
+// no ray, hit or shadow queue through memory for the camera rays (all of them) and the paths that
+// leave the terrain after one bounce (most), and a launch covers enough samples to fill the GPU
+// whatever the frame's size.  Device time against the wavefront alone: 301 x 203 x 16 spp 4.09 -> 0.75
+// ms, 512^2 x 16 spp 7.38 -> 2.76 ms, 2048^2 x 4 spp 13.15 -> 11.5 ms, 1024^2 direct 0.355 -> 0.331 ms.
+// Bound by instruction issue and fetch (56 % of the issue slots, 20 of 32 threads an instruction).
+template <int NB>
+__global__ void __launch_bounds__(64, VGB_FRONT_MINB) k_front(const DevScene s, DevState st, const __grid_constant__ FrameParams fp,
+                                                  uint32_t sample0, uint32_t nsamples) {
+    const uint32_t nb = fp.nb;
+    const size_t P = st.P;
+    const int lane = threadIdx.x & 31;
+    const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const uint32_t tile = w / nsamples, sl = w - tile * nsamples, sample = sample0 + sl;
+    if (tile >= fp.tiles_x * fp.tiles_y) return;   // whole warps
+    const uint32_t tx = tile % fp.tiles_x, ty = tile / fp.tiles_x;
+    const uint32_t pi = tx * 8u + (lane & 7u), pj = ty * 4u + (lane >> 3);
+    const bool valid = pi < fp.cam.width && pj < fp.cam.height;
+    const uint32_t pix = valid ? pj * fp.cam.width + pi : 0u;
+    const size_t slot = (size_t)sl * fp.npix + pix;
+    const uint32_t k0 = (uint32_t)fp.opt.seed, k1 = (uint32_t)(fp.opt.seed >> 32);
+    uint32_t err = 0, note = kPradEmpty;
+    bool cont = false;
+    F3 ro{0.f, 0.f, 0.f}, rd{0.f, 0.f, 1.f};
+    float thr[NB], rad[NB];
+#pragma unroll
+    for (int k = 0; k < NB; ++k) { thr[k] = 1.f; rad[k] = 0.f; }
+    HitOut h;
+    h.id = VGB_NO_HIT;
+    if (valid) {
+        pixel_ray(fp.cam, pi, pj, pix, sample, fp.opt.frame, k0, k1, ro, rd);
+        h.U = h.V = h.W = 0.f; h.det = 1.f;
+        trace_ool<4>(s, make_wray(ro, rd), 0.f, false, h, err);
+        if (h.id == VGB_NO_HIT) {
+            if (fp.opt.simulate_lighting && fp.opt.show_background) {
+                const float4 bw = background_weights(rd);
+#pragma unroll
+                for (int k = 0; k < NB; ++k) {
+                    const float bgv = fp.opt.background[k];
+                    const float bg = ((bw.x * bgv + bw.y * bgv) + bw.z * bgv) + bw.w * bgv;
+                    rad[k] = 0.f + 1.f * (bg * 1.f);
+                }
+                note = 0u;
+            }
+            if (fp.aux & AUX_TRI) st.atri[slot] = VGB_NO_HIT;
+        } else {
+            const float rcp = 1.0f / h.det;
+            F3 Pp, N, fnrm, tg, bt, nf;
+            float alb[NB];
+            surface_at<NB>(s, nb, fp.opt.smooth_shading != 0, h.id, h.V * rcp, h.W * rcp, Pp, N, fnrm, tg, bt, nf, alb);
+            note |= kPendHit;
+            if (fp.aux & AUX_TRI) {
+                st.atri[slot] = h.id;
+                if (fp.tsz || fp.vel_g || fp.vel_c)
+                    first_hit_passes(s, fp.cam, h.id, Pp, fp.vel_g ? st.pfh : nullptr, fp.vel_c ? st.pfh + 3 * P : nullptr,
+                                     fp.tsz ? st.pfh + 6 * P : nullptr, P, (uint32_t)slot);
+            }
+            if (fp.aux & AUX_ALB) {
+#pragma unroll
+                for (int k = 0; k < NB; ++k) if (k < (int)nb) st.aalb[k * P + slot] = alb[k];
+            }
+            if (fp.aux & AUX_NRM) { st.anrm[slot] = N.x; st.anrm[P + slot] = N.y; st.anrm[2 * P + slot] = N.z; }
+            if (fp.aux & AUX_DEP) st.adep[slot] = h.t;
+            if (fp.opt.simulate_lighting) {
+                Pp = F3{offset1(Pp.x, fnrm.x), offset1(Pp.y, fnrm.y), offset1(Pp.z, fnrm.z)};
+                if (fp.opt.has_ambient) {
+#pragma unroll
+                    for (int k = 0; k < NB; ++k) if (k < (int)nb) rad[k] = 0.f + 1.f * (fp.opt.ambient[k] * alb[k]);
+                }
+                const U4 r0 = philox(U4{pix, sample, fp.opt.frame, kSlotMain}, k0, k1);
+                for (uint32_t l = 0; l < fp.nlights; ++l) {
+                    float ru1 = u01(r0.x), ru2 = u01(r0.y);
+                    if (l != 0) {
+                        const U4 rl = philox(U4{pix, sample, fp.opt.frame, 1u + l}, k0, k1);
+                        ru1 = u01(rl.x); ru2 = u01(rl.y);
+                    }
+                    F3 Ld;
+                    float dist, con[NB];
+                    if (!nee_light<NB>(fp.lights[l], Pp, N, alb, thr, nb, fp.opt.deterministic_light != 0, ru1, ru2, Ld, dist, con))
+                        continue;
+                    HitOut hs;
+                    trace_ool<4>(s, make_wray(Pp, Ld), dist, true, hs, err);
+                    note += 1u << kPendShadow;
+                    if (hs.id == VGB_NO_HIT) {
+#pragma unroll
+                        for (int k = 0; k < NB; ++k) if (k < (int)nb) rad[k] += con[k];
+                    }
+                }
+                if (fp.aux & AUX_DIR) {
+#pragma unroll
+                    for (int k = 0; k < NB; ++k) if (k < (int)nb) st.adir[k * P + slot] = rad[k];
+                }
+                note &= ~kPradEmpty;
+#pragma unroll
+                for (int k = 0; k < NB; ++k) rad[k] = 0.f + rad[k];
+                if (fp.opt.bounces != 0) {
+                    F3 nd;
+                    bool new_ray;
+                    cont = continue_path<NB>(fp.lights, fp.nlights, fp.opt, nb, Pp, N, tg, bt, nf, alb, thr, r0, pix, sample,
+                                             fp.opt.frame, 0u, nd, new_ray);
+                    if (new_ray) { ro = Pp; rd = nd; }   // pdf 0: the reference keeps the incoming ray and throughput
+                }
+            } else if (fp.aux & AUX_DIR) {
+#pragma unroll
+                for (int k = 0; k < NB; ++k) if (k < (int)nb) st.adir[k * P + slot] = 0.f;
+            }
+        }
+    }
+    h.id = VGB_NO_HIT;
+    if (cont) {
+        h.U = h.V = h.W = 0.f; h.det = 1.f;
+        trace_ool<4>(s, make_wray(ro, rd), 0.f, false, h, err);
+        note |= kPendRay1;
+        if (h.id == VGB_NO_HIT && fp.opt.show_background) {
+            const float4 bw = background_weights(rd);
+#pragma unroll
+            for (int k = 0; k < NB; ++k) {
+                const float bgv = fp.opt.background[k];
+                const float bg = ((bw.x * bgv + bw.y * bgv) + bw.z * bgv) + bw.w * bgv;
+                rad[k] = rad[k] + thr[k] * (bg * 1.f);
+            }
+        }
+    }
+    const bool live = h.id != VGB_NO_HIT;
+    const uint32_t qi = warp_append(&st.counters[C_PQ0], live);
+    if (live) {
+        const float rcp = 1.0f / h.det;
+        st.hit[qi] = make_float4(h.t, __uint_as_float(h.id), h.V * rcp, h.W * rcp);
+        st.pq[0][qi] = (uint32_t)slot;
+        st.org[slot] = ro.x; st.org[P + slot] = ro.y; st.org[2 * P + slot] = ro.z;
+        st.dir[slot] = rd.x; st.dir[P + slot] = rd.y; st.dir[2 * P + slot] = rd.z;
+#pragma unroll
+        for (int k = 0; k < NB; ++k) if (k < (int)nb) st.thr[k * P + slot] = thr[k];
+    }
+    if (valid) {
+        st.pend[slot] = note;
+        if (!(note & kPradEmpty)) {
+#pragma unroll
+            for (int k = 0; k < NB; ++k) if (k < (int)nb) st.prad[k * P + slot] = rad[k];
+        }
+    }
+    if (err) atomicOr(&st.counters[C_ERR], err);
+}
+
+// ------------------------------------------------------------------ k_fold
+// The chunk's samples of a pixel, summed in sample order (the reference's order, which the FP32
+// sums depend on) after the sums of the chunks before, and on the frame's last chunk the film.
+// Bound by HBM: it reads each slot's planes once.
+template <int NB>
+__global__ void __launch_bounds__(256, 3) k_fold(DevState st, const __grid_constant__ FrameParams fp, uint32_t nsamples,
+                                              uint32_t first, uint32_t last, FilmOut f) {
+    const size_t P = st.P;
+    const uint32_t nb = fp.nb, npix = fp.npix, aux = fp.aux;
+    const size_t A = npix;                 // plane stride of the sums: rad[B] dir[B] alb[B] nrm[3] dep cnt tri
+    uint32_t nclosest = 0, nshadow = 0, nhits = 0;
+    for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < npix; p += gridDim.x * blockDim.x) {
+        float tot[NB], dir[NB], alb[NB];
+        F3 ns{0.f, 0.f, 0.f};
+        float dep = 0.f;
+        uint32_t cnt = 0, tri = VGB_NO_HIT;
+#pragma unroll
+        for (int k = 0; k < NB; ++k) {
+            const bool on = !first && k < (int)nb;
+            tot[k] = on ? st.acc[k * A + p] : 0.f;
+            dir[k] = (on && (aux & AUX_DIR)) ? st.acc[(nb + k) * A + p] : 0.f;
+            alb[k] = (on && (aux & AUX_ALB)) ? st.acc[(2 * nb + k) * A + p] : 0.f;
+        }
+        const float* rest = st.acc + (size_t)3 * nb * A + p;
+        if (!first) {
+            if (aux & AUX_NRM) ns = F3{rest[0], rest[A], rest[2 * A]};
+            if (aux & AUX_DEP) { dep = rest[3 * A]; cnt = __float_as_uint(rest[4 * A]); }
+            if (aux & AUX_TRI) tri = __float_as_uint(rest[5 * A]);
+        }
+        bool fresh = first != 0;           // no chunk before wrote this pixel's first-hit passes
+        for (uint32_t sl = 0; sl < nsamples; ++sl) {
+            const size_t o = (size_t)sl * npix + p;
+            const uint32_t note = st.pend[o];
+            if (!(note & kPradEmpty)) {
+#pragma unroll
+                for (int k = 0; k < NB; ++k) {
+                    if (k < (int)nb) {
+                        float pr = st.prad[k * P + o];
+                        if (note & kPendMask) pr += st.brad[k * P + o];
+                        tot[k] = tot[k] + pr;
+                    }
+                }
+            }
+            nclosest += 1u + ((note & kPendRay1) ? 1u : 0u);
+            nshadow += note >> kPendShadow;
+            if (!(note & kPendHit)) continue;
+            nhits += 1u;
+            if (aux & AUX_DIR) {
+#pragma unroll
+                for (int k = 0; k < NB; ++k) if (k < (int)nb) dir[k] += st.adir[k * P + o];
+            }
+            if (aux & AUX_ALB) {
+#pragma unroll
+                for (int k = 0; k < NB; ++k) if (k < (int)nb) alb[k] += st.aalb[k * P + o];
+            }
+            if (aux & AUX_NRM) { ns.x += st.anrm[o]; ns.y += st.anrm[P + o]; ns.z += st.anrm[2 * P + o]; }
+            if (aux & AUX_DEP) { dep += st.adep[o]; cnt += 1u; }
+            if ((aux & AUX_TRI) && tri == VGB_NO_HIT) {
+                tri = st.atri[o];
+                fresh = false;
+                if (fp.vel_g) for (int c = 0; c < 3; ++c) fp.vel_g[c * A + p] = st.pfh[c * P + o];
+                if (fp.vel_c) for (int c = 0; c < 3; ++c) fp.vel_c[c * A + p] = st.pfh[(3 + c) * P + o];
+                if (fp.tsz) fp.tsz[p] = st.pfh[6 * P + o];
+            }
+        }
+        if (fresh) {
+            if (fp.tsz) fp.tsz[p] = __int_as_float(0x7f800000);
+            if (fp.vel_g) for (int c = 0; c < 3; ++c) fp.vel_g[c * A + p] = 0.f;
+            if (fp.vel_c) for (int c = 0; c < 3; ++c) fp.vel_c[c * A + p] = 0.f;
+        }
+        if (last) {
+            film_pixel<NB>(fp, f, p, tot, (float)fp.opt.samples, dep, cnt, tri, ns, [&](int k) { return dir[k]; },
+                           [&](int k) { return alb[k]; });
+            continue;
+        }
+        float* out = st.acc + p;
 #pragma unroll
         for (int k = 0; k < NB; ++k) {
             if (k < (int)nb) {
-                const float total = tot[k] / sf;
-                const float direct = want_dir ? st.adir[k * P + p] / sf : 0.f;
-                if (f.total) f.total[k * FP + p] = total;
-                if (f.direct) f.direct[k * FP + p] = direct;
-                if (f.indirect) f.indirect[k * FP + p] = total - direct;
-                if (f.albedo) f.albedo[k * FP + p] = st.aalb[k * P + p] / sf;
-                if (f.power) f.power[k * FP + p] = (fp.cam.power_scale[k] * f.omega[p]) * total;
+                out[k * A] = tot[k];
+                if (aux & AUX_DIR) out[(nb + k) * A] = dir[k];
+                if (aux & AUX_ALB) out[(2 * nb + k) * A] = alb[k];
             }
         }
-        if (f.normal) {
-            F3 n = normalize(F3{st.anrm[p], st.anrm[P + p], st.anrm[2 * P + p]});
-            f.normal[p] = n.x; f.normal[FP + p] = n.y; f.normal[2 * FP + p] = n.z;
-        }
-        if (f.depth) f.depth[p] = (count == 0) ? __int_as_float(0x7f800000) : st.adep[p] / (float)count;
-        if (f.alpha) f.alpha[p] = (float)count / sf;
-        if (f.tri) f.tri[p] = st.atri[p];
+        out += (size_t)3 * nb * A;
+        if (aux & AUX_NRM) { out[0] = ns.x; out[A] = ns.y; out[2 * A] = ns.z; }
+        if (aux & AUX_DEP) { out[3 * A] = dep; out[4 * A] = __uint_as_float(cnt); }
+        if (aux & AUX_TRI) out[5 * A] = __uint_as_float(tri);
     }
+    warp_reduce_add(&st.stats[2], nclosest);
+    warp_reduce_add(&st.stats[3], nshadow);
+    warp_reduce_add(&st.stats[6], nhits);
 }
 
 // ------------------------------------------------------------------ pixel solid angle (FP64)
@@ -1413,7 +1711,8 @@ struct vgb_context {
     bool h_pos_stale = false;       // device positions moved by a device-side update
     uint32_t* d_vnl = nullptr;      // per-vertex corner lists of the uploaded mesh (vertex-normal updates)
     // render scratch
-    size_t cap_P = 0, cap_items = 0;
+    size_t cap_P = 0, cap_items = 0, cap_npix = 0;
+    bool cap_fh = false;
     uint32_t cap_B = 0, cap_L = 0;
     std::vector<void*> scratch;
     DevState st{};
@@ -1506,7 +1805,7 @@ void free_bvh(vgb_context* ctx) {
 void free_scratch(vgb_context* ctx) {
     for (void* p : ctx->scratch) dfree(p);
     ctx->scratch.clear();
-    ctx->cap_P = 0; ctx->cap_items = 0; ctx->cap_B = 0; ctx->cap_L = 0;
+    ctx->cap_P = 0; ctx->cap_items = 0; ctx->cap_npix = 0; ctx->cap_B = 0; ctx->cap_L = 0; ctx->cap_fh = false;
 }
 void free_staging(vgb_context* ctx) {
     dfree(ctx->staging_base);
@@ -1535,12 +1834,18 @@ vgb_status ensure_staging(vgb_context* ctx, size_t bytes) {
     return VGB_OK;
 }
 
-// Scratch for a frame of P pixels whose bounce-0 launch covers n_items queue items (the frame
-// rounded up to whole 8x4-pixel tiles, so n_items >= P): the hit records of bounce 0 are indexed
-// by item, every other plane by pixel or by a queue position below P.
-vgb_status ensure_scratch(vgb_context* ctx, size_t P, size_t n_items, uint32_t B, uint32_t L) {
-    if (P <= ctx->cap_P && n_items <= ctx->cap_items && B <= ctx->cap_B && L <= ctx->cap_L) return VGB_OK;
+// Scratch for P state slots (pixels times samples in flight) of a frame of npix pixels whose
+// bounce-0 launch covers n_items queue items (the frame rounded up to whole 8x4-pixel tiles, so
+// n_items >= P where the wavefront starts the camera rays): the hit records of bounce 0 are indexed
+// by item, the planes kept from sample to sample by pixel, every other plane by slot or by a queue
+// position below P.
+vgb_status ensure_scratch(vgb_context* ctx, size_t P, size_t n_items, size_t npix, uint32_t B, uint32_t L, bool first_hit) {
+    if (P <= ctx->cap_P && n_items <= ctx->cap_items && npix <= ctx->cap_npix && B <= ctx->cap_B && L <= ctx->cap_L &&
+        first_hit <= ctx->cap_fh)
+        return VGB_OK;
     P = std::max(P, ctx->cap_P);
+    npix = std::max(npix, ctx->cap_npix);
+    first_hit = first_hit || ctx->cap_fh;
     n_items = std::max(std::max(n_items, P), ctx->cap_items);
     B = std::max(B, ctx->cap_B);
     L = std::max(L, ctx->cap_L);
@@ -1556,11 +1861,15 @@ vgb_status ensure_scratch(vgb_context* ctx, size_t P, size_t n_items, uint32_t B
 #define AL(ptr, n) do { s = A(&(ptr), (n)); if (s != VGB_OK) { free_scratch(ctx); return s; } } while (0)
     AL(st.org, 3 * P * f); AL(st.dir, 3 * P * f); AL(st.thr, B * P * f); AL(st.prad, B * P * f);
     AL(st.brad, B * P * f); AL(st.pend, P * u);
-    AL(st.arad, B * P * f); AL(st.adir, B * P * f); AL(st.aalb, B * P * f); AL(st.anrm, 3 * P * f);
+    AL(st.adir, B * P * f); AL(st.aalb, B * P * f); AL(st.anrm, 3 * P * f);
     AL(st.adep, P * f); AL(st.acnt, P * u); AL(st.atri, P * u);
+    AL(st.acc, (3 * (size_t)B + 6) * npix * f);
+    st.arad = st.acc;
+    st.pfh = nullptr;
+    if (first_hit) AL(st.pfh, 7 * P * f);
     AL(st.pq[0], P * u); AL(st.pq[1], P * u);
     AL(st.hit, n_items * sizeof(float4));
-    AL(st.as1, P * f); AL(st.as2, P * f); AL(st.anum, P * u);
+    AL(st.as1, npix * f); AL(st.as2, npix * f); AL(st.anum, npix * u);
     for (uint32_t l = 0; l < VGB_MAX_LIGHTS; ++l) {
         if (l < L) {
             AL(st.sq_org[l], 3 * P * f); AL(st.sq_dir[l], 3 * P * f); AL(st.sq_tmax[l], P * f);
@@ -1573,7 +1882,7 @@ vgb_status ensure_scratch(vgb_context* ctx, size_t P, size_t n_items, uint32_t B
     st.counters = ctx->d_counters;
     st.stats = ctx->d_stats;
     st.P = P;
-    ctx->cap_P = P; ctx->cap_items = n_items; ctx->cap_B = B; ctx->cap_L = L;
+    ctx->cap_P = P; ctx->cap_items = n_items; ctx->cap_npix = npix; ctx->cap_B = B; ctx->cap_L = L; ctx->cap_fh = first_hit;
     return VGB_OK;
 }
 
@@ -1633,6 +1942,14 @@ inline bool frame_fits(uint32_t W, uint32_t H) {
     return W != 0 && H != 0 && (uint64_t)W * H <= (1ull << 31) && tile_items(W, H) <= (1ull << 31);
 }
 
+// Samples of a frame of P pixels in flight at a time: as many as fit VGB_CHUNK_SLOTS state slots,
+// in chunks of even size.
+inline uint32_t chunk_samples(size_t P, uint32_t samples) {
+    const uint32_t most = (uint32_t)std::max<size_t>(1, VGB_CHUNK_SLOTS / P);
+    const uint32_t chunks = (uint32_t)(((uint64_t)samples + most - 1) / most);
+    return (samples + chunks - 1) / chunks;
+}
+
 // The render's launch sequence (per sample: per bounce k_trace, k_shade, k_shadow per light;
 // then k_end_sample) over the scratch `st`.  vgb_render passes the context's scratch,
 // vgb_render_noalloc the fixed array; `prof` allows CUDA-event profiling of the launches.
@@ -1642,6 +1959,55 @@ int resident_grid(const vgb_context* ctx, K kernel) {
     int per_sm = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 256, 0) != cudaSuccess || per_sm < 1) per_sm = 1;
     return per_sm * ctx->num_sms;
+}
+
+inline void reset_bounce_counters(const DevState& st, uint32_t out_q, cudaStream_t stream) {
+    cudaMemsetAsync(&st.counters[out_q ? C_SQ : C_PQ0], 0, sizeof(uint32_t) * kBounceResetWords, stream);
+}
+
+// The render in chunks of `chunk` samples: k_front, the wavefront kernels over the paths that hit a
+// second time, k_fold.  st.P is the chunk's slots.
+template <int NB>
+void launch_chunks(vgb_context* ctx, const FrameParams& fp, const FilmOut& film, const DevState& st, uint32_t chunk,
+                   bool prof, uint32_t& launches) {
+    const DevScene s = dev_scene(ctx);
+    const size_t tiles = (size_t)fp.tiles_x * fp.tiles_y;
+    const int gp = grid_for(ctx, fp.npix, VGB_END_GRID);
+    for (uint32_t s0 = 0; s0 < fp.opt.samples; s0 += chunk) {
+        const uint32_t n = std::min(chunk, fp.opt.samples - s0);
+        const size_t items = tiles * n * 32;
+        cudaMemsetAsync(&st.counters[C_PQ0], 0, sizeof(uint32_t), ctx->stream);
+        {
+            Prof p(ctx, 0, prof);
+            k_front<NB><<<(unsigned)((items + 63) / 64), 64, 0, ctx->stream>>>(s, st, fp, s0, n);
+        }
+        launches++;
+        const int gt = grid_for(ctx, items, VGB_LATE_GRID * 256 / VGB_TRACE_BLOCK, VGB_TRACE_BLOCK);
+        const int gs = grid_for(ctx, items, VGB_LATE_GRID, VGB_SHADE_BLOCK);
+        uint32_t q = 0;
+        for (uint32_t b = 1; b <= fp.opt.bounces; ++b) {
+            reset_bounce_counters(st, q ^ 1u, ctx->stream);
+            if (b > 1) {
+                Prof p(ctx, 0, prof);
+                k_trace<4, false, false><<<gt, VGB_TRACE_BLOCK, 0, ctx->stream>>>(s, st, fp, b, s0, q, 0u);
+                launches++;
+            }
+            {
+                Prof p(ctx, 3, prof);
+                k_shade<NB, false><<<gs, VGB_SHADE_BLOCK, 0, ctx->stream>>>(s, st, fp, b, s0, q, 0u);
+            }
+            launches++;
+            for (uint32_t l = 0; l < fp.nlights; ++l) {
+                Prof p(ctx, 1, prof);
+                k_shadow<NB, 4, false><<<gt, VGB_SHADOW_BLOCK, 0, ctx->stream>>>(s, st, l, fp.nb);
+                launches++;
+            }
+            q ^= 1u;
+        }
+        Prof p(ctx, 2, prof);
+        k_fold<NB><<<gp, 256, 0, ctx->stream>>>(st, fp, n, s0 == 0 ? 1u : 0u, s0 + n == fp.opt.samples ? 1u : 0u, film);
+        launches++;
+    }
 }
 
 template <int NB, int L, bool COUNT>
@@ -1673,9 +2039,7 @@ void launch_render(vgb_context* ctx, const FrameParams& fp, const FilmOut& film,
     for (uint32_t smp = 0; smp < fp.opt.samples; ++smp) {
         uint32_t q = 0;
         for (uint32_t b = 0; b <= fp.opt.bounces; ++b) {
-            // reset the output path queue, the shadow queues and the persistent item counters
-            cudaMemsetAsync(&st.counters[(q ^ 1u)], 0, sizeof(uint32_t), ctx->stream);
-            cudaMemsetAsync(&st.counters[C_SQ], 0, sizeof(uint32_t) * kBounceResetWords, ctx->stream);
+            reset_bounce_counters(st, q ^ 1u, ctx->stream);
             {
                 Prof p(ctx, 0, prof);
                 if (persist) k_trace_p<COUNT><<<gtp, 256, 0, ctx->stream>>>(s, st, fp, b, smp, q, n0, budget, refill);
@@ -3122,7 +3486,20 @@ VGB_API vgb_status vgb_render(vgb_context* ctx, const vgb_camera* cam, const vgb
     cudaSetDevice(ctx->device);
     const size_t P = (size_t)cam->width * cam->height;
     const uint32_t B = ctx->nbands;
-    vgb_status s = ensure_scratch(ctx, P, tile_items(cam->width, cam->height), B, std::max<uint32_t>(1, nlights));
+    // Samples in flight.  The wavefront kernels alone (chunk 0) take what k_front does not do: adaptive
+    // sampling, whose next sample depends on the last, the 8-wide layout, the persistent traversal
+    // and the counting pass, which needs counted traversals.
+    const bool fused = !opts->adaptive_sampling && ctx->bvh_layout == 2 && !ctx->trav_persistent;
+    const uint32_t nq = std::max<uint32_t>(1, nlights);
+    const bool first_hit = film->velocity_global || film->velocity_camera || film->triangle_size;
+    uint32_t chunk = fused ? chunk_samples(P, opts->samples) : 0u;
+    vgb_status s;
+    do {
+        const size_t items = (chunk && !ctx->count_pass) ? chunk * P : tile_items(cam->width, cam->height);
+        s = ensure_scratch(ctx, std::max<size_t>(chunk, 1) * P, items, P, B, nq, chunk && first_hit);
+        if (s != VGB_ERR_OUT_OF_MEMORY || chunk <= 1) break;
+        chunk = chunk / 2;   // no memory for that many samples at a time
+    } while (true);
     if (s != VGB_OK) return s;
     FrameParams fp;
     std::memset(&fp, 0, sizeof(fp));
@@ -3133,6 +3510,8 @@ VGB_API vgb_status vgb_render(vgb_context* ctx, const vgb_camera* cam, const vgb
     fp.nb = B;
     fp.tiles_x = (cam->width + 7) / 8;
     fp.tiles_y = (cam->height + 3) / 4;
+    fp.npix = (uint32_t)P;
+    DevState st = ctx->st;
     // film planes: device pointers as given, or staging buffers for host films
     FilmOut f{};
     struct Plane { float** host_f; uint32_t** host_u; size_t n; };
@@ -3207,7 +3586,14 @@ VGB_API vgb_status vgb_render(vgb_context* ctx, const vgb_camera* cam, const vgb
     uint32_t launches = 0;
     ctx->prof_used = 0;
     CK(cudaEventRecord(ctx->ev0, ctx->stream));
-    dispatch_render<false>(ctx, fp, fr, ctx->st, true, launches);
+    st.P = std::max<size_t>(chunk, 1) * P;
+    if (chunk) {
+        if (fp.nb <= 1) launch_chunks<1>(ctx, fp, fr, st, chunk, true, launches);
+        else if (fp.nb <= 4) launch_chunks<4>(ctx, fp, fr, st, chunk, true, launches);
+        else launch_chunks<8>(ctx, fp, fr, st, chunk, true, launches);
+    } else {
+        dispatch_render<false>(ctx, fp, fr, st, true, launches);
+    }
     if (dn_scratch) {
         PowerScale ps{};
         for (uint32_t k = 0; k < B && k < VGB_MAX_BANDS; ++k) ps.v[k] = cam->power_scale[k];
@@ -3257,7 +3643,8 @@ VGB_API vgb_status vgb_render(vgb_context* ctx, const vgb_camera* cam, const vgb
         none.power = nullptr;
         CK(cudaMemsetAsync(ctx->d_stats, 0, sizeof(uint64_t) * 8, ctx->stream));
         uint32_t l2 = 0;
-        dispatch_render<true>(ctx, fp, none, ctx->st, false, l2);
+        st.P = P;
+        dispatch_render<true>(ctx, fp, none, st, false, l2);
         CK(cudaGetLastError());
         CK(cudaStreamSynchronize(ctx->stream));
         CK(cudaMemcpy(hs, ctx->d_stats, sizeof(hs), cudaMemcpyDeviceToHost));
@@ -3457,6 +3844,7 @@ extern "C" VGB_API vgb_status vgb_render_noalloc(vgb_context* ctx, const vgb_cam
     fp.nb = B;
     fp.tiles_x = (cam->width + 7) / 8;
     fp.tiles_y = (cam->height + 3) / 4;
+    fp.npix = (uint32_t)P;
     FilmOut fo{};
     fo.total = film->total_radiance; fo.direct = film->direct_radiance; fo.indirect = film->indirect_radiance;
     fo.power = film->received_power; fo.albedo = film->albedo; fo.normal = film->normal_global;
@@ -3502,17 +3890,6 @@ extern "C" VGB_API vgb_status vgb_render_noalloc(vgb_context* ctx, const vgb_cam
     return vgb::status_of_exception(ctx ? &ctx->err : nullptr);
 }
 
-
-// Out-of-line traversal for the kernels that trace both ray kinds in one large body (k_batch,
-// the adjoint replay): one copy of the loop, called for closest-hit and occlusion rays, keeps
-// those kernels' instruction footprint small (instruction fetch was their leading stall; the
-// batch kernel ran 12 % and the adjoint 28 % faster than with both loops inlined).
-template <int L>
-__device__ __noinline__ void trace_ool(const DevScene& s, WRay r, float tmax, bool any, HitOut& h, uint32_t& err) {
-    Counters c{0, 0};
-    if (L == 8) traverse8_rt<false>(s.nodes, s.tris, r, tmax, any, h, err, c, s.iter_cap);
-    else traverse4_rt<false>(s.wide, s.tris, r, tmax, any, h, err, c, s.iter_cap);
-}
 
 // ====================================================================== batched trajectory
 namespace {
