@@ -81,10 +81,16 @@ using namespace vgbd;
 #ifndef VGB_LATE_GRID
 #define VGB_LATE_GRID 20
 #endif
-// State slots (pixels times samples in flight) of a chunk of a frame's samples: 2^22 took 12.5 ms for
-// 2048^2 x 4 spp, 2^23 11.5 (fewer launches over short queues); about 0.4 KB each at 8 bands.
+// k_fold: 256-thread blocks per SM and band (8 / 16 / 60: 81 / 98 / 125 us at 1024^2, 4 bands; more
+// blocks only add DRAM streams).
+#ifndef VGB_FOLD_GRID
+#define VGB_FOLD_GRID 8
+#endif
+// State slots (pixels times samples in flight) of a chunk of a frame's samples: 2048^2 x 4 spp takes
+// 12.5 ms at 2^22, 11.1 at 2^23 and 10.1 at 2^24 (fewer launches over short queues, and the sums of a
+// single chunk stay in registers); about 0.3 KB each at 8 bands.
 #ifndef VGB_CHUNK_SLOTS
-#define VGB_CHUNK_SLOTS (1u << 23)
+#define VGB_CHUNK_SLOTS (1u << 24)
 #endif
 // Grids of the wavefront kernels (grid-stride loops over the bounce's items), in blocks per SM;
 // 0 launches one 256-thread block per 256 items.  Many waves of short blocks let the block
@@ -1247,25 +1253,23 @@ __global__ void __launch_bounds__(VGB_SHADOW_BLOCK, (L == 8 ? VGB_SHADOW8_MINB :
 
 // ------------------------------------------------------------------ k_end_sample
 // A pixel's film values from its sums over the samples: unidirectional (cpu_path_tracer.ipp:229-240)
-// and RenderPasses::updateImages (passes.ipp:82-128).  dir(k), alb(k): the direct and albedo sums.
-template <int NB, typename Dir, typename Alb>
-__device__ __forceinline__ void film_pixel(const FrameParams& fp, const FilmOut& f, size_t p, const float* tot, float sf,
-                                           float dep, uint32_t count, uint32_t tri, F3 nsum, Dir&& dir, Alb&& alb) {
+// and RenderPasses::updateImages (passes.ipp:82-128).  One band, and the planes without bands.
+__device__ __forceinline__ void film_band(const FrameParams& fp, const FilmOut& f, size_t p, uint32_t k, float tot,
+                                          float dir, float alb, float sf) {
     const size_t FP = fp.npix;   // plane stride of the caller's film
-#pragma unroll
-    for (int k = 0; k < NB; ++k) {
-        if (k < (int)fp.nb) {
-            const float total = tot[k] / sf;
-            if (f.total) f.total[k * FP + p] = total;
-            if (f.direct || f.indirect) {
-                const float direct = dir(k) / sf;
-                if (f.direct) f.direct[k * FP + p] = direct;
-                if (f.indirect) f.indirect[k * FP + p] = total - direct;
-            }
-            if (f.albedo) f.albedo[k * FP + p] = alb(k) / sf;
-            if (f.power) f.power[k * FP + p] = (fp.cam.power_scale[k] * f.omega[p]) * total;
-        }
+    const float total = tot / sf;
+    if (f.total) f.total[k * FP + p] = total;
+    if (f.direct || f.indirect) {
+        const float direct = dir / sf;
+        if (f.direct) f.direct[k * FP + p] = direct;
+        if (f.indirect) f.indirect[k * FP + p] = total - direct;
     }
+    if (f.albedo) f.albedo[k * FP + p] = alb / sf;
+    if (f.power) f.power[k * FP + p] = (fp.cam.power_scale[k] * f.omega[p]) * total;
+}
+__device__ __forceinline__ void film_rest(const FrameParams& fp, const FilmOut& f, size_t p, float sf, float dep,
+                                          uint32_t count, uint32_t tri, F3 nsum) {
+    const size_t FP = fp.npix;
     if (f.normal) {
         const F3 n = normalize(nsum);
         f.normal[p] = n.x; f.normal[FP + p] = n.y; f.normal[2 * FP + p] = n.z;
@@ -1338,11 +1342,14 @@ __global__ void __launch_bounds__(256) k_end_sample(DevState st, const __grid_co
         if (!last) continue;
         // a pixel that stopped early divides by the index of its last sample, as the reference does
         const float sf = stopped ? (float)stopped : sf_all;
-        film_pixel<NB>(fp, f, p, tot, sf, (fp.aux & AUX_DEP) ? st.adep[p] : 0.f, (fp.aux & AUX_DEP) ? st.acnt[p] : 0u,
-                       (fp.aux & AUX_TRI) ? st.atri[p] : VGB_NO_HIT,
-                       f.normal ? F3{st.anrm[p], st.anrm[P + p], st.anrm[2 * P + p]} : F3{0.f, 0.f, 0.f},
-                       [&](int k) { return want_dir ? st.adir[k * P + p] : 0.f; },
-                       [&](int k) { return st.aalb[k * P + p]; });
+#pragma unroll
+        for (int k = 0; k < NB; ++k)
+            if (k < (int)nb)
+                film_band(fp, f, p, k, tot[k], want_dir ? st.adir[k * P + p] : 0.f,
+                          (fp.aux & AUX_ALB) ? st.aalb[k * P + p] : 0.f, sf);
+        film_rest(fp, f, p, sf, (fp.aux & AUX_DEP) ? st.adep[p] : 0.f, (fp.aux & AUX_DEP) ? st.acnt[p] : 0u,
+                  (fp.aux & AUX_TRI) ? st.atri[p] : VGB_NO_HIT,
+                  f.normal ? F3{st.anrm[p], st.anrm[P + p], st.anrm[2 * P + p]} : F3{0.f, 0.f, 0.f});
     }
 }
 
@@ -1501,58 +1508,64 @@ __global__ void __launch_bounds__(64, VGB_FRONT_MINB) k_front(const DevScene s, 
 // ------------------------------------------------------------------ k_fold
 // The chunk's samples of a pixel, summed in sample order (the reference's order, which the FP32
 // sums depend on) after the sums of the chunks before, and on the frame's last chunk the film.
-// Bound by HBM: it reads each slot's planes once.
-template <int NB>
-__global__ void __launch_bounds__(256, 3) k_fold(DevState st, const __grid_constant__ FrameParams fp, uint32_t nsamples,
+// blockIdx.y: a band, or after the last one the planes without bands.  Bound by HBM latency: one
+// thread per (pixel, band) keeps (bands + 1) times the loads in flight of a thread per pixel.
+__global__ void __launch_bounds__(256) k_fold(DevState st, const __grid_constant__ FrameParams fp, uint32_t nsamples,
                                               uint32_t first, uint32_t last, FilmOut f) {
     const size_t P = st.P;
-    const uint32_t nb = fp.nb, npix = fp.npix, aux = fp.aux;
+    const uint32_t nb = fp.nb, npix = fp.npix, aux = fp.aux, k = blockIdx.y;
     const size_t A = npix;                 // plane stride of the sums: rad[B] dir[B] alb[B] nrm[3] dep cnt tri
+    const float sf = (float)fp.opt.samples;
+    const bool want_dir = (aux & AUX_DIR) != 0, want_alb = (aux & AUX_ALB) != 0;
+    if (k < nb) {
+        const float* prad = st.prad + k * P;
+        const float* brad = st.brad + k * P;
+        const float* adir = st.adir + k * P;
+        const float* aalb = st.aalb + k * P;
+        for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < npix; p += gridDim.x * blockDim.x) {
+            float tot = first ? 0.f : st.acc[k * A + p];
+            float dir = (first || !want_dir) ? 0.f : st.acc[(nb + k) * A + p];
+            float alb = (first || !want_alb) ? 0.f : st.acc[(2 * nb + k) * A + p];
+#pragma unroll 4
+            for (uint32_t sl = 0; sl < nsamples; ++sl) {
+                const size_t o = (size_t)sl * npix + p;
+                const uint32_t note = st.pend[o];
+                float pr = prad[o];
+                const float d = want_dir ? adir[o] : 0.f, a = want_alb ? aalb[o] : 0.f;
+                if (note & kPendMask) pr += brad[o];
+                if (!(note & kPradEmpty)) tot = tot + pr;
+                if (note & kPendHit) { dir += d; alb += a; }
+            }
+            if (!last) {
+                st.acc[k * A + p] = tot;
+                if (want_dir) st.acc[(nb + k) * A + p] = dir;
+                if (want_alb) st.acc[(2 * nb + k) * A + p] = alb;
+                continue;
+            }
+            film_band(fp, f, p, k, tot, dir, alb, sf);
+        }
+        return;
+    }
     uint32_t nclosest = 0, nshadow = 0, nhits = 0;
     for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < npix; p += gridDim.x * blockDim.x) {
-        float tot[NB], dir[NB], alb[NB];
         F3 ns{0.f, 0.f, 0.f};
         float dep = 0.f;
         uint32_t cnt = 0, tri = VGB_NO_HIT;
-#pragma unroll
-        for (int k = 0; k < NB; ++k) {
-            const bool on = !first && k < (int)nb;
-            tot[k] = on ? st.acc[k * A + p] : 0.f;
-            dir[k] = (on && (aux & AUX_DIR)) ? st.acc[(nb + k) * A + p] : 0.f;
-            alb[k] = (on && (aux & AUX_ALB)) ? st.acc[(2 * nb + k) * A + p] : 0.f;
-        }
-        const float* rest = st.acc + (size_t)3 * nb * A + p;
+        float* rest = st.acc + (size_t)3 * nb * A + p;
         if (!first) {
             if (aux & AUX_NRM) ns = F3{rest[0], rest[A], rest[2 * A]};
             if (aux & AUX_DEP) { dep = rest[3 * A]; cnt = __float_as_uint(rest[4 * A]); }
             if (aux & AUX_TRI) tri = __float_as_uint(rest[5 * A]);
         }
         bool fresh = first != 0;           // no chunk before wrote this pixel's first-hit passes
+#pragma unroll 2
         for (uint32_t sl = 0; sl < nsamples; ++sl) {
             const size_t o = (size_t)sl * npix + p;
             const uint32_t note = st.pend[o];
-            if (!(note & kPradEmpty)) {
-#pragma unroll
-                for (int k = 0; k < NB; ++k) {
-                    if (k < (int)nb) {
-                        float pr = st.prad[k * P + o];
-                        if (note & kPendMask) pr += st.brad[k * P + o];
-                        tot[k] = tot[k] + pr;
-                    }
-                }
-            }
             nclosest += 1u + ((note & kPendRay1) ? 1u : 0u);
             nshadow += note >> kPendShadow;
             if (!(note & kPendHit)) continue;
             nhits += 1u;
-            if (aux & AUX_DIR) {
-#pragma unroll
-                for (int k = 0; k < NB; ++k) if (k < (int)nb) dir[k] += st.adir[k * P + o];
-            }
-            if (aux & AUX_ALB) {
-#pragma unroll
-                for (int k = 0; k < NB; ++k) if (k < (int)nb) alb[k] += st.aalb[k * P + o];
-            }
             if (aux & AUX_NRM) { ns.x += st.anrm[o]; ns.y += st.anrm[P + o]; ns.z += st.anrm[2 * P + o]; }
             if (aux & AUX_DEP) { dep += st.adep[o]; cnt += 1u; }
             if ((aux & AUX_TRI) && tri == VGB_NO_HIT) {
@@ -1568,24 +1581,13 @@ __global__ void __launch_bounds__(256, 3) k_fold(DevState st, const __grid_const
             if (fp.vel_g) for (int c = 0; c < 3; ++c) fp.vel_g[c * A + p] = 0.f;
             if (fp.vel_c) for (int c = 0; c < 3; ++c) fp.vel_c[c * A + p] = 0.f;
         }
-        if (last) {
-            film_pixel<NB>(fp, f, p, tot, (float)fp.opt.samples, dep, cnt, tri, ns, [&](int k) { return dir[k]; },
-                           [&](int k) { return alb[k]; });
+        if (!last) {
+            if (aux & AUX_NRM) { rest[0] = ns.x; rest[A] = ns.y; rest[2 * A] = ns.z; }
+            if (aux & AUX_DEP) { rest[3 * A] = dep; rest[4 * A] = __uint_as_float(cnt); }
+            if (aux & AUX_TRI) rest[5 * A] = __uint_as_float(tri);
             continue;
         }
-        float* out = st.acc + p;
-#pragma unroll
-        for (int k = 0; k < NB; ++k) {
-            if (k < (int)nb) {
-                out[k * A] = tot[k];
-                if (aux & AUX_DIR) out[(nb + k) * A] = dir[k];
-                if (aux & AUX_ALB) out[(2 * nb + k) * A] = alb[k];
-            }
-        }
-        out += (size_t)3 * nb * A;
-        if (aux & AUX_NRM) { out[0] = ns.x; out[A] = ns.y; out[2 * A] = ns.z; }
-        if (aux & AUX_DEP) { out[3 * A] = dep; out[4 * A] = __uint_as_float(cnt); }
-        if (aux & AUX_TRI) out[5 * A] = __uint_as_float(tri);
+        film_rest(fp, f, p, sf, dep, cnt, tri, ns);
     }
     warp_reduce_add(&st.stats[2], nclosest);
     warp_reduce_add(&st.stats[3], nshadow);
@@ -1972,7 +1974,7 @@ void launch_chunks(vgb_context* ctx, const FrameParams& fp, const FilmOut& film,
                    bool prof, uint32_t& launches) {
     const DevScene s = dev_scene(ctx);
     const size_t tiles = (size_t)fp.tiles_x * fp.tiles_y;
-    const int gp = grid_for(ctx, fp.npix, VGB_END_GRID);
+    const int gp = grid_for(ctx, fp.npix, VGB_FOLD_GRID);
     for (uint32_t s0 = 0; s0 < fp.opt.samples; s0 += chunk) {
         const uint32_t n = std::min(chunk, fp.opt.samples - s0);
         const size_t items = tiles * n * 32;
@@ -2005,7 +2007,7 @@ void launch_chunks(vgb_context* ctx, const FrameParams& fp, const FilmOut& film,
             q ^= 1u;
         }
         Prof p(ctx, 2, prof);
-        k_fold<NB><<<gp, 256, 0, ctx->stream>>>(st, fp, n, s0 == 0 ? 1u : 0u, s0 + n == fp.opt.samples ? 1u : 0u, film);
+        k_fold<<<dim3(gp, fp.nb + 1), 256, 0, ctx->stream>>>(st, fp, n, s0 == 0 ? 1u : 0u, s0 + n == fp.opt.samples ? 1u : 0u, film);
         launches++;
     }
 }
