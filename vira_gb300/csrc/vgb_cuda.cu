@@ -252,6 +252,7 @@ struct FrameParams {
     uint32_t aux;   // AUX_* bits: the per-pixel sums the requested film planes need
     // first-hit film planes k_shade writes directly (null when not requested)
     float *vel_g, *vel_c, *tsz;
+    const float4* dirs;   // integer-pixel ray directions (k_direction_table), or null
     uint32_t npix;   // pixels of the frame: a state slot is (sample in flight) * npix + pixel
 };
 
@@ -655,22 +656,43 @@ __device__ __forceinline__ F3 direction_helper(const vgb_camera& cam, float X, f
 
 // Camera::pixelToDirection (camera.ipp:1105-1117): with a distortion and direction interpolation,
 // Image::interpolatePixel (image.ipp:619-671) of the table precomputePixelDirections fills with
-// normalize(pixelToDirectionHelper(i, j)) -- evaluated here at the four corners on the fly.
-__device__ __noinline__ F3 interpolated_direction(const vgb_camera& cam, float X, float Y) {
+// normalize(pixelToDirectionHelper(i, j)) -- read from `dirs` where the render filled one
+// (k_direction_table), else evaluated here at the four corners on the fly.
+__device__ __noinline__ F3 interpolated_direction(const vgb_camera& cam, const float4* __restrict__ dirs, float X, float Y) {
     int x0 = (int)floorf(X), y0 = (int)floorf(Y);
     x0 = min(x0, (int)cam.width - 1);
     y0 = min(y0, (int)cam.height - 1);
     const int x1 = min(x0 + 1, (int)cam.width - 1), y1 = min(y0 + 1, (int)cam.height - 1);
-    const F3 p00 = normalize(direction_helper(cam, (float)x0, (float)y0));
-    const F3 p10 = normalize(direction_helper(cam, (float)x1, (float)y0));
-    const F3 p01 = normalize(direction_helper(cam, (float)x0, (float)y1));
-    const F3 p11 = normalize(direction_helper(cam, (float)x1, (float)y1));
+    F3 p00, p10, p01, p11;
+    if (dirs) {
+        const float4* r0 = dirs + (size_t)y0 * cam.width;
+        const float4* r1 = dirs + (size_t)y1 * cam.width;
+        p00 = ld3(__ldg(r0 + x0)); p10 = ld3(__ldg(r0 + x1)); p01 = ld3(__ldg(r1 + x0)); p11 = ld3(__ldg(r1 + x1));
+    } else {
+        p00 = normalize(direction_helper(cam, (float)x0, (float)y0));
+        p10 = normalize(direction_helper(cam, (float)x1, (float)y0));
+        p01 = normalize(direction_helper(cam, (float)x0, (float)y1));
+        p11 = normalize(direction_helper(cam, (float)x1, (float)y1));
+    }
     const float dx = X - (float)x0, dy = Y - (float)y0;
     return (((1.f - dx) * (1.f - dy) * p00 + dx * (1.f - dy) * p10) + (1.f - dx) * dy * p01) + dx * dy * p11;
 }
 
-__device__ __forceinline__ F3 camera_direction(const vgb_camera& cam, float X, float Y) {
-    if (cam.distortion && cam.interpolate_directions) return interpolated_direction(cam, X, Y);
+// The table of integer-pixel directions of a camera with a lens distortion, for the renders that start
+// several rays a pixel: each entry is 20 undistortion steps, which a ray between four pixels would
+// otherwise run four times (1920 x 1080 x 4 spp: the camera rays' share of the call fell from about
+// half).
+__global__ void k_direction_table(const __grid_constant__ vgb_camera cam, float4* __restrict__ dirs) {
+    const uint32_t n = cam.width * cam.height;
+    for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x) {
+        const uint32_t y = p / cam.width;
+        const F3 d = normalize(direction_helper(cam, (float)(p - y * cam.width), (float)y));
+        dirs[p] = make_float4(d.x, d.y, d.z, 0.f);
+    }
+}
+
+__device__ __forceinline__ F3 camera_direction(const vgb_camera& cam, const float4* __restrict__ dirs, float X, float Y) {
+    if (cam.distortion && cam.interpolate_directions) return interpolated_direction(cam, dirs, X, Y);
     return direction_helper(cam, X, Y);
 }
 
@@ -680,7 +702,8 @@ __device__ __forceinline__ F3 camera_direction(const vgb_camera& cam, float X, f
 // draw's first two words move the pixel coordinate, its last two sample the aperture disc
 // (UniformDiskSample, sampling.ipp:43-52).
 __device__ __forceinline__ void pixel_ray(const vgb_camera& cam, uint32_t pi, uint32_t pj, uint32_t slot,
-                                          uint32_t sample, uint32_t frame, uint32_t k0, uint32_t k1, F3& ro, F3& rd) {
+                                          uint32_t sample, uint32_t frame, uint32_t k0, uint32_t k1, F3& ro, F3& rd,
+                                          const float4* __restrict__ dirs = nullptr) {
     float X = (float)pi, Y = (float)pj;
     U4 jr{0, 0, 0, 0};
     if (sample != 0) {
@@ -688,7 +711,7 @@ __device__ __forceinline__ void pixel_ray(const vgb_camera& cam, uint32_t pi, ui
         X = X + u01(jr.x);
         Y = Y + u01(jr.y);
     }
-    F3 dc = camera_direction(cam, X, Y);
+    F3 dc = camera_direction(cam, dirs, X, Y);
     const float* R = cam.rotation;
     ro = F3{cam.origin[0], cam.origin[1], cam.origin[2]};
     if (sample != 0 && cam.depth_of_field) {
@@ -711,7 +734,8 @@ __device__ __forceinline__ bool camera_ray(const FrameParams& fp, uint32_t item,
     const uint32_t pi = tx * 8u + (ln & 7u), pj = ty * 4u + (ln >> 3);
     if (pi >= fp.cam.width || pj >= fp.cam.height) return false;
     slot = pj * fp.cam.width + pi;
-    pixel_ray(fp.cam, pi, pj, slot, sample, fp.opt.frame, (uint32_t)fp.opt.seed, (uint32_t)(fp.opt.seed >> 32), ro, rd);
+    pixel_ray(fp.cam, pi, pj, slot, sample, fp.opt.frame, (uint32_t)fp.opt.seed, (uint32_t)(fp.opt.seed >> 32), ro, rd,
+              fp.dirs);
     return true;
 }
 
@@ -1391,7 +1415,7 @@ __global__ void __launch_bounds__(64, VGB_FRONT_MINB) k_front(const DevScene s, 
     HitOut h;
     h.id = VGB_NO_HIT;
     if (valid) {
-        pixel_ray(fp.cam, pi, pj, pix, sample, fp.opt.frame, k0, k1, ro, rd);
+        pixel_ray(fp.cam, pi, pj, pix, sample, fp.opt.frame, k0, k1, ro, rd, fp.dirs);
         h.U = h.V = h.W = 0.f; h.det = 1.f;
         trace_ool<4>(s, make_wray(ro, rd), 0.f, false, h, err);
         if (h.id == VGB_NO_HIT) {
@@ -1751,6 +1775,9 @@ struct vgb_context {
     // pinned host staging of file payloads (Quipu LoDs)
     void* h_pin = nullptr;
     size_t cap_pin = 0;
+    // integer-pixel ray directions of the render in hand (cameras with a lens distortion)
+    float4* d_dirs = nullptr;
+    size_t cap_dirs = 0;
     // device address of vgb_render_noalloc's fixed array, looked up by its first call
     unsigned char* noalloc_base = nullptr;
     // traversal steps per ray before the ray gives up (vgb_set_traversal_limit)
@@ -2354,6 +2381,7 @@ VGB_API vgb_status vgb_context_destroy(vgb_context* ctx) try {
     if (ctx->h_frames) cudaFreeHost(ctx->h_frames);
     dfree(ctx->d_adj); dfree(ctx->d_views); dfree(ctx->d_loss); dfree(ctx->d_dn);
     if (ctx->h_pin) cudaFreeHost(ctx->h_pin);
+    dfree(ctx->d_dirs);
     if (ctx->ev0) cudaEventDestroy(ctx->ev0);
     if (ctx->ev1) cudaEventDestroy(ctx->ev1);
     if (ctx->own_stream && ctx->stream) cudaStreamDestroy(ctx->stream);
@@ -3587,7 +3615,21 @@ VGB_API vgb_status vgb_render(vgb_context* ctx, const vgb_camera* cam, const vgb
     CK(cudaMemsetAsync(ctx->d_stats, 0, sizeof(uint64_t) * 8, ctx->stream));
     uint32_t launches = 0;
     ctx->prof_used = 0;
+    if (cam->distortion && cam->interpolate_directions) {
+        if (P > ctx->cap_dirs) {
+            dfree(ctx->d_dirs);
+            ctx->d_dirs = nullptr;
+            ctx->cap_dirs = 0;
+            if ((s = dalloc(ctx, &ctx->d_dirs, P * sizeof(float4))) != VGB_OK) return s;
+            ctx->cap_dirs = P;
+        }
+        fp.dirs = ctx->d_dirs;
+    }
     CK(cudaEventRecord(ctx->ev0, ctx->stream));
+    if (fp.dirs) {
+        k_direction_table<<<grid_for(ctx, P, 16), 256, 0, ctx->stream>>>(fp.cam, ctx->d_dirs);
+        launches++;
+    }
     st.P = std::max<size_t>(chunk, 1) * P;
     if (chunk) {
         if (fp.nb <= 1) launch_chunks<1>(ctx, fp, fr, st, chunk, true, launches);
