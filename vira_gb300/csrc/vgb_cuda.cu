@@ -301,6 +301,10 @@ __device__ __forceinline__ uint32_t warp_append(uint32_t* count, bool pred) {
     return base + (uint32_t)__popc(mask & ((1u << lane) - 1u));
 }
 
+// sinf and cosf of one angle, out of line: their code (argument reduction included) is long, and the
+// kernels that shade call it for the light, the continuation and the lens.
+__device__ __noinline__ float2 sin_cos(float a) { return make_float2(sinf(a), cosf(a)); }
+
 // SphereLight::sample with and without RNG (sphere_light.ipp:31-124)
 __device__ __forceinline__ void light_sample(const vgb_light& L, F3 p, bool det, float rand1, float rand2,
                                              F3& dir, float& distance, float& pdf) {
@@ -331,7 +335,8 @@ __device__ __forceinline__ void light_sample(const vgb_light& L, F3 p, bool det,
     float zeta = rand2;
     float cc = r / distance;
     float theta = acosf(1 - zeta + zeta * sqrtf(1 - (cc * cc)));
-    float sinT = sinf(theta), sinP = sinf(phi), cosT = cosf(theta), cosP = cosf(phi);
+    const float2 T = sin_cos(theta), Q = sin_cos(phi);
+    float sinT = T.x, sinP = Q.x, cosT = T.y, cosP = Q.y;
     float a = cosP * sinT, b = cosT, e = sinP * sinT;
     dir = F3{(a * U.x + b * W.x) + e * Vv.x, (a * U.y + b * W.y) + e * Vv.y, (a * U.z + b * W.z) + e * Vv.z};
     float r2 = r * r;
@@ -371,17 +376,24 @@ __device__ __forceinline__ F3 cosine_sample(float rand1, float rand2) {
         const float P4 = kPi / 4.0f, P2 = kPi / 2.0f;
         if (fabsf(ux) > fabsf(uy)) { r = ux; theta = P4 * (uy / ux); }
         else { r = uy; theta = P2 - P4 * (ux / uy); }
-        dx = r * cosf(theta); dy = r * sinf(theta);
+        const float2 q = sin_cos(theta);
+        dx = r * q.y; dy = r * q.x;
     }
     float z = sqrtf(smax(0.f, 1 - dx * dx - dy * dy));
     return F3{dx, dy, z};
 }
 
+// fmodf(x, r) for r > 0; the coordinates of a texture that does not wrap are already in [0, r),
+// where it is x itself.
+__device__ __noinline__ float fmod_wrapped(float x, float r) { return fmodf(x, r); }
+__device__ __forceinline__ float texture_mod(float x, float r) { return (x >= 0.f && x < r) ? x : fmod_wrapped(x, r); }
+
 // Image::sampleUVs + interpolatePixel (image.ipp:589-671), one band
-template <int NB>
+template <int NB, bool ROLL = false>
 __device__ __forceinline__ void sample_uvs(const DevScene& s, uint32_t nb, float u, float v, float* out) {
+    constexpr int U = ROLL ? 1 : NB;   // band loops rolled: less code, the bands in local memory
     float rx = (float)s.tw, ry = (float)s.th;
-    float px = fmodf(u * rx, rx), py = fmodf(v * ry, ry);
+    float px = texture_mod(u * rx, rx), py = texture_mod(v * ry, ry);
     if (px < 0) px += rx;
     if (py < 0) py += ry;
     int x0 = (int)floorf(px), y0 = (int)floorf(py);
@@ -394,7 +406,7 @@ __device__ __forceinline__ void sample_uvs(const DevScene& s, uint32_t nb, float
         const float t00 = __ldg(&s.tex[(size_t)y0 * s.tw + x0]), t10 = __ldg(&s.tex[(size_t)y0 * s.tw + x1]);
         const float t01 = __ldg(&s.tex[(size_t)y1 * s.tw + x0]), t11 = __ldg(&s.tex[(size_t)y1 * s.tw + x1]);
         const float val = ((a * t00 + b * t10) + c * t01) + e * t11;
-#pragma unroll
+#pragma unroll U
         for (int k = 0; k < NB; ++k) out[k] = val;
         return;
     }
@@ -402,7 +414,7 @@ __device__ __forceinline__ void sample_uvs(const DevScene& s, uint32_t nb, float
     const float* p10 = &s.tex[((size_t)y0 * s.tw + x1) * nb];
     const float* p01 = &s.tex[((size_t)y1 * s.tw + x0) * nb];
     const float* p11 = &s.tex[((size_t)y1 * s.tw + x1) * nb];
-#pragma unroll
+#pragma unroll U
     for (int k = 0; k < NB; ++k)
         if (k < (int)nb) out[k] = ((a * __ldg(p00 + k) + b * __ldg(p10 + k)) + c * __ldg(p01 + k)) + e * __ldg(p11 + k);
 }
@@ -410,7 +422,7 @@ __device__ __forceinline__ void sample_uvs(const DevScene& s, uint32_t nb, float
 // Image<Normal>::sampleUVs of the normal map (wrap + bilinear, image.ipp:589-671).
 __device__ __forceinline__ F3 sample_normal_map(const DevScene& s, float u, float v) {
     const float rx = (float)s.nw, ry = (float)s.nh;
-    float px = fmodf(u * rx, rx), py = fmodf(v * ry, ry);
+    float px = texture_mod(u * rx, rx), py = texture_mod(v * ry, ry);
     if (px < 0) px += rx;
     if (py < 0) py += ry;
     int x0 = (int)floorf(px), y0 = (int)floorf(py);
@@ -454,7 +466,7 @@ __device__ __forceinline__ void tangent_frame(F3 N, F3& tg, F3& bt) {
 // (tg, bt, nf): the tangent frame built before the map, which the continuation samples in;
 // FRAME = false for callers that sample no continuation (tg and bt are then left unset unless
 // the scene has a normal map, which needs them).
-template <int NB, bool FRAME = true>
+template <int NB, bool FRAME = true, bool ROLL = false>
 __device__ __forceinline__ void surface_at(const DevScene& s, uint32_t nb, bool smooth, uint32_t t, float w0f,
                                            float w1f, F3& Pp, F3& N, F3& fnrm, F3& tg, F3& bt, F3& nf, float* alb,
                                            float* va_out = nullptr, float* tex_out = nullptr, float* uv_out = nullptr) {
@@ -481,9 +493,10 @@ __device__ __forceinline__ void surface_at(const DevScene& s, uint32_t nb, bool 
         tangent_frame(Nl, tg, bt);
         N = mapped_normal(s, uvx, uvy, Nl, tg, bt);
     }
+    constexpr int U = ROLL ? 1 : NB;
     float texv[NB];
-    sample_uvs<NB>(s, nb, uvx, uvy, texv);
-#pragma unroll
+    sample_uvs<NB, ROLL>(s, nb, uvx, uvy, texv);
+#pragma unroll U
     for (int k = 0; k < NB; ++k) {
         if (k < (int)nb) {
             float va;
@@ -513,10 +526,11 @@ __device__ __forceinline__ void surface_at(const DevScene& s, uint32_t nb, bool 
 // Direct lighting from one light (cpu_path_tracer.ipp:399-428): samples the light and returns
 // whether a shadow ray is needed, its direction and length, and the contribution per band if
 // the shadow ray is unoccluded.
-template <int NB>
+template <int NB, bool ROLL = false>
 __device__ __forceinline__ bool nee_light(const vgb_light& L, F3 Pp, F3 N, const float* alb, const float* thr,
                                           uint32_t nb, bool det, float ru1, float ru2, F3& Ld, float& dist,
                                           float* con) {
+    constexpr int U = ROLL ? 1 : NB;
     float lpdf = 0.f;
     light_sample(L, Pp, det, ru1, ru2, Ld, dist, lpdf);
     if (!(lpdf > 0)) return false;
@@ -524,7 +538,7 @@ __device__ __forceinline__ bool nee_light(const vgb_light& L, F3 Pp, F3 N, const
     const float cos_t = smax(0.0f, dot(Ld, N));
     const float mpdf = (nl <= 0.f) ? 0.f : nl * kInvPi;
     const float wgt = power_heuristic(lpdf, mpdf);
-#pragma unroll
+#pragma unroll U
     for (int k = 0; k < NB; ++k) {
         const float bsdf = alb[k] * kInvPi * smax(nl, 0.f);
         con[k] = (k < (int)nb) ? thr[k] * bsdf * L.radiance[k] * cos_t * wgt / lpdf : 0.f;
@@ -535,11 +549,12 @@ __device__ __forceinline__ bool nee_light(const vgb_light& L, F3 Pp, F3 N, const
 // BSDF-sampled continuation (cpu_path_tracer.ipp:431-461) with optional Russian roulette.
 // Returns whether the path continues; new_ray is false when the sampled pdf is 0 (the reference
 // then keeps the incoming ray and throughput).
-template <int NB>
+template <int NB, bool ROLL = false>
 __device__ __forceinline__ bool continue_path(const vgb_light* lights, uint32_t nlights, const vgb_pt_options& opt,
                                               uint32_t nb, F3 Pp, F3 N, F3 tg, F3 bt, F3 nf, const float* alb,
                                               float* thr, U4 r0, uint32_t slot, uint32_t sample, uint32_t frame,
                                               uint32_t bounce, F3& nd, bool& new_ray) {
+    constexpr int U = ROLL ? 1 : NB;
     new_ray = false;
     F3 ls = cosine_sample(u01(r0.z), u01(r0.w));
     const float mpdf = ls.z * kInvPi;
@@ -552,7 +567,7 @@ __device__ __forceinline__ bool continue_path(const vgb_light* lights, uint32_t 
     for (uint32_t l = 0; l < nlights; ++l) lp += light_pdf(lights[l], Pp, nd);
     lp /= (float)nlights;
     const float wgt = power_heuristic(mpdf, lp);
-#pragma unroll
+#pragma unroll U
     for (int k = 0; k < NB; ++k) {
         const float bsdf = alb[k] * kInvPi * smax(nl, 0.f);
         if (k < (int)nb) thr[k] *= bsdf * cos_t * wgt / mpdf;
@@ -560,13 +575,13 @@ __device__ __forceinline__ bool continue_path(const vgb_light* lights, uint32_t 
     new_ray = true;
     if (opt.rr_depth != 0 && bounce + 1 >= opt.rr_depth) {
         float q = 0.f;
-#pragma unroll
+#pragma unroll U
         for (int k = 0; k < NB; ++k) if (k < (int)nb) q = smax(q, thr[k]);
         q = smin(q, 1.0f);
         const U4 rr = philox(U4{slot, sample, frame, (bounce << 8) | kSlotRR}, (uint32_t)opt.seed,
                              (uint32_t)(opt.seed >> 32));
         if (u01(rr.x) >= q) return false;
-#pragma unroll
+#pragma unroll U
         for (int k = 0; k < NB; ++k) if (k < (int)nb) thr[k] = thr[k] / q;
     }
     return true;
@@ -696,6 +711,19 @@ __device__ __forceinline__ F3 camera_direction(const vgb_camera& cam, const floa
     return direction_helper(cam, X, Y);
 }
 
+// Depth of field: the ray moved to a point of the aperture disc (camera.ipp:1143-1163).  Out of line,
+// as most cameras are pinholes.
+__device__ __noinline__ void aperture_ray(const vgb_camera& cam, uint32_t z, uint32_t w, F3& ro, F3& dc) {
+    const float* R = cam.rotation;
+    const float r = sqrtf(u01(z));
+    const float theta = 2.f * kPi * u01(w);
+    const float2 q = sin_cos(theta);
+    const F3 off{cam.aperture_radius * (r * q.y), cam.aperture_radius * (r * q.x), cam.focal_length};
+    ro = ro + F3{(R[0] * off.x + R[3] * off.y) + R[6] * off.z, (R[1] * off.x + R[4] * off.y) + R[7] * off.z,
+                 (R[2] * off.x + R[5] * off.y) + R[8] * off.z};
+    if (!isinf(cam.focus_distance)) dc = cam.focus_distance * normalize(dc) - off;
+}
+
 // Camera::pixelToRay for pixel (pi, pj) = slot: sample 0 through the pixel corner with the
 // pinhole overload, later samples jittered and, with depth of field, through a point of the
 // aperture (camera.ipp:1126-1163, cpu_path_tracer.ipp:182-192).  Random numbers: the jitter
@@ -714,14 +742,7 @@ __device__ __forceinline__ void pixel_ray(const vgb_camera& cam, uint32_t pi, ui
     F3 dc = camera_direction(cam, dirs, X, Y);
     const float* R = cam.rotation;
     ro = F3{cam.origin[0], cam.origin[1], cam.origin[2]};
-    if (sample != 0 && cam.depth_of_field) {
-        const float r = sqrtf(u01(jr.z));
-        const float theta = 2.f * kPi * u01(jr.w);
-        const F3 off{cam.aperture_radius * (r * cosf(theta)), cam.aperture_radius * (r * sinf(theta)), cam.focal_length};
-        ro = ro + F3{(R[0] * off.x + R[3] * off.y) + R[6] * off.z, (R[1] * off.x + R[4] * off.y) + R[7] * off.z,
-                     (R[2] * off.x + R[5] * off.y) + R[8] * off.z};
-        if (!isinf(cam.focus_distance)) dc = cam.focus_distance * normalize(dc) - off;
-    }
+    if (sample != 0 && cam.depth_of_field) aperture_ray(cam, jr.z, jr.w, ro, dc);
     F3 dw{(R[0] * dc.x + R[3] * dc.y) + R[6] * dc.z, (R[1] * dc.x + R[4] * dc.y) + R[7] * dc.z,
           (R[2] * dc.x + R[5] * dc.y) + R[8] * dc.z};
     rd = normalize(dw);
@@ -1394,6 +1415,10 @@ __global__ void __launch_bounds__(256) k_end_sample(DevState st, const __grid_co
 template <int NB>
 __global__ void __launch_bounds__(64, VGB_FRONT_MINB) k_front(const DevScene s, DevState st, const __grid_constant__ FrameParams fp,
                                                   uint32_t sample0, uint32_t nsamples) {
+    // Band loops rolled, the bands in local memory (they wait there through each traversal anyway): the
+    // kernel is bound by instruction fetch as much as by issue.  2048^2 x 4 spp 8.96 -> 8.70 ms.
+    constexpr bool ROLL = NB > 1;
+    constexpr int U = ROLL ? 1 : NB;
     const uint32_t nb = fp.nb;
     const size_t P = st.P;
     const int lane = threadIdx.x & 31;
@@ -1410,7 +1435,7 @@ __global__ void __launch_bounds__(64, VGB_FRONT_MINB) k_front(const DevScene s, 
     bool cont = false;
     F3 ro{0.f, 0.f, 0.f}, rd{0.f, 0.f, 1.f};
     float thr[NB], rad[NB];
-#pragma unroll
+#pragma unroll U
     for (int k = 0; k < NB; ++k) { thr[k] = 1.f; rad[k] = 0.f; }
     HitOut h;
     h.id = VGB_NO_HIT;
@@ -1421,7 +1446,7 @@ __global__ void __launch_bounds__(64, VGB_FRONT_MINB) k_front(const DevScene s, 
         if (h.id == VGB_NO_HIT) {
             if (fp.opt.simulate_lighting && fp.opt.show_background) {
                 const float4 bw = background_weights(rd);
-#pragma unroll
+#pragma unroll U
                 for (int k = 0; k < NB; ++k) {
                     const float bgv = fp.opt.background[k];
                     const float bg = ((bw.x * bgv + bw.y * bgv) + bw.z * bgv) + bw.w * bgv;
@@ -1434,7 +1459,7 @@ __global__ void __launch_bounds__(64, VGB_FRONT_MINB) k_front(const DevScene s, 
             const float rcp = 1.0f / h.det;
             F3 Pp, N, fnrm, tg, bt, nf;
             float alb[NB];
-            surface_at<NB>(s, nb, fp.opt.smooth_shading != 0, h.id, h.V * rcp, h.W * rcp, Pp, N, fnrm, tg, bt, nf, alb);
+            surface_at<NB, true, ROLL>(s, nb, fp.opt.smooth_shading != 0, h.id, h.V * rcp, h.W * rcp, Pp, N, fnrm, tg, bt, nf, alb);
             note |= kPendHit;
             if (fp.aux & AUX_TRI) {
                 st.atri[slot] = h.id;
@@ -1443,7 +1468,7 @@ __global__ void __launch_bounds__(64, VGB_FRONT_MINB) k_front(const DevScene s, 
                                      fp.tsz ? st.pfh + 6 * P : nullptr, P, (uint32_t)slot);
             }
             if (fp.aux & AUX_ALB) {
-#pragma unroll
+#pragma unroll U
                 for (int k = 0; k < NB; ++k) if (k < (int)nb) st.aalb[k * P + slot] = alb[k];
             }
             if (fp.aux & AUX_NRM) { st.anrm[slot] = N.x; st.anrm[P + slot] = N.y; st.anrm[2 * P + slot] = N.z; }
@@ -1451,7 +1476,7 @@ __global__ void __launch_bounds__(64, VGB_FRONT_MINB) k_front(const DevScene s, 
             if (fp.opt.simulate_lighting) {
                 Pp = F3{offset1(Pp.x, fnrm.x), offset1(Pp.y, fnrm.y), offset1(Pp.z, fnrm.z)};
                 if (fp.opt.has_ambient) {
-#pragma unroll
+#pragma unroll U
                     for (int k = 0; k < NB; ++k) if (k < (int)nb) rad[k] = 0.f + 1.f * (fp.opt.ambient[k] * alb[k]);
                 }
                 const U4 r0 = philox(U4{pix, sample, fp.opt.frame, kSlotMain}, k0, k1);
@@ -1463,32 +1488,32 @@ __global__ void __launch_bounds__(64, VGB_FRONT_MINB) k_front(const DevScene s, 
                     }
                     F3 Ld;
                     float dist, con[NB];
-                    if (!nee_light<NB>(fp.lights[l], Pp, N, alb, thr, nb, fp.opt.deterministic_light != 0, ru1, ru2, Ld, dist, con))
+                    if (!nee_light<NB, ROLL>(fp.lights[l], Pp, N, alb, thr, nb, fp.opt.deterministic_light != 0, ru1, ru2, Ld, dist, con))
                         continue;
                     HitOut hs;
                     trace_ool<4>(s, make_wray(Pp, Ld), dist, true, hs, err);
                     note += 1u << kPendShadow;
                     if (hs.id == VGB_NO_HIT) {
-#pragma unroll
+#pragma unroll U
                         for (int k = 0; k < NB; ++k) if (k < (int)nb) rad[k] += con[k];
                     }
                 }
                 if (fp.aux & AUX_DIR) {
-#pragma unroll
+#pragma unroll U
                     for (int k = 0; k < NB; ++k) if (k < (int)nb) st.adir[k * P + slot] = rad[k];
                 }
                 note &= ~kPradEmpty;
-#pragma unroll
+#pragma unroll U
                 for (int k = 0; k < NB; ++k) rad[k] = 0.f + rad[k];
                 if (fp.opt.bounces != 0) {
                     F3 nd;
                     bool new_ray;
-                    cont = continue_path<NB>(fp.lights, fp.nlights, fp.opt, nb, Pp, N, tg, bt, nf, alb, thr, r0, pix, sample,
+                    cont = continue_path<NB, ROLL>(fp.lights, fp.nlights, fp.opt, nb, Pp, N, tg, bt, nf, alb, thr, r0, pix, sample,
                                              fp.opt.frame, 0u, nd, new_ray);
                     if (new_ray) { ro = Pp; rd = nd; }   // pdf 0: the reference keeps the incoming ray and throughput
                 }
             } else if (fp.aux & AUX_DIR) {
-#pragma unroll
+#pragma unroll U
                 for (int k = 0; k < NB; ++k) if (k < (int)nb) st.adir[k * P + slot] = 0.f;
             }
         }
@@ -1500,7 +1525,7 @@ __global__ void __launch_bounds__(64, VGB_FRONT_MINB) k_front(const DevScene s, 
         note |= kPendRay1;
         if (h.id == VGB_NO_HIT && fp.opt.show_background) {
             const float4 bw = background_weights(rd);
-#pragma unroll
+#pragma unroll U
             for (int k = 0; k < NB; ++k) {
                 const float bgv = fp.opt.background[k];
                 const float bg = ((bw.x * bgv + bw.y * bgv) + bw.z * bgv) + bw.w * bgv;
@@ -1516,13 +1541,13 @@ __global__ void __launch_bounds__(64, VGB_FRONT_MINB) k_front(const DevScene s, 
         st.pq[0][qi] = (uint32_t)slot;
         st.org[slot] = ro.x; st.org[P + slot] = ro.y; st.org[2 * P + slot] = ro.z;
         st.dir[slot] = rd.x; st.dir[P + slot] = rd.y; st.dir[2 * P + slot] = rd.z;
-#pragma unroll
+#pragma unroll U
         for (int k = 0; k < NB; ++k) if (k < (int)nb) st.thr[k * P + slot] = thr[k];
     }
     if (valid) {
         st.pend[slot] = note;
         if (!(note & kPradEmpty)) {
-#pragma unroll
+#pragma unroll U
             for (int k = 0; k < NB; ++k) if (k < (int)nb) st.prad[k * P + slot] = rad[k];
         }
     }
