@@ -1785,6 +1785,8 @@ struct vgb_context {
     size_t cap_frames = 0;
     void* h_frames = nullptr;                // pinned staging of the table
     uint32_t tuned_threads = 0, tuned_bps = 0, tuned_grab = 0;
+    uint64_t tuned_key = 0;                  // the work they were tuned for
+    uint32_t bvh_serial = 0;                 // trees built in this context
     cudaGraphExec_t graph_exec = nullptr;
     uint64_t graph_key = 0;
     unsigned char graph_params_probe[1024] = {0};   // kernel parameters the graph was captured with
@@ -1855,6 +1857,7 @@ void free_bvh(vgb_context* ctx) {
     dfree(ctx->d_nodes); dfree(ctx->d_wide); dfree(ctx->d_tris); dfree(ctx->d_parent); dfree(ctx->d_refit);
     ctx->d_nodes = ctx->d_wide = nullptr; ctx->nwide = 0; ctx->d_tris = nullptr; ctx->d_parent = nullptr; ctx->d_refit = nullptr;
     ctx->bvh_ready = false; ctx->nnodes = 0;
+    ctx->bvh_serial++;
 }
 void free_scratch(vgb_context* ctx) {
     for (void* p : ctx->scratch) dfree(p);
@@ -4542,30 +4545,41 @@ extern "C" VGB_API vgb_status vgb_render_batch(vgb_context* ctx, const vgb_frame
     if (threads != 64 && threads != 128 && threads != 256)
         return fail(ctx, VGB_ERR_INVALID_ARGUMENT, "render_batch: block_threads must be 64, 128 or 256");
     CK(cudaMemsetAsync(ctx->d_stats, 0, sizeof(uint64_t) * 8, ctx->stream));
-    if (bo && bo->autotune) {
-        // autotuner: time candidate launch shapes on every 16th tile, keep the fastest
+    // The shape tuned for this kernel (bands, lean or general, sums, bounces), this tree and this
+    // magnitude of work; a call that asks for tuning again with the same uses it as it is.
+    uint32_t mag = 0;
+    while ((bp.total_tiles >> mag) > 1u) ++mag;
+    const uint64_t tune_key = 1ull | ((uint64_t)ctx->nbands << 1) | ((uint64_t)bp.sums << 5) |
+                              ((uint64_t)(opts->bounces != 0) << 6) | ((uint64_t)(opts->adaptive_sampling != 0) << 7) |
+                              ((uint64_t)mag << 8) | ((uint64_t)ctx->bvh_serial << 16);
+    if (bo && bo->autotune && ctx->tuned_key != tune_key) {
+        // Autotuner: time candidate launch shapes on every 16th tile, keep the fastest.  Every
+        // candidate fills the SMs (the launch clamps the blocks to what is resident): with the 24
+        // shapes of 2-16 blocks per SM tried on every call, most of them duplicates or a fraction of
+        // the resident warps, the probes took 23 ms beside a 3.3 ms render of 15 frames.
         const uint32_t cand_t[] = {64, 128, 256};
-        const uint32_t cand_b[] = {2, 4, 8, 16};
         const uint32_t cand_g[] = {1, 4};
         float best = INFINITY;
         BatchParams probe = bp;
         probe.tile_stride = 16;
         for (uint32_t ct : cand_t)
-            for (uint32_t cb : cand_b)
-                for (uint32_t cg : cand_g) {
-                    probe.grab = cg;
-                    CK(cudaEventRecord(ctx->ev0, ctx->stream));
-                    CK(launch_batch_any(ctx, dfr, probe, ct, cb));
-                    CK(cudaEventRecord(ctx->ev1, ctx->stream));
-                    CK(cudaEventSynchronize(ctx->ev1));
-                    float ms = 0.f;
-                    cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
-                    if (ms < best) { best = ms; threads = ct; bps = cb; grab = cg; }
-                }
+            for (uint32_t cg : cand_g) {
+                probe.grab = cg;
+                CK(cudaEventRecord(ctx->ev0, ctx->stream));
+                CK(launch_batch_any(ctx, dfr, probe, ct, 16));
+                CK(cudaEventRecord(ctx->ev1, ctx->stream));
+                CK(cudaEventSynchronize(ctx->ev1));
+                float ms = 0.f;
+                cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
+                if (ms < best) { best = ms; threads = ct; bps = 16; grab = cg; }
+            }
         ctx->tuned_threads = threads; ctx->tuned_bps = bps; ctx->tuned_grab = grab;
+        ctx->tuned_key = tune_key;
         CK(cudaMemsetAsync(ctx->d_stats, 0, sizeof(uint64_t) * 8, ctx->stream));
         vgb_status es = check_device_error(ctx);
         if (es != VGB_OK) return es;
+    } else if (bo && bo->autotune) {
+        threads = ctx->tuned_threads; bps = ctx->tuned_bps; grab = ctx->tuned_grab;
     }
     bp.grab = grab;
     bp.tile_stride = 1;
