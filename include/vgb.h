@@ -499,6 +499,20 @@ VGB_API vgb_status vgb_psf_convolve(vgb_context* ctx, float* received_power, uin
 /* Replaces the albedo texture (same size) without re-uploading the mesh or rebuilding the BVH. */
 VGB_API vgb_status vgb_texture_update(vgb_context* ctx, const float* texture, uint32_t tex_w, uint32_t tex_h);
 
+/* The reference's per-instance first-hit ids (passes.ipp:96-101) from a render's triangle ids, in one
+ * pass over device planes of `npixels` pixels, queued on `stream` (a cudaStream_t of the context's
+ * device, 0 for the default stream) without waiting for it.  tri (in: the flattened scene's triangle
+ * id + first, VGB_NO_HIT on a miss; out: the triangle within its instance + first); ranges: the
+ * instances in flattening order, ascending first_triangle from 0; normal_camera ([3][npixels]):
+ * `rotation` (3 x 3, row major) times normal_global, or zeros when rotation is NULL. */
+typedef struct vgb_instance_range {
+    uint32_t first_triangle, instance, mesh;
+} vgb_instance_range;
+VGB_API vgb_status vgb_first_hit_ids(vgb_context* ctx, void* stream, uint64_t npixels, uint32_t* tri, uint32_t first,
+                                     const vgb_instance_range* ranges, uint32_t nranges, const float* normal_global,
+                                     const float* rotation, int32_t* instance_id, int32_t* mesh_id,
+                                     int32_t* material_id, float* normal_camera);
+
 /* TLAS::intersect(Ray&) seam (include/vira/rendering/acceleration/tlas.hpp:24): a batch of
  * rays, closest hit (any_hit = 0) or occlusion (any_hit = 1, tmax per ray or +inf).
  * origins/dirs: 3 floats per ray.  tri_out: VGB_NO_HIT on a miss; t_out: +inf on a miss;

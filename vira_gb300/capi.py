@@ -200,6 +200,7 @@ SIGNATURES = {
     "vgb_denoise": (C.c_int, [_P, _P, _P, _P, _P, _P, _U32, _U32, _U32, _P, C.c_int]),
     "vgb_adjoint_positions": (C.c_int, [_P, C.POINTER(Camera), _P, _U32, C.POINTER(PtOptions), _P, _P, _P, C.c_int]),
     "vgb_render_adjoint_batch": (C.c_int, [_P, _P, _U32, C.POINTER(PtOptions), _P, _P, C.POINTER(C.c_double)]),
+    "vgb_first_hit_ids": (C.c_int, [_P, _P, C.c_uint64, _P, _U32, _P, _U32, _P, _P, _P, _P, _P, _P]),
     "vgb_texture_update": (C.c_int, [_P, _P, _U32, _U32]),
     "vgb_scene_normal_map": (C.c_int, [_P, _P, _U32, _U32]),
     "vgb_scene_motion": (C.c_int, [_P, _P, _U32]),

@@ -3232,6 +3232,97 @@ VGB_API vgb_status vgb_rasterize(vgb_context* ctx, const vgb_camera* cam, const 
     return vgb::status_of_exception(ctx ? &ctx->err : nullptr);
 }
 
+// ---------------------------------------------------------------- first-hit ids
+// RenderPasses::updateImages' ids (passes.ipp:96-101) from the triangle ids of the flattened scene, one
+// pass over the pixels: the triangle within its instance, the instance, its mesh, the material (0), and
+// the normal in the camera frame (rows of the inverse rotation in glm's order, or zeros).
+namespace {
+
+constexpr uint32_t kIdInstances = 256;   // instances whose table fits the kernel's parameters
+struct IdParams {
+    uint32_t* tri;
+    int32_t *instance, *mesh, *material;
+    const float* normal;
+    float* normal_camera;
+    size_t n;
+    uint32_t first, ninst, rotate;
+    float R[9];
+    const vgb_instance_range* table;     // device table when it does not fit
+    vgb_instance_range small[kIdInstances];
+};
+
+__global__ void k_first_hit_ids(const __grid_constant__ IdParams q) {
+    const vgb_instance_range* t = q.table ? q.table : q.small;
+    for (size_t p = (size_t)blockIdx.x * blockDim.x + threadIdx.x; p < q.n; p += (size_t)gridDim.x * blockDim.x) {
+        const uint32_t id = q.tri[p];
+        int32_t inst = -1, mesh = -1, mat = -1;
+        if (id != VGB_NO_HIT) {
+            const uint32_t f = (int32_t)(id - q.first) > 0 ? id - q.first : 0u;
+            uint32_t lo = 0, hi = q.ninst - 1;   // the last range that starts at or before f
+            while (lo < hi) {
+                const uint32_t mid = (lo + hi + 1) >> 1;
+                if (t[mid].first_triangle <= f) lo = mid; else hi = mid - 1;
+            }
+            q.tri[p] = f - t[lo].first_triangle + q.first;
+            inst = (int32_t)t[lo].instance;
+            mesh = (int32_t)t[lo].mesh;
+            mat = 0;
+        }
+        q.instance[p] = inst;
+        q.mesh[p] = mesh;
+        q.material[p] = mat;
+        if (q.rotate) {
+            const float nx = q.normal[p], ny = q.normal[q.n + p], nz = q.normal[2 * q.n + p];
+#pragma unroll
+            for (int r = 0; r < 3; ++r)
+                q.normal_camera[r * q.n + p] = (nx * q.R[3 * r] + ny * q.R[3 * r + 1]) + nz * q.R[3 * r + 2];
+        } else {
+            q.normal_camera[p] = q.normal_camera[q.n + p] = q.normal_camera[2 * q.n + p] = 0.f;
+        }
+    }
+}
+
+}  // namespace
+
+VGB_API vgb_status vgb_first_hit_ids(vgb_context* ctx, void* stream, uint64_t npixels, uint32_t* tri, uint32_t first,
+                                     const vgb_instance_range* ranges, uint32_t nranges, const float* normal_global,
+                                     const float* rotation, int32_t* instance_id, int32_t* mesh_id, int32_t* material_id,
+                                     float* normal_camera) try {
+    if (!ctx) return VGB_ERR_INVALID_ARGUMENT;
+    if (!tri || !ranges || nranges == 0 || !instance_id || !mesh_id || !material_id || !normal_camera ||
+        (rotation && !normal_global))
+        return fail(ctx, VGB_ERR_INVALID_ARGUMENT, "first_hit_ids: null buffer or no instance");
+    if (npixels == 0) return VGB_OK;
+    cudaSetDevice(ctx->device);
+    IdParams q;
+    std::memset(&q, 0, sizeof(q));
+    q.tri = tri; q.instance = instance_id; q.mesh = mesh_id; q.material = material_id;
+    q.normal = normal_global; q.normal_camera = normal_camera; q.n = (size_t)npixels; q.first = first; q.ninst = nranges;
+    q.rotate = rotation ? 1u : 0u;
+    if (rotation) for (int k = 0; k < 9; ++k) q.R[k] = rotation[k];
+    cudaStream_t s = (cudaStream_t)stream;
+    vgb_instance_range* table = nullptr;
+    if (nranges <= kIdInstances) {
+        std::memcpy(q.small, ranges, sizeof(vgb_instance_range) * nranges);
+    } else {
+        vgb_status e = dalloc(ctx, &table, sizeof(vgb_instance_range) * nranges);
+        if (e != VGB_OK) return e;
+        const cudaError_t ce = cudaMemcpy(table, ranges, sizeof(vgb_instance_range) * nranges, cudaMemcpyHostToDevice);
+        if (ce != cudaSuccess) { dfree(table); CK(ce); }
+        q.table = table;
+    }
+    k_first_hit_ids<<<grid_for(ctx, q.n, 16), 256, 0, s>>>(q);
+    const cudaError_t le = cudaGetLastError();
+    if (table) {
+        cudaStreamSynchronize(s);
+        dfree(table);
+    }
+    CK(le);
+    return VGB_OK;
+} catch (...) {
+    return vgb::status_of_exception(ctx ? &ctx->err : nullptr);
+}
+
 // DEMQuipu::readBuffers (dem_quipu.ipp:124-221): the file's stored codes are read and LZ4-decoded
 // on the host into pinned memory, copied to the device as stored (1-4 bytes per post), and
 // decoded, posed (DEM::makeVertexBuffer), triangulated (imageToIndexBuffer) and given vertex

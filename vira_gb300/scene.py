@@ -477,35 +477,30 @@ class RenderPasses:
 
 def _id_passes(rp: "RenderPasses", scene: "Scene", camera: "Camera", first: int, raster: bool):
     """Turns the device's triangle ids (index in the flattened scene, + `first`) into the reference's
-    per-instance ids and derives instance_id, mesh_id, material_id and normal_camera."""
+    per-instance ids and derives instance_id, mesh_id, material_id and normal_camera, in one pass over
+    the pixels (vgb_first_hit_ids) on torch's current stream."""
     import torch
 
     dev = rp.triangle_id.device
-    tid = rp.triangle_id.to(torch.int64)
-    hit = tid != -1
-    fi = (tid - first).clamp(min=0)
-    offs = scene.flat["tri_offsets"]
-    counts = [n for (_, _, n) in offs]
-    starts = torch.tensor(np.cumsum([0] + counts[:-1]), dtype=torch.int64, device=dev)
-    k = (torch.searchsorted(starts, fi, right=True) - 1).clamp(min=0)
-    inst = torch.tensor([ii for (ii, _, _) in offs], dtype=torch.int64, device=dev)
-    mesh = torch.tensor([scene.instances[ii].mesh for (ii, _, _) in offs], dtype=torch.int64, device=dev)
-    none = torch.full_like(tid, -1)
-    rp.triangle_id = torch.where(hit, fi - starts[k] + first, none).to(torch.int32)
-    rp.instance_id = torch.where(hit, inst[k], none).to(torch.int32)
-    rp.mesh_id = torch.where(hit, mesh[k], none).to(torch.int32)
-    rp.material_id = torch.where(hit, torch.zeros_like(tid), none).to(torch.int32)
-    n = rp.normal_global
-    if raster:
-        # Camera::getViewNormalMatrix (the inverse rotation) times the normal, glm's row sums
-        R = np.asarray(camera.rotation, np.float64).astype(np.float32)
-        rows = []
-        for r in range(3):
-            a, b, c = (float(R[0, r]), float(R[1, r]), float(R[2, r]))
-            rows.append((n[0] * a + n[1] * b) + n[2] * c)
-        rp.normal_camera = torch.stack(rows)
-    else:
-        rp.normal_camera = torch.zeros_like(n)
+    H, W = rp.triangle_id.shape
+    offs = scene._flat["tri_offsets"]
+    table = np.empty((len(offs), 3), np.uint32)
+    start = 0
+    for k, (ii, _, n) in enumerate(offs):
+        table[k] = (start, ii, scene.instances[ii].mesh)
+        start += n
+    rp.instance_id = torch.empty((H, W), dtype=torch.int32, device=dev)
+    rp.mesh_id = torch.empty((H, W), dtype=torch.int32, device=dev)
+    rp.material_id = torch.empty((H, W), dtype=torch.int32, device=dev)
+    rp.normal_camera = torch.empty((3, H, W), dtype=torch.float32, device=dev)
+    # Camera::getViewNormalMatrix (the inverse rotation), for the rasterizer
+    R = np.ascontiguousarray(np.asarray(camera.rotation, np.float64).astype(np.float32).T) if raster else None
+    ctx = scene.context()
+    capi.check(capi.load().vgb_first_hit_ids(ctx, torch.cuda.current_stream(dev).cuda_stream, H * W,
+                                             rp.triangle_id.data_ptr(), first, capi.ptr(table), len(offs),
+                                             rp.normal_global.data_ptr(), capi.ptr(R), rp.instance_id.data_ptr(),
+                                             rp.mesh_id.data_ptr(), rp.material_id.data_ptr(),
+                                             rp.normal_camera.data_ptr()), ctx, "first_hit_ids")
 
 
 class PathTracer:
