@@ -122,9 +122,6 @@ using namespace vgbd;
 #ifndef VGB_SHADOW_GRID
 #define VGB_SHADOW_GRID 60
 #endif
-// k_adjoint (128-thread blocks over the frame's pixels): blocks per SM as above, and pixels per
-// block before the cap.  One pixel per thread replayed the inversion workload's 16 views of 512^2
-// in 0.156 s against 0.169 s at two per thread (16 blocks per SM).
 // k_trace_batch (vgb_trace_rays), in blocks per SM as above: 4.2M device-resident closest-hit rays
 // on a 2049^2 DEM (8.4M triangles) took 0.326 / 1.44 ms (one eye / scattered origins and random
 // directions) at 60 blocks per SM against 0.418 / 2.01 ms at 8.
@@ -148,16 +145,22 @@ using namespace vgbd;
 #ifndef VGB_TRAV_REFILL
 #define VGB_TRAV_REFILL 8
 #endif
+// k_adjoint: blocks per SM, and blocks resident per SM (2 / 3 blocks of 256 threads, 4 blocks of 64 at
+// the same registers: within 2 % of each other on 4 views of 256^2 x 16 spp); k_adjoint_batch: 128-thread
+// blocks resident per SM (2 / 3 / 4 / 5 / 6 / 8 / 10 / 12: 5.6 / 4.7 / 4.4 / 4.25 / 4.1 / 4.0 / 4.1 / 4.2
+// ms for 12 asteroid views; the spills of 64 registers cost less than the idle issue slots).
 #ifndef VGB_ADJOINT_GRID
-#define VGB_ADJOINT_GRID 32
+#define VGB_ADJOINT_GRID 64
 #endif
-#ifndef VGB_ADJOINT_BLOCK_ITEMS
-#define VGB_ADJOINT_BLOCK_ITEMS 128
+#ifndef VGB_ADJOINT_MINB
+#define VGB_ADJOINT_MINB 3
+#endif
+#ifndef VGB_ADJB_MINB
+#define VGB_ADJB_MINB 8
 #endif
 // threads per block of k_adjoint and of k_trace_batch (vgb_trace_rays).  4.2M device-resident
 // closest-hit rays on a 2049^2 DEM: 0.954 / 0.806 ms (from one eye / scattered) at 256 threads,
-// 0.918 / 0.674 at 128, 0.913 / 0.654 at 64.  The inversion workload's backward pass: 0.159 s
-// at 128 threads, 0.154 s at 256 (same threads per SM in the grid), 0.160 s at 64.
+// 0.918 / 0.674 at 128, 0.913 / 0.654 at 64.
 #ifndef VGB_ADJOINT_BLOCK
 #define VGB_ADJOINT_BLOCK 256
 #endif
@@ -1796,6 +1799,8 @@ struct vgb_context {
     void* d_views = nullptr;                 // DevView table of vgb_render_adjoint_batch
     size_t cap_views = 0;
     double* d_loss = nullptr;
+    float4* d_rec = nullptr;                 // hit records of the fused adjoint's resident warps
+    size_t cap_rec = 0;
     // denoiser scratch: ping-pong illumination planes and the render's internal passes
     float* d_dn = nullptr;
     size_t cap_dn = 0;
@@ -2407,7 +2412,7 @@ VGB_API vgb_status vgb_context_destroy(vgb_context* ctx) try {
     if (ctx->graph_exec) cudaGraphExecDestroy(ctx->graph_exec);
     dfree(ctx->d_frames);
     if (ctx->h_frames) cudaFreeHost(ctx->h_frames);
-    dfree(ctx->d_adj); dfree(ctx->d_views); dfree(ctx->d_loss); dfree(ctx->d_dn);
+    dfree(ctx->d_adj); dfree(ctx->d_views); dfree(ctx->d_loss); dfree(ctx->d_rec); dfree(ctx->d_dn);
     if (ctx->h_pin) cudaFreeHost(ctx->h_pin);
     dfree(ctx->d_dirs);
     if (ctx->ev0) cudaEventDestroy(ctx->ev0);
@@ -4773,12 +4778,15 @@ struct AdjOut {
 // Replays one pixel sample and records its path vertices; returns their number.  `g` (dL/dI
 // per band, already divided by the sample count) may be null: no normal gradients are formed.
 // prad receives the sample's path radiance, summed in the order of the forward renderer.
+// rec (or null): one float4 per vertex, `rstride` apart.  Without `again` the closest hits and the
+// lights' visibility are traced and written there; with it they are read back instead of traced.
 template <int NB, int L>
 __device__ __forceinline__ int adj_replay(const DevScene& s, const vgb_camera& cam, const vgb_light* lights,
                                           uint32_t nlights, const vgb_pt_options& opt, uint32_t nb, uint32_t pi,
                                           uint32_t pj, uint32_t slot, uint32_t sample, uint32_t frame,
                                           const float* g, AdjVtx<NB>* vx, float* bgc, float* prad,
-                                          uint32_t& err, uint32_t& nrays) {
+                                          uint32_t& err, uint32_t& nrays, float4* rec = nullptr, uint32_t rstride = 0,
+                                          bool again = false) {
     const uint32_t k0 = (uint32_t)opt.seed, k1 = (uint32_t)(opt.seed >> 32);
     F3 ro, rd;
     pixel_ray(cam, pi, pj, slot, sample, frame, k0, k1, ro, rd);
@@ -4788,11 +4796,24 @@ __device__ __forceinline__ int adj_replay(const DevScene& s, const vgb_camera& c
     int nv = 0;
     for (uint32_t bounce = 0; bounce <= opt.bounces && nv < kAdjMaxVerts; ++bounce) {
         HitOut h;
-        h.U = h.V = h.W = 0.f; h.det = 1.f;
-        const WRay wr = make_wray(ro, rd);
-        trace_ool<L>(s, wr, 0.f, false, h, err);
-        nrays++;
+        float hw0 = 0.f, hw1 = 0.f;
+        uint32_t seen = 0;   // lights whose shadow ray was unoccluded
+        if (again) {
+            const float4 q = rec[bounce * rstride];
+            h.id = __float_as_uint(q.x);
+            hw0 = q.y; hw1 = q.z;
+            seen = __float_as_uint(q.w);
+        } else {
+            h.U = h.V = h.W = 0.f; h.det = 1.f;
+            const WRay wr = make_wray(ro, rd);
+            trace_ool<L>(s, wr, 0.f, false, h, err);
+            nrays++;
+            const float rcp = 1.0f / h.det;
+            hw0 = h.V * rcp;
+            hw1 = h.W * rcp;
+        }
         if (h.id == VGB_NO_HIT) {
+            if (rec && !again) rec[bounce * rstride] = make_float4(__uint_as_float(h.id), 0.f, 0.f, 0.f);
             if (opt.simulate_lighting && opt.show_background) {
                 float x = rd.x, y = rd.y, z = rd.z;
                 float u = atan2f(y, x) / (2 * kPi);
@@ -4811,10 +4832,9 @@ __device__ __forceinline__ int adj_replay(const DevScene& s, const vgb_camera& c
             break;
         }
         AdjVtx<NB>& V = vx[nv++];
-        const float rcp = 1.0f / h.det;
         V.tri = h.id;
-        V.w0 = h.V * rcp;
-        V.w1 = h.W * rcp;
+        V.w0 = hw0;
+        V.w1 = hw1;
         F3 Pp, N, fnrm, tg, bt, nf;
         float uv[2];
         surface_at<NB>(s, nb, opt.smooth_shading != 0, h.id, V.w0, V.w1, Pp, N, fnrm, tg, bt, nf, V.alb, V.va, V.tex, uv);
@@ -4834,7 +4854,10 @@ __device__ __forceinline__ int adj_replay(const DevScene& s, const vgb_camera& c
         V.gnx = V.gny = V.gnz = 0.f;
 #pragma unroll
         for (int k = 0; k < NB; ++k) V.rad[k] = 0.f;
-        if (!opt.simulate_lighting) break;
+        if (!opt.simulate_lighting) {
+            if (rec && !again) rec[bounce * rstride] = make_float4(__uint_as_float(h.id), hw0, hw1, 0.f);
+            break;
+        }
         Pp = F3{offset1(Pp.x, fnrm.x), offset1(Pp.y, fnrm.y), offset1(Pp.z, fnrm.z)};
 #pragma unroll
         for (int k = 0; k < NB; ++k)
@@ -4850,11 +4873,14 @@ __device__ __forceinline__ int adj_replay(const DevScene& s, const vgb_camera& c
             F3 Ld; float dist, lpdf = 0.f;
             light_sample(lights[l], Pp, opt.deterministic_light != 0, ru1, ru2, Ld, dist, lpdf);
             if (!(lpdf > 0)) continue;
-            HitOut hs;
-            const WRay ws = make_wray(Pp, Ld);
-            trace_ool<L>(s, ws, dist, true, hs, err);
-            nrays++;
-            if (hs.id != VGB_NO_HIT) continue;
+            if (!again) {
+                HitOut hs;
+                const WRay ws = make_wray(Pp, Ld);
+                trace_ool<L>(s, ws, dist, true, hs, err);
+                nrays++;
+                if (hs.id == VGB_NO_HIT) seen |= 1u << l;
+            }
+            if (!((seen >> l) & 1u)) continue;
             const float nl = dot(N, Ld);
             const float cos_t = smax(0.0f, dot(Ld, N));
             const float mpdf = (nl <= 0.f) ? 0.f : nl * kInvPi;
@@ -4875,6 +4901,7 @@ __device__ __forceinline__ int adj_replay(const DevScene& s, const vgb_camera& c
                 V.gnx += s_c * Ld.x; V.gny += s_c * Ld.y; V.gnz += s_c * Ld.z;
             }
         }
+        if (rec && !again) rec[bounce * rstride] = make_float4(__uint_as_float(h.id), hw0, hw1, __uint_as_float(seen));
 #pragma unroll
         for (int k = 0; k < NB; ++k) prad[k] = prad[k] + V.rad[k];
         if (bounce >= opt.bounces) break;
@@ -5005,19 +5032,23 @@ __device__ __forceinline__ void adj_scatter(const DevScene& s, uint32_t nb, bool
     }
 }
 
+// A warp per (8x4-pixel tile, sample): the samples of a pixel only meet in the atomic sums, and a
+// view of 256^2 pixels alone is a sixth of the threads the GPU holds.  4 views of 256^2 x 16 spp, 2
+// bounces: 14.9 -> 6.4 ms of backward pass against a thread per pixel.
 template <int NB, int L>
-__global__ void __launch_bounds__(VGB_ADJOINT_BLOCK) k_adjoint(const DevScene s, const __grid_constant__ FrameParams fp,
+__global__ void __launch_bounds__(VGB_ADJOINT_BLOCK, VGB_ADJOINT_MINB) k_adjoint(const DevScene s, const __grid_constant__ FrameParams fp,
                                                  const float* __restrict__ dldi, const AdjOut out, uint32_t* errw,
                                                  uint64_t* stats) {
     const uint32_t nb = fp.nb;
     const vgb_pt_options& opt = fp.opt;
     const uint32_t npix = fp.cam.width * fp.cam.height;
-    const uint32_t n_items = fp.tiles_x * fp.tiles_y * 32u;
+    const uint32_t ln = threadIdx.x & 31u;
+    const size_t n_warps = (size_t)fp.tiles_x * fp.tiles_y * opt.samples;
     const float sf = (float)opt.samples;
     const bool smooth = opt.smooth_shading != 0;
     uint32_t err = 0, nrays = 0;
-    for (uint32_t item = blockIdx.x * blockDim.x + threadIdx.x; item < n_items; item += gridDim.x * blockDim.x) {
-        const uint32_t tile = item >> 5, ln = item & 31u;
+    for (size_t w = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < n_warps; w += ((size_t)gridDim.x * blockDim.x) >> 5) {
+        const uint32_t tile = (uint32_t)(w / opt.samples), sample = (uint32_t)(w - (size_t)tile * opt.samples);
         const uint32_t pi = (tile % fp.tiles_x) * 8u + (ln & 7u), pj = (tile / fp.tiles_x) * 4u + (ln >> 3);
         if (pi >= fp.cam.width || pj >= fp.cam.height) continue;
         const uint32_t slot = pj * fp.cam.width + pi;
@@ -5029,13 +5060,11 @@ __global__ void __launch_bounds__(VGB_ADJOINT_BLOCK) k_adjoint(const DevScene s,
             any |= g[k] != 0.f;
         }
         if (!any) continue;
-        for (uint32_t sample = 0; sample < opt.samples; ++sample) {
-            AdjVtx<NB> vx[kAdjMaxVerts];
-            float bgc[NB], prad[NB];
-            const int nv = adj_replay<NB, L>(s, fp.cam, fp.lights, fp.nlights, opt, nb, pi, pj, slot, sample,
-                                             opt.frame, g, vx, bgc, prad, err, nrays);
-            adj_scatter<NB>(s, nb, smooth, vx, nv, bgc, g, out);
-        }
+        AdjVtx<NB> vx[kAdjMaxVerts];
+        float bgc[NB], prad[NB];
+        const int nv = adj_replay<NB, L>(s, fp.cam, fp.lights, fp.nlights, opt, nb, pi, pj, slot, sample, opt.frame, g,
+                                         vx, bgc, prad, err, nrays);
+        adj_scatter<NB>(s, nb, smooth, vx, nv, bgc, g, out);
     }
     if (err) atomicOr(errw, err);
     warp_reduce_add(&stats[2], nrays);
@@ -5119,17 +5148,21 @@ struct DevView {
 
 struct AdjBatchParams {
     vgb_pt_options opt;
-    uint32_t nviews, nb, total_tiles;
+    uint32_t nviews, nb, total_tiles, max_samples;
 };
 
 // One persistent launch over every (view, 8x4-pixel tile) item; a lane owns a pixel: its
 // samples are traced (forward radiance, in the forward renderer's order), dL/dI = 2 (I - T)
-// is formed and the samples are replayed for the gradients.
+// is formed and the samples are replayed for the gradients, from the hits and the visibility that
+// the first pass left in the warp's records (L2-resident: a few KB a warp), so no ray is traced twice.
 template <int NB, int L>
-__global__ void __launch_bounds__(128) k_adjoint_batch(const DevScene s, const DevView* __restrict__ views,
+__global__ void __launch_bounds__(128, VGB_ADJB_MINB) k_adjoint_batch(const DevScene s, const DevView* __restrict__ views,
                                                        const __grid_constant__ AdjBatchParams bp, const AdjOut out,
                                                        uint32_t* counter, double* loss, uint32_t* errw,
-                                                       uint64_t* stats) {
+                                                       uint64_t* stats, float4* __restrict__ records) {
+    // this warp's records: [samples][bounces + 1][32 lanes], or none
+    const uint32_t nvert = bp.opt.bounces + 1u;
+    float4* rec = records ? records + (((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * bp.max_samples * nvert * 32u + (threadIdx.x & 31u) : nullptr;
     const int lane = threadIdx.x & 31;
     const uint32_t nb = bp.nb;
     const vgb_pt_options& opt = bp.opt;
@@ -5179,7 +5212,9 @@ __global__ void __launch_bounds__(128) k_adjoint_batch(const DevScene s, const D
                 AdjVtx<NB> vx[kAdjMaxVerts];
                 float bgc[NB], prad[NB];
                 const int nv = adj_replay<NB, L>(s, Vw.cam, Vw.lights, Vw.nlights, opt, nb, pi, pj, slot, sample,
-                                                 Vw.frame, pass ? g : nullptr, vx, bgc, prad, err, nrays);
+                                                 Vw.frame, pass ? g : nullptr, vx, bgc, prad, err, nrays,
+                                                 rec ? rec + (size_t)sample * nvert * 32u : nullptr, 32u,
+                                                 rec && pass == 1);
                 if (pass == 0) {
 #pragma unroll
                     for (int k = 0; k < NB; ++k) if (k < (int)nb) acc[k] = acc[k] + prad[k];
@@ -5197,8 +5232,8 @@ __global__ void __launch_bounds__(128) k_adjoint_batch(const DevScene s, const D
 
 template <int NB, int L>
 void launch_adjoint(vgb_context* ctx, const FrameParams& fp, const float* dldi, const AdjOut& out) {
-    const uint32_t n = fp.tiles_x * fp.tiles_y * 32u;
-    const int g = grid_for(ctx, n, VGB_ADJOINT_GRID * 128 / VGB_ADJOINT_BLOCK, VGB_ADJOINT_BLOCK_ITEMS * VGB_ADJOINT_BLOCK / 128);
+    const size_t n = (size_t)fp.tiles_x * fp.tiles_y * 32u * fp.opt.samples;
+    const int g = grid_for(ctx, n, VGB_ADJOINT_GRID, VGB_ADJOINT_BLOCK);
     k_adjoint<NB, L><<<g, VGB_ADJOINT_BLOCK, 0, ctx->stream>>>(dev_scene(ctx), fp, dldi, out, &ctx->d_counters[C_ERR], ctx->d_stats);
 }
 
@@ -5207,8 +5242,18 @@ void launch_adjoint_batch(vgb_context* ctx, const DevView* views, const AdjBatch
     int per_sm = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_adjoint_batch<NB, L>, 128, 0);
     const uint32_t blocks = (uint32_t)std::max(1, per_sm) * (uint32_t)ctx->num_sms;
+    // records of every resident warp; past 1 GiB (or without memory for them) the replay traces again
+    const size_t need = (size_t)blocks * 4 * bp.max_samples * (bp.opt.bounces + 1) * 32 * sizeof(float4);
+    if (need > ctx->cap_rec && need <= (size_t(1) << 30)) {
+        dfree(ctx->d_rec);
+        ctx->d_rec = nullptr;
+        ctx->cap_rec = 0;
+        if (cudaMalloc((void**)&ctx->d_rec, need) == cudaSuccess) ctx->cap_rec = need;
+        else { cudaGetLastError(); ctx->d_rec = nullptr; }
+    }
     k_adjoint_batch<NB, L><<<blocks, 128, 0, ctx->stream>>>(dev_scene(ctx), views, bp, out, &ctx->d_counters[C_BATCH],
-                                                            ctx->d_loss, &ctx->d_counters[C_ERR], ctx->d_stats);
+                                                            ctx->d_loss, &ctx->d_counters[C_ERR], ctx->d_stats,
+                                                            need <= ctx->cap_rec ? ctx->d_rec : nullptr);
 }
 
 template <typename F>
@@ -5359,7 +5404,7 @@ extern "C" VGB_API vgb_status vgb_render_adjoint_batch(vgb_context* ctx, const v
     if (ctx->d_nmap) return fail(ctx, VGB_ERR_INVALID_ARGUMENT, "render_adjoint_batch: normal maps are not differentiated");
     cudaSetDevice(ctx->device);
     std::vector<DevView> hv(nviews);
-    uint32_t tiles = 0;
+    uint32_t tiles = 0, most = 0;
     for (uint32_t i = 0; i < nviews; ++i) {
         const vgb_view& v = views[i];
         if (v.samples == 0 || v.nlights > VGB_MAX_LIGHTS || !v.target || !frame_fits(v.camera.width, v.camera.height))
@@ -5378,6 +5423,7 @@ extern "C" VGB_API vgb_status vgb_render_adjoint_batch(vgb_context* ctx, const v
         const uint64_t t = (uint64_t)tiles + (uint64_t)d.tiles_x * ((v.camera.height + 3) / 4);
         if (t > 0xFFFFFFFFull) return fail(ctx, VGB_ERR_INVALID_ARGUMENT, "render_adjoint_batch: too many tiles");
         tiles = (uint32_t)t;
+        most = std::max(most, v.samples);
     }
     vgb_status s;
     if (nviews * sizeof(DevView) > ctx->cap_views) {
@@ -5398,6 +5444,7 @@ extern "C" VGB_API vgb_status vgb_render_adjoint_batch(vgb_context* ctx, const v
     bp.nviews = nviews;
     bp.nb = ctx->nbands;
     bp.total_tiles = tiles;
+    bp.max_samples = most;
     CK(cudaEventRecord(ctx->ev0, ctx->stream));
     s = run_adjoint(ctx, opts->smooth_shading != 0, d_texture, d_position, nullptr, [&](const AdjOut& out) {
         dispatch_nb_layout(ctx, [&](auto nbc, auto lc) {
