@@ -3609,6 +3609,9 @@ VGB_API vgb_status vgb_get_stats(vgb_context* ctx, vgb_stats* out) try {
     return vgb::status_of_exception(ctx ? &ctx->err : nullptr);
 }
 
+// One frame through the lean direct-lighting kernel of the batch renderer (defined with it).
+static vgb_status launch_direct_frame(vgb_context* ctx, const FrameParams& fp, const FilmOut& film);
+
 static vgb_status check_device_error(vgb_context* ctx) {
     uint32_t e = 0;
     CK(cudaMemcpy(&e, &ctx->d_counters[C_ERR], sizeof(uint32_t), cudaMemcpyDeviceToHost));
@@ -3645,10 +3648,18 @@ VGB_API vgb_status vgb_render(vgb_context* ctx, const vgb_camera* cam, const vgb
     // and the counting pass, which needs counted traversals.
     const bool fused = !opts->adaptive_sampling && ctx->bvh_layout == 2 && !ctx->trav_persistent;
     const uint32_t nq = std::max<uint32_t>(1, nlights);
+    // Without bounces a pixel's samples are summed in one thread's registers (k_batch_direct, one launch,
+    // no planes between launches) where the pixels alone fill the GPU several times over, or once with one
+    // sample: k_front and k_fold / k_batch_direct took 325 / 297 us at 1024^2 x 1 spp, 3.84 / 3.53 ms at
+    // 1024^2 x 16, 554 / 576 us at 512^2 x 8, 316 / 567 us at 256^2 x 16, 35 / 41 us at 96^2 x 1 (4 bands;
+    // the frame table's upload is 5 us of it).
+    // Its film stores are 8-pixel rows of a tile: films across the host link keep k_fold's whole lines.
+    const bool lean = fused && film->on_device && opts->bounces == 0 && 
+                      P >= (opts->samples == 1 ? size_t(1) << 18 : size_t(1) << 20);
     const bool first_hit = film->velocity_global || film->velocity_camera || film->triangle_size;
-    uint32_t chunk = fused ? chunk_samples(P, opts->samples) : 0u;
-    vgb_status s;
-    do {
+    uint32_t chunk = fused && !lean ? chunk_samples(P, opts->samples) : 0u;
+    vgb_status s = VGB_OK;
+    if (!lean || ctx->count_pass) do {
         const size_t items = (chunk && !ctx->count_pass) ? chunk * P : tile_items(cam->width, cam->height);
         s = ensure_scratch(ctx, std::max<size_t>(chunk, 1) * P, items, P, B, nq, chunk && first_hit);
         if (s != VGB_ERR_OUT_OF_MEMORY || chunk <= 1) break;
@@ -3755,7 +3766,11 @@ VGB_API vgb_status vgb_render(vgb_context* ctx, const vgb_camera* cam, const vgb
         launches++;
     }
     st.P = std::max<size_t>(chunk, 1) * P;
-    if (chunk) {
+    if (lean) {
+        Prof p(ctx, 0, true);
+        if ((s = launch_direct_frame(ctx, fp, fr)) != VGB_OK) return s;
+        launches++;
+    } else if (chunk) {
         if (fp.nb <= 1) launch_chunks<1>(ctx, fp, fr, st, chunk, true, launches);
         else if (fp.nb <= 4) launch_chunks<4>(ctx, fp, fr, st, chunk, true, launches);
         else launch_chunks<8>(ctx, fp, fr, st, chunk, true, launches);
@@ -4067,6 +4082,7 @@ struct DevFrame {
     vgb_light lights[VGB_MAX_LIGHTS];
     uint32_t nlights, samples, frame, tiles_x, tile_begin, pad[3];
     FilmOut film;
+    const float4* dirs;   // integer-pixel ray directions (k_direction_table), or null
 };
 
 struct BatchParams {
@@ -4327,7 +4343,7 @@ __global__ void __launch_bounds__(256, VGB_BATCH_LEAN_MINB) k_batch_direct(const
     const vgb_pt_options& opt = bp.opt;
     const uint32_t k0 = (uint32_t)opt.seed, k1 = (uint32_t)(opt.seed >> 32);
     const uint32_t n_items = (bp.total_tiles + bp.tile_stride - 1) / bp.tile_stride;
-    uint32_t err = 0, nclosest = 0, nshadow = 0;
+    uint32_t err = 0, nclosest = 0, nshadow = 0, nhits = 0;
     while (true) {
         uint32_t base = 0;
         if (lane == 0) base = atomicAdd(counter, bp.grab);
@@ -4354,7 +4370,7 @@ __global__ void __launch_bounds__(256, VGB_BATCH_LEAN_MINB) k_batch_direct(const
             uint32_t count = 0, first_tri = VGB_NO_HIT;
             for (uint32_t sample = 0; sample < F.samples; ++sample) {
                 F3 ro{0.f, 0.f, 0.f}, rd{0.f, 0.f, 1.f};
-                if (valid) pixel_ray(F.cam, pi, pj, slot, sample, F.frame, k0, k1, ro, rd);
+                if (valid) pixel_ray(F.cam, pi, pj, slot, sample, F.frame, k0, k1, ro, rd, F.dirs);
                 HitOut h;
                 h.U = h.V = h.W = 0.f; h.det = 1.f;
                 h.id = VGB_NO_HIT;
@@ -4456,6 +4472,7 @@ __global__ void __launch_bounds__(256, VGB_BATCH_LEAN_MINB) k_batch_direct(const
                     }
                 }
             }
+            nhits += count;
             if (!valid) continue;
             // RenderPasses::updateImages for this pixel
             const size_t P = (size_t)W * H;
@@ -4490,6 +4507,7 @@ __global__ void __launch_bounds__(256, VGB_BATCH_LEAN_MINB) k_batch_direct(const
     if (err) atomicOr(errw, err);
     warp_reduce_add(&stats[2], nclosest);
     warp_reduce_add(&stats[3], nshadow);
+    warp_reduce_add(&stats[6], nhits);
 }
 
 // The lean direct-lighting kernel applies when there is no bounce and no adaptive sampling; SUMS
@@ -4557,6 +4575,47 @@ cudaError_t launch_batch_any(vgb_context* ctx, const DevFrame* d_frames, const B
 
 }  // namespace
 
+// The frame table of `n` frames: device memory and its pinned staging.
+static vgb_status ensure_frames(vgb_context* ctx, uint32_t n) {
+    if (n <= ctx->cap_frames) return VGB_OK;
+    dfree(ctx->d_frames);
+    if (ctx->h_frames) cudaFreeHost(ctx->h_frames);
+    ctx->d_frames = nullptr; ctx->h_frames = nullptr; ctx->cap_frames = 0;
+    vgb_status s = dalloc(ctx, &ctx->d_frames, sizeof(DevFrame) * n);
+    if (s != VGB_OK) return s;
+    CK(cudaMallocHost(&ctx->h_frames, sizeof(DevFrame) * n));
+    ctx->cap_frames = n;
+    if (ctx->graph_exec) { cudaGraphExecDestroy(ctx->graph_exec); ctx->graph_exec = nullptr; }
+    return VGB_OK;
+}
+
+static vgb_status launch_direct_frame(vgb_context* ctx, const FrameParams& fp, const FilmOut& film) {
+    vgb_status s = ensure_frames(ctx, 1);
+    if (s != VGB_OK) return s;
+    DevFrame& d = *static_cast<DevFrame*>(ctx->h_frames);
+    std::memset(&d, 0, sizeof(d));
+    d.cam = fp.cam;
+    for (uint32_t l = 0; l < fp.nlights; ++l) d.lights[l] = fp.lights[l];
+    d.nlights = fp.nlights;
+    d.samples = fp.opt.samples;
+    d.frame = fp.opt.frame;
+    d.tiles_x = fp.tiles_x;
+    d.film = film;
+    d.dirs = fp.dirs;
+    CK(cudaMemcpyAsync(ctx->d_frames, &d, sizeof(DevFrame), cudaMemcpyHostToDevice, ctx->stream));
+    BatchParams bp;
+    std::memset(&bp, 0, sizeof(bp));
+    bp.opt = fp.opt;
+    bp.nframes = 1;
+    bp.nb = fp.nb;
+    bp.total_tiles = fp.tiles_x * fp.tiles_y;
+    bp.grab = 1;
+    bp.tile_stride = 1;
+    bp.sums = (film.direct || film.indirect || film.albedo || film.normal) ? 1u : 0u;
+    CK(launch_batch_any(ctx, static_cast<const DevFrame*>(ctx->d_frames), bp, 256, 4));
+    return VGB_OK;
+}
+
 extern "C" VGB_API vgb_status vgb_batch_tuning(vgb_context* ctx, uint32_t* threads, uint32_t* bps, uint32_t* grab) try {
     if (!ctx) return VGB_ERR_INVALID_ARGUMENT;
     if (threads) *threads = ctx->tuned_threads;
@@ -4591,16 +4650,7 @@ extern "C" VGB_API vgb_status vgb_render_batch(vgb_context* ctx, const vgb_frame
     }
     std::stable_sort(order.begin(), order.end(), [&](uint32_t a, uint32_t b) { return frames[a].samples > frames[b].samples; });
     cudaSetDevice(ctx->device);
-    if (nframes > ctx->cap_frames) {
-        dfree(ctx->d_frames);
-        if (ctx->h_frames) cudaFreeHost(ctx->h_frames);
-        ctx->d_frames = nullptr; ctx->h_frames = nullptr; ctx->cap_frames = 0;
-        vgb_status s = dalloc(ctx, &ctx->d_frames, sizeof(DevFrame) * nframes);
-        if (s != VGB_OK) return s;
-        CK(cudaMallocHost(&ctx->h_frames, sizeof(DevFrame) * nframes));
-        ctx->cap_frames = nframes;
-        if (ctx->graph_exec) { cudaGraphExecDestroy(ctx->graph_exec); ctx->graph_exec = nullptr; }
-    }
+    if (const vgb_status s = ensure_frames(ctx, nframes); s != VGB_OK) return s;
     CK(cudaStreamSynchronize(ctx->stream));  // the pinned table may still feed a previous copy
     DevFrame* hf = static_cast<DevFrame*>(ctx->h_frames);
     uint64_t total_tiles = 0;
