@@ -71,7 +71,6 @@ struct WRay {
     F3 o, d;
     int kx, ky, kz;
     float Sx, Sy, Sz;
-    float ix, iy, iz;  // slab reciprocals, |d| clamped away from 0
 };
 
 __device__ __forceinline__ float safe_rcp(float d) {
@@ -93,7 +92,6 @@ __device__ __forceinline__ WRay make_wray(F3 o, F3 d) {
     r.Sx = pick(d, kx) / dz;
     r.Sy = pick(d, ky) / dz;
     r.Sz = 1.0f / dz;
-    r.ix = safe_rcp(d.x); r.iy = safe_rcp(d.y); r.iz = safe_rcp(d.z);
     return r;
 }
 
@@ -160,15 +158,15 @@ struct SlabRay {
 };
 __device__ __forceinline__ SlabRay make_slab(const WRay& r) {
     SlabRay q;
-    q.ix = r.ix; q.iy = r.iy; q.iz = r.iz;
-    const float ox = r.o.x * r.ix, oy = r.o.y * r.iy, oz = r.o.z * r.iz;
+    q.ix = safe_rcp(r.d.x); q.iy = safe_rcp(r.d.y); q.iz = safe_rcp(r.d.z);
+    const float ox = r.o.x * q.ix, oy = r.o.y * q.iy, oz = r.o.z * q.iz;
     const float ex = fabsf(ox) * 0x1p-20f, ey = fabsf(oy) * 0x1p-20f, ez = fabsf(oz) * 0x1p-20f;
-    q.lx = (r.ix >= 0.f) ? (-ox - ex) : (-ox + ex);
-    q.hx = (r.ix >= 0.f) ? (-ox + ex) : (-ox - ex);
-    q.ly = (r.iy >= 0.f) ? (-oy - ey) : (-oy + ey);
-    q.hy = (r.iy >= 0.f) ? (-oy + ey) : (-oy - ey);
-    q.lz = (r.iz >= 0.f) ? (-oz - ez) : (-oz + ez);
-    q.hz = (r.iz >= 0.f) ? (-oz + ez) : (-oz - ez);
+    q.lx = (q.ix >= 0.f) ? (-ox - ex) : (-ox + ex);
+    q.hx = (q.ix >= 0.f) ? (-ox + ex) : (-ox - ex);
+    q.ly = (q.iy >= 0.f) ? (-oy - ey) : (-oy + ey);
+    q.hy = (q.iy >= 0.f) ? (-oy + ey) : (-oy - ey);
+    q.lz = (q.iz >= 0.f) ? (-oz - ez) : (-oz + ez);
+    q.hz = (q.iz >= 0.f) ? (-oz + ez) : (-oz - ez);
     return q;
 }
 
@@ -265,7 +263,7 @@ __device__ __forceinline__ void traverse_rt(const float4* __restrict__ nodes, co
 // box test on the binary nodes (7.91 against 7.38 ms of device time at 512^2, 13.38 against 13.15
 // at 2048^2); walking the children of occlusion rays unsorted lost (2.94 -> 3.16 ms at 512^2).
 //
-// Conservative: m carries a relative error below 4 * 2^-24, so a plane distance m -+ h / |d| is
+// Conservative: m carries a relative error below 6 * 2^-24, so a plane distance m -+ h / |d| is
 // off by at most that part of |distance| + h / |d|; the builder enlarges h (wide_half_extent) by
 // far more than the second part, and the exit distance is widened by 2^-18 for the first, which
 // also covers the rounding of the triangle test's own distance and edge functions.  No box that
@@ -300,13 +298,21 @@ __device__ __forceinline__ void ldg32(const void* p, u64& a, u64& b, u64& c, u64
     asm("ld.global.nc.v4.b64 {%0, %1, %2, %3}, [%4];" : "=l"(a), "=l"(b), "=l"(c), "=l"(d) : "l"(p));
 }
 
+// 1 / d to one unit in the last place, |d| clamped away from 0: enough for the box test's margins.
+__device__ __forceinline__ float approx_rcp(float d) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(fabsf(d) < 1e-30f ? copysignf(1e-30f, d) : d));
+    return r;
+}
+
 // Per-ray constants: minus the origin, 1/d and +-1/|d|, the x and y axes as a pair, z twice.
 struct WideRay { u64 noxy, nozz, ixy, izz, axy, azz, nxy, nzz; };
 __device__ __forceinline__ WideRay make_wide(const WRay& r) {
     WideRay q;
-    const float ax = fabsf(r.ix), ay = fabsf(r.iy), az = fabsf(r.iz);
+    const float ix = approx_rcp(r.d.x), iy = approx_rcp(r.d.y), iz = approx_rcp(r.d.z);
+    const float ax = fabsf(ix), ay = fabsf(iy), az = fabsf(iz);
     q.noxy = pk2(-r.o.x, -r.o.y); q.nozz = pk2(-r.o.z, -r.o.z);
-    q.ixy = pk2(r.ix, r.iy); q.izz = pk2(r.iz, r.iz);
+    q.ixy = pk2(ix, iy); q.izz = pk2(iz, iz);
     q.axy = pk2(ax, ay); q.azz = pk2(az, az);
     q.nxy = pk2(-ax, -ay); q.nzz = pk2(-az, -az);
     return q;
@@ -472,7 +478,8 @@ __device__ __forceinline__ void traverse8_rt(const uint4* __restrict__ nodes, co
     const float widen = 1.0f + 0x1p-20f;
     const uint32_t oct = (r.d.x < 0.f ? 1u : 0u) | (r.d.y < 0.f ? 2u : 0u) | (r.d.z < 0.f ? 4u : 0u);
     // the near plane of an axis is the box's low side for a positive reciprocal, else the high side
-    const bool nx = r.ix < 0.f, ny = r.iy < 0.f, nz = r.iz < 0.f;
+    const float ix = safe_rcp(r.d.x), iy = safe_rcp(r.d.y), iz = safe_rcp(r.d.z);
+    const bool nx = ix < 0.f, ny = iy < 0.f, nz = iz < 0.f;
     uint2 stack[kStack8];
     int sp = 0;
     uint32_t node = 0;
@@ -488,9 +495,9 @@ __device__ __forceinline__ void traverse8_rt(const uint4* __restrict__ nodes, co
         const uint4 w3 = __ldg(&nodes[5 * node + 3]);
         const uint4 w4 = __ldg(&nodes[5 * node + 4]);
         if (COUNT) cnt.nodes++;
-        const AxisPlanes X = axis_planes(__uint_as_float(w0.x), __uint_as_float((w0.w & 0xFFu) << 23), r.o.x, r.ix);
-        const AxisPlanes Y = axis_planes(__uint_as_float(w0.y), __uint_as_float(((w0.w >> 8) & 0xFFu) << 23), r.o.y, r.iy);
-        const AxisPlanes Z = axis_planes(__uint_as_float(w0.z), __uint_as_float(((w0.w >> 16) & 0xFFu) << 23), r.o.z, r.iz);
+        const AxisPlanes X = axis_planes(__uint_as_float(w0.x), __uint_as_float((w0.w & 0xFFu) << 23), r.o.x, ix);
+        const AxisPlanes Y = axis_planes(__uint_as_float(w0.y), __uint_as_float(((w0.w >> 8) & 0xFFu) << 23), r.o.y, iy);
+        const AxisPlanes Z = axis_planes(__uint_as_float(w0.z), __uint_as_float(((w0.w >> 16) & 0xFFu) << 23), r.o.z, iz);
         const uint32_t imask = w0.w >> 24;
         const uint32_t child_base = w1.x, tri_base = w1.y;
         const uint32_t valid = nonzero_bytes(w1.z) | (nonzero_bytes(w1.w) << 4);
