@@ -2566,13 +2566,15 @@ VGB_API vgb_status vgb_scene_upload(vgb_context* ctx, const float* pos, uint32_t
     return vgb::status_of_exception(ctx ? &ctx->err : nullptr);
 }
 
-// The wide nodes of the context's binary BVH.
-static vgb_status build_wide(vgb_context* ctx) {
+// The wide nodes of the context's binary BVH.  too_deep: the tree has more levels than the traversal's
+// stack holds (a binary tree of more than 63 levels, and skewed so that folding does not shorten it).
+static vgb_status build_wide(vgb_context* ctx, bool& too_deep) {
     uint32_t* work = nullptr;
+    uint32_t levels = 0;
     vgb_status s = dalloc(ctx, &work, vgb::wide_work_words(ctx->nnodes) * sizeof(uint32_t));
     if (s != VGB_OK) return s;
     const uint32_t* nodes = reinterpret_cast<const uint32_t*>(ctx->d_nodes);
-    cudaError_t e = (cudaError_t)vgb::launch_wide_fold(ctx->stream, ctx->num_sms, nodes, ctx->nnodes, work, &ctx->nwide);
+    cudaError_t e = (cudaError_t)vgb::launch_wide_fold(ctx->stream, ctx->num_sms, nodes, ctx->nnodes, work, &ctx->nwide, &levels);
     if (e == cudaSuccess) s = dalloc(ctx, &ctx->d_wide, (size_t)ctx->nwide * 128);
     if (e == cudaSuccess && s == VGB_OK)
         e = (cudaError_t)vgb::launch_wide_emit(ctx->stream, ctx->num_sms, nodes, ctx->nnodes, work, ctx->nwide, ctx->d_wide);
@@ -2581,6 +2583,7 @@ static vgb_status build_wide(vgb_context* ctx) {
     if (s != VGB_OK) return s;
     CK(e);
     CK(e2);
+    too_deep = levels > (uint32_t)vgb::kWideLevels;
     ctx->stats.bvh_nodes = ctx->nwide;
     ctx->stats.bvh_node_bytes = 128;
     return VGB_OK;
@@ -2625,7 +2628,9 @@ VGB_API vgb_status vgb_bvh_build(vgb_context* ctx, const vgb_bvh_options* opts) 
         ctx->nnodes = nn;
         ctx->bvh_layout = 2;
         ctx->bvh_leaf = leaf; ctx->bvh_threads = 0;
-        if ((s = build_wide(ctx)) != VGB_OK) return s;
+        bool deep = false;
+        if ((s = build_wide(ctx, deep)) != VGB_OK) return s;
+        if (deep) return fail(ctx, VGB_ERR_INVALID_ARGUMENT, "bvh_build: the tree is too deep to traverse");
         ctx->bvh_ready = true;
         ctx->stats.tri_record_bytes = 48;
         return VGB_OK;
@@ -2664,7 +2669,14 @@ VGB_API vgb_status vgb_bvh_build(vgb_context* ctx, const vgb_bvh_options* opts) 
     ctx->bvh_leaf = leaf; ctx->bvh_threads = threads;
     ctx->stats.bvh_nodes = bvh.num_nodes;
     ctx->stats.bvh_node_bytes = 80;
-    if (layout == 2 && (s = build_wide(ctx)) != VGB_OK) return s;
+    if (layout == 2) {
+        bool deep = false;
+        if ((s = build_wide(ctx, deep)) != VGB_OK) return s;
+        if (deep) {   // Morton order splits at most 63 + 32 times, whatever the triangles
+            const vgb_bvh_options o{leaf, 1u, threads, 2u};
+            return vgb_bvh_build(ctx, &o);
+        }
+    }
     ctx->bvh_ready = true;
     ctx->stats.tri_record_bytes = 48;
     return VGB_OK;

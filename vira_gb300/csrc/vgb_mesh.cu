@@ -606,7 +606,8 @@ WideWork wide_work(uint32_t* work, uint32_t nnodes) {
 }
 }  // namespace
 
-int launch_wide_fold(void* stream, int sms, const uint32_t* nodes, uint32_t nnodes, uint32_t* work, uint32_t* nwide_out) {
+int launch_wide_fold(void* stream, int sms, const uint32_t* nodes, uint32_t nnodes, uint32_t* work, uint32_t* nwide_out,
+                     uint32_t* levels_out) {
     cudaStream_t s = (cudaStream_t)stream;
     const WideWork w = wide_work(work, nnodes);
     const uint32_t one = 1;
@@ -614,6 +615,7 @@ int launch_wide_fold(void* stream, int sms, const uint32_t* nodes, uint32_t nnod
     cudaMemsetAsync(w.flag, 0, ((size_t)nnodes + 1) * sizeof(uint32_t), s);
     cudaMemcpyAsync(w.tail, &one, sizeof(uint32_t), cudaMemcpyHostToDevice, s);
     uint32_t begin = 0, end = 1;
+    *levels_out = 0;
     while (begin < end) {   // one level of wide nodes per pass; every binary node is a root at most once
         k_wide_fold<<<grid(end - begin, sms), 256, 0, s>>>(nodes, w.queue, begin, end, w.src, w.flag, w.tail);
         uint32_t tail = 0;
@@ -622,6 +624,7 @@ int launch_wide_fold(void* stream, int sms, const uint32_t* nodes, uint32_t nnod
         if (e != cudaSuccess) return (int)e;
         begin = end;
         end = tail;
+        ++*levels_out;
     }
     scan(s, w.flag, w.rank, (size_t)nnodes + 1, w.tmp);
     *nwide_out = end;
