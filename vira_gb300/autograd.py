@@ -69,13 +69,7 @@ def _apply_positions(scene: Scene, texture, positions):
 
 def _lights_for(scene: Scene, view: View):
     arr = (capi.Light * 1)()
-    L = scene.lights[0]
-    p = (np.asarray(view.sun_position, np.float64) - scene.origin).astype(np.float32)
-    for a in range(3):
-        arr[0].position[a] = float(p[a])
-    arr[0].radius = float(L.radius)
-    for b in range(scene.bands.size):
-        arr[0].radiance[b] = float(L.radiance[b])
+    scene._light_c(arr[0], scene.lights[0], view.sun_position)
     return arr
 
 

@@ -236,8 +236,8 @@ struct DevState {
 // the persistent closest-hit and occlusion launches (reset with the shadow queues each bounce),
 // the error word and the batch kernels' work counter.
 enum {
-    C_PQ0 = 0, C_SQ = 1, C_FTRACE = 1 + VGB_MAX_LIGHTS, C_FSHADOW = 2 + VGB_MAX_LIGHTS, C_PQ1 = 2 + 2 * VGB_MAX_LIGHTS,
-    C_ERR = 3 + 2 * VGB_MAX_LIGHTS, C_BATCH = 4 + 2 * VGB_MAX_LIGHTS,
+    C_ERR = 0, C_PQ0 = 1, C_SQ = 2, C_FTRACE = 2 + VGB_MAX_LIGHTS, C_FSHADOW = 3 + VGB_MAX_LIGHTS,
+    C_PQ1 = 3 + 2 * VGB_MAX_LIGHTS, C_BATCH = 4 + 2 * VGB_MAX_LIGHTS,
     C_COUNT
 };
 // Counters cleared at the start of every bounce: the shadow queues, the persistent item counters and
@@ -1771,7 +1771,9 @@ struct vgb_context {
     std::vector<void*> scratch;
     DevState st{};
     uint32_t* d_counters = nullptr;
-    uint64_t* d_stats = nullptr;
+    uint64_t* d_stats = nullptr;      // 8 statistics; d_counters follows, the error word first
+    struct Readback { uint64_t stats[8]; uint32_t err; };
+    Readback* h_back = nullptr;       // pinned: what a call reads back with one copy (read_back)
     // staging for host films / host rays
     std::vector<void*> staging;
     size_t staging_bytes = 0;
@@ -2386,14 +2388,15 @@ VGB_API vgb_status vgb_context_create(vgb_context** out, int device) try {
     cudaDeviceGetAttribute(&ctx->num_sms, cudaDevAttrMultiProcessorCount, device);
     if (cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking) != cudaSuccess) { delete ctx; return VGB_ERR_CUDA; }
     ctx->own_stream = true;
-    if (cudaMalloc(&ctx->d_counters, sizeof(uint32_t) * C_COUNT) != cudaSuccess ||
-        cudaMalloc(&ctx->d_stats, sizeof(uint64_t) * 8) != cudaSuccess) {
+    if (cudaMalloc(&ctx->d_stats, sizeof(uint64_t) * 8 + sizeof(uint32_t) * C_COUNT) != cudaSuccess ||
+        cudaMallocHost(&ctx->h_back, sizeof(vgb_context::Readback)) != cudaSuccess) {
+        dfree(ctx->d_stats);
         cudaStreamDestroy(ctx->stream);
         delete ctx;
         return VGB_ERR_OUT_OF_MEMORY;
     }
-    cudaMemset(ctx->d_counters, 0, sizeof(uint32_t) * C_COUNT);
-    cudaMemset(ctx->d_stats, 0, sizeof(uint64_t) * 8);
+    ctx->d_counters = reinterpret_cast<uint32_t*>(ctx->d_stats + 8);
+    cudaMemset(ctx->d_stats, 0, sizeof(uint64_t) * 8 + sizeof(uint32_t) * C_COUNT);
     cudaEventCreate(&ctx->ev0);
     cudaEventCreate(&ctx->ev1);
     *out = ctx;
@@ -2407,7 +2410,8 @@ VGB_API vgb_status vgb_context_destroy(vgb_context* ctx) try {
     cudaSetDevice(ctx->device);
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
     free_scene(ctx); free_bvh(ctx); free_scratch(ctx); free_staging(ctx);
-    dfree(ctx->d_counters); dfree(ctx->d_stats);
+    dfree(ctx->d_stats);
+    if (ctx->h_back) cudaFreeHost(ctx->h_back);
     for (cudaEvent_t e : ctx->prof_events) cudaEventDestroy(e);
     if (ctx->graph_exec) cudaGraphExecDestroy(ctx->graph_exec);
     dfree(ctx->d_frames);
@@ -3624,9 +3628,16 @@ VGB_API vgb_status vgb_get_stats(vgb_context* ctx, vgb_stats* out) try {
 // One frame through the lean direct-lighting kernel of the batch renderer (defined with it).
 static vgb_status launch_direct_frame(vgb_context* ctx, const FrameParams& fp, const FilmOut& film);
 
+// Waits for the stream and brings statistics and the error word back on the way (h_back).
+static cudaError_t read_back(vgb_context* ctx) {
+    const cudaError_t e = cudaMemcpyAsync(ctx->h_back, ctx->d_stats, 8 * sizeof(uint64_t) + sizeof(uint32_t),
+                                          cudaMemcpyDeviceToHost, ctx->stream);
+    return e != cudaSuccess ? e : cudaStreamSynchronize(ctx->stream);
+}
+
+// The error word that read_back brought, as a status; the device's is cleared for the next call.
 static vgb_status check_device_error(vgb_context* ctx) {
-    uint32_t e = 0;
-    CK(cudaMemcpy(&e, &ctx->d_counters[C_ERR], sizeof(uint32_t), cudaMemcpyDeviceToHost));
+    const uint32_t e = ctx->h_back->err;
     ctx->stats.device_error = e;
     if (e) {
         CK(cudaMemset(&ctx->d_counters[C_ERR], 0, sizeof(uint32_t)));
@@ -3802,11 +3813,11 @@ VGB_API vgb_status vgb_render(vgb_context* ctx, const vgb_camera* cam, const vgb
             if (staged[k]) CK(cudaMemcpyAsync(hf[k], df[k], nplane[k] * sizeof(float), cudaMemcpyDeviceToHost, ctx->stream));
         if (tri_staged) CK(cudaMemcpyAsync(film->triangle_id, dtri, P * sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx->stream));
     }
-    CK(cudaStreamSynchronize(ctx->stream));
+    CK(read_back(ctx));
     float ms = 0.f;
     cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
     uint64_t hs[8];
-    CK(cudaMemcpy(hs, ctx->d_stats, sizeof(hs), cudaMemcpyDeviceToHost));
+    std::memcpy(hs, ctx->h_back->stats, sizeof(hs));
     ctx->stats.rays_closest = hs[2];
     ctx->stats.rays_shadow = hs[3];
     ctx->stats.hits_closest = hs[6];
@@ -3841,8 +3852,8 @@ VGB_API vgb_status vgb_render(vgb_context* ctx, const vgb_camera* cam, const vgb
         st.P = P;
         dispatch_render<true>(ctx, fp, none, st, false, l2);
         CK(cudaGetLastError());
-        CK(cudaStreamSynchronize(ctx->stream));
-        CK(cudaMemcpy(hs, ctx->d_stats, sizeof(hs), cudaMemcpyDeviceToHost));
+        CK(read_back(ctx));
+        std::memcpy(hs, ctx->h_back->stats, sizeof(hs));
         ctx->stats.nodes_visited = hs[0];
         ctx->stats.tris_tested = hs[1];
         ctx->stats.nodes_closest = hs[4];
@@ -3914,11 +3925,11 @@ VGB_API vgb_status vgb_trace_rays(vgb_context* ctx, const float* org, const floa
         if (tout && !mp[4]) CK(cudaMemcpyAsync(tout, dt, 4 * (size_t)n, cudaMemcpyDeviceToHost, ctx->stream));
         if (bary && !mp[5]) CK(cudaMemcpyAsync(bary, db, 12 * (size_t)n, cudaMemcpyDeviceToHost, ctx->stream));
     }
-    CK(cudaStreamSynchronize(ctx->stream));
+    CK(read_back(ctx));
     float ms = 0.f;
     cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
     uint64_t hs[8];
-    CK(cudaMemcpy(hs, ctx->d_stats, sizeof(hs), cudaMemcpyDeviceToHost));
+    std::memcpy(hs, ctx->h_back->stats, sizeof(hs));
     ctx->stats.ms_last = ms;
     ctx->stats.kernel_launches = 1;
     ctx->stats.nodes_visited = hs[0];
@@ -4733,6 +4744,7 @@ extern "C" VGB_API vgb_status vgb_render_batch(vgb_context* ctx, const vgb_frame
             }
         ctx->tuned_threads = threads; ctx->tuned_bps = bps; ctx->tuned_grab = grab;
         ctx->tuned_key = tune_key;
+        CK(read_back(ctx));
         CK(cudaMemsetAsync(ctx->d_stats, 0, sizeof(uint64_t) * 8, ctx->stream));
         vgb_status es = check_device_error(ctx);
         if (es != VGB_OK) return es;
@@ -4786,11 +4798,11 @@ extern "C" VGB_API vgb_status vgb_render_batch(vgb_context* ctx, const vgb_frame
         CK(cudaGetLastError());
     }
     CK(cudaEventRecord(ctx->ev1, ctx->stream));
-    CK(cudaStreamSynchronize(ctx->stream));
+    CK(read_back(ctx));
     float ms = 0.f;
     cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
     uint64_t hs[8];
-    CK(cudaMemcpy(hs, ctx->d_stats, sizeof(hs), cudaMemcpyDeviceToHost));
+    std::memcpy(hs, ctx->h_back->stats, sizeof(hs));
     ctx->stats.rays_closest = hs[2];
     ctx->stats.rays_shadow = hs[3];
     ctx->stats.kernel_launches = 1;
@@ -5420,11 +5432,11 @@ vgb_status adjoint_common(vgb_context* ctx, const vgb_camera* cam, const vgb_lig
         if (d_texture) CK(cudaMemcpyAsync(d_texture, gt, ntex * sizeof(float), cudaMemcpyDeviceToHost, ctx->stream));
         if (d_pos) CK(cudaMemcpyAsync(d_pos, gp, npos * sizeof(float), cudaMemcpyDeviceToHost, ctx->stream));
     }
-    CK(cudaStreamSynchronize(ctx->stream));
+    CK(read_back(ctx));
     float ms = 0.f;
     cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
     uint64_t hs[8];
-    CK(cudaMemcpy(hs, ctx->d_stats, sizeof(hs), cudaMemcpyDeviceToHost));
+    std::memcpy(hs, ctx->h_back->stats, sizeof(hs));
     ctx->stats.rays_closest = hs[2];
     ctx->stats.rays_shadow = 0;
     ctx->stats.kernel_launches = 1;
@@ -5517,12 +5529,12 @@ extern "C" VGB_API vgb_status vgb_render_adjoint_batch(vgb_context* ctx, const v
     CK(cudaEventRecord(ctx->ev1, ctx->stream));
     double hl = 0.0;
     CK(cudaMemcpyAsync(&hl, ctx->d_loss, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
-    CK(cudaStreamSynchronize(ctx->stream));
+    CK(read_back(ctx));
     if (loss) *loss = hl;
     float ms = 0.f;
     cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
     uint64_t hs[8];
-    CK(cudaMemcpy(hs, ctx->d_stats, sizeof(hs), cudaMemcpyDeviceToHost));
+    std::memcpy(hs, ctx->h_back->stats, sizeof(hs));
     ctx->stats.rays_closest = hs[2];
     ctx->stats.rays_shadow = 0;
     ctx->stats.kernel_launches = 1;

@@ -179,15 +179,19 @@ class Camera:
         once carries +1 in K and K^-1 and -1 only in its ray directions, behind test and mirror."""
         return np.float32(1.0)
 
-    def kinv(self) -> np.ndarray:
-        """Inverse intrinsic matrix, FP32, through the C ABI (camera.ipp:1526-1568)."""
+    def _kinv_c(self):
+        """Inverse intrinsic matrix through the C ABI, as the ABI's six floats."""
         lib = capi.load()
         out = (C.c_float * 6)()
         W, H = self.resolution
         capi.check(lib.vgb_camera_intrinsics(self.focal_length, self.sensor_size[0], self.sensor_size[1], W, H,
                                              self.principal_point[0], self.principal_point[1], self.skew[0],
                                              self.skew[1], self.intrinsics_z_dir, out), what="camera_intrinsics")
-        return np.array(out[:], np.float32)
+        return out
+
+    def kinv(self) -> np.ndarray:
+        """Inverse intrinsic matrix, FP32, through the C ABI (camera.ipp:1526-1568)."""
+        return np.array(self._kinv_c()[:], np.float32)
 
     def intrinsic_matrix(self) -> np.ndarray:
         """The rows of K, FP32 (camera.ipp:1526-1556): fx, kxy, px, kyx, fy, py with z_dir folded in."""
@@ -213,38 +217,31 @@ class Camera:
     def to_c(self, scene_origin: np.ndarray, nbands: int, kinv=None) -> capi.Camera:
         """The C-ABI camera: FP64 pose rebased on `scene_origin`, then FP32.  `kinv`: the six
         FP32 entries of K^-1 when the caller has them (default: vgb_camera_intrinsics)."""
+        f32 = np.float32
         c = capi.Camera()
         c.width, c.height = self.resolution
-        o = (self.position - scene_origin).astype(np.float32)    # FP64 rebasing, then FP32
-        for k in range(3):
-            c.origin[k] = float(o[k])
-        R = self.rotation.astype(np.float32)
-        for col in range(3):
-            for row in range(3):
-                c.rotation[3 * col + row] = float(R[row, col])
-        kinv = self.kinv() if kinv is None else np.asarray(kinv, np.float32)
-        for k in range(6):
-            c.kinv[k] = float(kinv[k])
+        c.origin[:] = (self.position - scene_origin).astype(f32).tolist()    # FP64 rebasing, then FP32
+        c.rotation[:] = self.rotation.astype(f32).T.ravel().tolist()         # column major
+        c.kinv[:] = self._kinv_c() if kinv is None else np.asarray(kinv, f32).tolist()
         c.z_dir = float(self.z_dir)
-        eff = np.broadcast_to(np.asarray(self.optical_efficiency, np.float32), (nbands,))
         area = self.aperture_area()
-        for k in range(nbands):
-            c.power_scale[k] = float(np.float32(eff[k] * area))
+        if isinstance(self.optical_efficiency, (int, float)):
+            c.power_scale[:nbands] = [float(f32(f32(self.optical_efficiency) * area))] * nbands
+        else:
+            eff = np.broadcast_to(np.asarray(self.optical_efficiency, f32), (nbands,))
+            c.power_scale[:nbands] = (eff * area).astype(f32).tolist()
         if self.distortion is not None:
             c.distortion = int(self.distortion[0])
-            for k, v in enumerate(self.distortion[1]):
-                c.distortion_coeffs[k] = float(v)
+            c.distortion_coeffs[:len(self.distortion[1])] = self.distortion[1].tolist()
         c.interpolate_directions = int(bool(self.interpolate_distortion_directions))
         c.depth_of_field = int(bool(self.depth_of_field))
         c.aperture_radius = float(self.aperture_radius())
         c.focal_length = float(self.focal_length)
         c.focus_distance = float(self.focus_distance)
-        c.sensor_size[0], c.sensor_size[1] = float(self.sensor_size[0]), float(self.sensor_size[1])
-        ro = (self.rotation @ np.asarray(scene_origin, np.float64)).astype(np.float32)
-        for k in range(3):
-            c.velocity[k] = float(np.float32(self.velocity[k]))
-            c.angular_rate[k] = float(np.float32(self.angular_rate[k]))
-            c.rot_origin[k] = float(ro[k])
+        c.sensor_size[:] = [float(self.sensor_size[0]), float(self.sensor_size[1])]
+        c.velocity[:] = np.asarray(self.velocity, np.float64).astype(f32).tolist()
+        c.angular_rate[:] = np.asarray(self.angular_rate, np.float64).astype(f32).tolist()
+        c.rot_origin[:] = (self.rotation @ np.asarray(scene_origin, np.float64)).astype(f32).tolist()
         return c
 
 
@@ -904,13 +901,15 @@ class Scene:
     def c_lights(self):
         arr = (capi.Light * max(1, len(self.lights)))()
         for k, L in enumerate(self.lights):
-            p = (L.position - self.origin).astype(np.float32)
-            for a in range(3):
-                arr[k].position[a] = float(p[a])
-            arr[k].radius = float(L.radius)
-            for b in range(self.bands.size):
-                arr[k].radiance[b] = float(L.radiance[b])
+            self._light_c(arr[k], L, L.position)
         return arr, len(self.lights)
+
+    def _light_c(self, out, light: SphereLight, position):
+        """One light of the C ABI at `position` (FP64, rebased on the scene origin, then FP32)."""
+        out.position[:] = (np.asarray(position, np.float64) - self.origin).astype(np.float32).tolist()
+        out.radius = float(light.radius)
+        n = self.bands.size
+        out.radiance[:n] = np.asarray(light.radiance[:n], np.float32).tolist()
 
     def pixel_solid_angle(self, camera: Camera, cam_c: capi.Camera):
         """Camera::initializePixelSolidAngle (camera.ipp:1622-1666) on the device, FP64, cached."""
@@ -964,12 +963,7 @@ class Scene:
             f.camera = cam
             pos = fr.light_positions if fr.light_positions is not None else [L.position for L in self.lights]
             for k, L in enumerate(self.lights):
-                p = (np.asarray(pos[k], np.float64) - self.origin).astype(np.float32)
-                for a in range(3):
-                    f.lights[k].position[a] = float(p[a])
-                f.lights[k].radius = float(L.radius)
-                for b in range(B):
-                    f.lights[k].radiance[b] = float(L.radiance[b])
+                self._light_c(f.lights[k], L, pos[k])
             f.nlights = len(self.lights)
             f.samples = int(fr.samples)
             f.frame = int(fr.frame)
