@@ -149,6 +149,19 @@ using namespace vgbd;
 // the same registers: within 2 % of each other on 4 views of 256^2 x 16 spp); k_adjoint_batch: 128-thread
 // blocks resident per SM (2 / 3 / 4 / 5 / 6 / 8 / 10 / 12: 5.6 / 4.7 / 4.4 / 4.25 / 4.1 / 4.0 / 4.1 / 4.2
 // ms for 12 asteroid views; the spills of 64 registers cost less than the idle issue slots).
+// k_raster_cover and k_raster_resolve: 64-thread blocks, blocks per SM as above, and k_raster_resolve's
+// resident blocks (64 registers).  Triangles and pixels cost unevenly, and 8 blocks of 256 threads per SM
+// left two thirds of the warp slots idle behind the slowest: 2.1M triangles at 1024^2, 8 bands 152 -> 126
+// us with the cover pass in short blocks, 116 with both.
+#ifndef VGB_RASTER_BLOCK
+#define VGB_RASTER_BLOCK 64
+#endif
+#ifndef VGB_RASTER_GRID
+#define VGB_RASTER_GRID 60
+#endif
+#ifndef VGB_RESOLVE_MINB
+#define VGB_RESOLVE_MINB 4
+#endif
 #ifndef VGB_ADJOINT_GRID
 #define VGB_ADJOINT_GRID 64
 #endif
@@ -3010,7 +3023,7 @@ __device__ __forceinline__ void raster_fragment(unsigned long long* keys, uint32
 
 constexpr uint32_t kRasterSmall = 256;   // box pixels a thread walks by itself
 
-__global__ void k_raster_cover(DevScene s, RasterParams rp, uint32_t ntris, unsigned long long* __restrict__ keys,
+__global__ void __launch_bounds__(VGB_RASTER_BLOCK) k_raster_cover(DevScene s, RasterParams rp, uint32_t ntris, unsigned long long* __restrict__ keys,
                                uint32_t* __restrict__ bigq, uint32_t* __restrict__ nbig) {
     for (size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x; t < ntris; t += (size_t)gridDim.x * blockDim.x) {
         RTri r;
@@ -3052,7 +3065,7 @@ struct RasterOut {
 
 // The winner's passes (cpu_rasterizer.ipp:148-250, passes.ipp:80-128): the fragment is
 // recomputed from its triangle with the same arithmetic as the coverage pass.
-__global__ void k_raster_resolve(DevScene s, RasterParams rp, const unsigned long long* __restrict__ keys,
+__global__ void __launch_bounds__(VGB_RASTER_BLOCK, VGB_RESOLVE_MINB * 256 / VGB_RASTER_BLOCK) k_raster_resolve(DevScene s, RasterParams rp, const unsigned long long* __restrict__ keys,
                                  RasterOut o) {
     const uint32_t W = rp.cam.width, H = rp.cam.height, nb = rp.nb;
     const size_t P = (size_t)W * H;
@@ -3223,9 +3236,9 @@ VGB_API vgb_status vgb_rasterize(vgb_context* ctx, const vgb_camera* cam, const 
     CK(cudaMemsetAsync(keys, 0xFF, P * sizeof(unsigned long long), ctx->stream));
     CK(cudaMemsetAsync(nbig, 0, sizeof(uint32_t), ctx->stream));
     CK(cudaEventRecord(ctx->ev0, ctx->stream));
-    k_raster_cover<<<grid_for(ctx, ctx->ntris, 8), 256, 0, ctx->stream>>>(sc, rp, ctx->ntris, keys, bigq, nbig);
+    k_raster_cover<<<grid_for(ctx, ctx->ntris, VGB_RASTER_GRID * 256 / VGB_RASTER_BLOCK, VGB_RASTER_BLOCK), VGB_RASTER_BLOCK, 0, ctx->stream>>>(sc, rp, ctx->ntris, keys, bigq, nbig);
     k_raster_big<<<ctx->num_sms * 4, 256, 0, ctx->stream>>>(sc, rp, bigq, nbig, keys);
-    k_raster_resolve<<<grid_for(ctx, P, 8), 256, 0, ctx->stream>>>(sc, rp, keys, o);
+    k_raster_resolve<<<grid_for(ctx, P, VGB_RASTER_GRID * 256 / VGB_RASTER_BLOCK, VGB_RASTER_BLOCK), VGB_RASTER_BLOCK, 0, ctx->stream>>>(sc, rp, keys, o);
     CK(cudaGetLastError());
     CK(cudaEventRecord(ctx->ev1, ctx->stream));
     if (!film->on_device) {
