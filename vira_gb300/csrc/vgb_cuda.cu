@@ -30,10 +30,11 @@ using namespace vgbd;
 
 #define VGB_MAX_LIGHTS 8
 
-// Minimum resident blocks per SM requested from the register allocator (occupancy knobs).
-// Defaults from a sweep on the path-traced workload (GB300, 256-thread blocks).
+// Minimum resident blocks per SM (of 256 threads) requested from the register allocator.  k_trace and
+// k_shadow walk wide nodes over the short queues behind k_front: 4 / 5 / 6 blocks 107 / 123 / 127 us of
+// occlusion launches at 512^2 x 16 spp.
 #ifndef VGB_TRACE_MINB
-#define VGB_TRACE_MINB 5
+#define VGB_TRACE_MINB 4
 #endif
 #ifndef VGB_SHADE_MINB
 #define VGB_SHADE_MINB 4
@@ -62,7 +63,7 @@ using namespace vgbd;
 #define VGB_L1_CARVEOUT -1
 #endif
 #ifndef VGB_SHADOW_MINB
-#define VGB_SHADOW_MINB 5
+#define VGB_SHADOW_MINB 4
 #endif
 // the same two knobs for the compressed 8-wide layout (k_trace<8>, k_shadow<NB, 8>)
 #ifndef VGB_TRACE8_MINB
@@ -71,10 +72,15 @@ using namespace vgbd;
 #ifndef VGB_SHADOW8_MINB
 #define VGB_SHADOW8_MINB 5
 #endif
-// k_front: 64-thread blocks resident per SM; 12 / 16 / 20 gave 2.86 / 2.76 / 2.80 ms at 512^2 x 16 spp
-// and 12.0 / 11.5 / 11.6 at 2048^2 x 4 spp.
+// k_front: threads per block and blocks resident per SM (64 registers).  32 / 64 / 128 / 256 / 512 threads
+// at 32 resident warps: 9.64 / 9.47 / 9.32 / 9.54 / 10.05 ms at 2048^2 x 4 spp, 2.35 / 2.31 / 2.27 / 2.30 /
+// 2.45 at 512^2 x 16: the warps of a block start in step and share instruction fetches, but a block waits
+// for its slowest warp.  24 / 36 / 40 warps lost 1-4 %.
+#ifndef VGB_FRONT_BLOCK
+#define VGB_FRONT_BLOCK 128
+#endif
 #ifndef VGB_FRONT_MINB
-#define VGB_FRONT_MINB 16
+#define VGB_FRONT_MINB 8
 #endif
 // Grids of the wavefront kernels after k_front, in 256-thread blocks per SM: their queues hold the
 // few paths that hit a second time (8 / 20 / 60: 2.756 / 2.760 / 2.791 ms at 512^2 x 16 spp).
@@ -1429,7 +1435,7 @@ __global__ void __launch_bounds__(256) k_end_sample(DevState st, const __grid_co
 // ms, 512^2 x 16 spp 7.38 -> 2.76 ms, 2048^2 x 4 spp 13.15 -> 11.5 ms, 1024^2 direct 0.355 -> 0.331 ms.
 // Bound by instruction issue and fetch (56 % of the issue slots, 20 of 32 threads an instruction).
 template <int NB>
-__global__ void __launch_bounds__(64, VGB_FRONT_MINB) k_front(const DevScene s, DevState st, const __grid_constant__ FrameParams fp,
+__global__ void __launch_bounds__(VGB_FRONT_BLOCK, VGB_FRONT_MINB) k_front(const DevScene s, DevState st, const __grid_constant__ FrameParams fp,
                                                   uint32_t sample0, uint32_t nsamples) {
     // Band loops rolled, the bands in local memory (they wait there through each traversal anyway): the
     // kernel is bound by instruction fetch as much as by issue.  2048^2 x 4 spp 8.96 -> 8.70 ms.
@@ -1574,8 +1580,9 @@ __global__ void __launch_bounds__(64, VGB_FRONT_MINB) k_front(const DevScene s, 
 // The chunk's samples of a pixel, summed in sample order (the reference's order, which the FP32
 // sums depend on) after the sums of the chunks before, and on the frame's last chunk the film.
 // blockIdx.y: a band, or after the last one the planes without bands.  Bound by HBM latency: one
-// thread per (pixel, band) keeps (bands + 1) times the loads in flight of a thread per pixel.
-__global__ void __launch_bounds__(256) k_fold(DevState st, const __grid_constant__ FrameParams fp, uint32_t nsamples,
+// thread per (pixel, band) keeps (bands + 1) times the loads in flight of a thread per pixel, and 40
+// registers (6 blocks per SM) more of them than 62 or 32: 2048^2 x 4 spp 809 -> 733 us (817 at 32).
+__global__ void __launch_bounds__(256, 6) k_fold(DevState st, const __grid_constant__ FrameParams fp, uint32_t nsamples,
                                               uint32_t first, uint32_t last, FilmOut f) {
     const size_t P = st.P;
     const uint32_t nb = fp.nb, npix = fp.npix, aux = fp.aux, k = blockIdx.y;
@@ -2056,7 +2063,7 @@ void launch_chunks(vgb_context* ctx, const FrameParams& fp, const FilmOut& film,
         cudaMemsetAsync(&st.counters[C_PQ0], 0, sizeof(uint32_t), ctx->stream);
         {
             Prof p(ctx, 0, prof);
-            k_front<NB><<<(unsigned)((items + 63) / 64), 64, 0, ctx->stream>>>(s, st, fp, s0, n);
+            k_front<NB><<<(unsigned)((items + VGB_FRONT_BLOCK - 1) / VGB_FRONT_BLOCK), VGB_FRONT_BLOCK, 0, ctx->stream>>>(s, st, fp, s0, n);
         }
         launches++;
         const int gt = grid_for(ctx, items, VGB_LATE_GRID * 256 / VGB_TRACE_BLOCK, VGB_TRACE_BLOCK);
