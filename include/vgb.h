@@ -192,19 +192,21 @@ typedef struct vgb_bvh_options {
                                   binary layout only; seconds -> milliseconds at tens of millions of
                                   triangles, at some traversal speed) */
     uint32_t threads;          /* host threads for the build; 0 = all */
-    uint32_t layout;           /* device node layout: 2 = binary (default, 0), 8 = compressed 8-wide */
+    uint32_t layout;           /* device node layout: 2 = binary (default, 0), folded into nodes of four
+                                  children for the traversal, 8 = compressed 8-wide */
 } vgb_bvh_options;
 
 /* ---- statistics of the last render / trace ------------------------------------ */
 typedef struct vgb_stats {
     uint64_t rays_closest;     /* closest-hit queries (primary + bounce) */
     uint64_t rays_shadow;      /* shadow (any-hit) queries */
-    uint64_t nodes_visited;    /* counting pass only: wide nodes visited, all queries */
+    uint64_t nodes_visited;    /* counting pass only: nodes visited, all queries (the folded nodes of layout 2;
+                                  binary ones, 64 bytes, by the occlusion queries of vgb_trace_rays) */
     uint64_t tris_tested;      /* counting pass only: triangle records tested, all queries */
     uint64_t nodes_closest;    /* counting pass only: nodes visited by closest-hit queries */
     uint64_t tris_closest;     /* counting pass only: triangles tested by closest-hit queries */
     uint64_t hits_closest;     /* closest-hit queries that hit (shaded) */
-    uint32_t bvh_nodes;        /* nodes in the device BVH */
+    uint32_t bvh_nodes;        /* nodes of the BVH that the traversal walks */
     uint32_t bvh_node_bytes;   /* bytes per node */
     uint32_t tri_record_bytes; /* bytes per triangle record */
     uint32_t kernel_launches;  /* kernels launched by the last render */

@@ -1,16 +1,21 @@
 // vgb_cuda.cu -- wavefront path-tracing kernels for sm_103a and the C ABI around them.
 //
-// Stages of one render (CPUPathTracer::render, cpu_path_tracer.ipp:29-161), per sample:
-//   k_trace   (bounce 0: camera rays over all pixels, 8x4-pixel warp tiles; bounce b>0: the
-//              compacted queue of live paths)  closest-hit traversal, one hit record per ray;
-//   k_shade   processIntersection for the same items: AOVs, shading point, origin offset, NEE
-//              shadow-ray enqueue (one queue per light), cosine bounce sampling, throughput
-//              update, live-path enqueue (warp ballot);
+// One render (CPUPathTracer::render, cpu_path_tracer.ipp:29-161), per chunk of its samples:
+//   k_front   every path from the camera through its first surface, its shadow rays and its
+//             continuation to the second hit, in registers;
+//   per bounce after that, over the queue of paths that hit again:
+//   k_trace   closest-hit traversal, one hit record per ray;
+//   k_shade   processIntersection: shading point, origin offset, NEE shadow-ray enqueue (one queue
+//             per light), cosine bounce sampling, throughput update, live-path enqueue (warp ballot);
 //   k_shadow  (one launch per light)  occlusion traversal of the queued shadow rays, adding
-//              each unoccluded contribution to the path's per-bounce radiance;
-//   k_end_sample  per pixel: folds the last bounce's radiance into the path and the path into
-//              the pixel; on the last sample writes the RenderPasses planes.
-// Path state, queues and accumulators are structure-of-arrays planes indexed by pixel.
+//             each unoccluded contribution to the path's per-bounce radiance;
+//   k_fold    per pixel and band: the chunk's samples summed in order; after the last chunk the
+//             RenderPasses planes.
+// Adaptive sampling, the 8-wide layout, the persistent traversal, the counting pass and the
+// no-allocation render run k_trace, k_shade and k_shadow from bounce 0 on, a sample at a time, and
+// k_end_sample in k_fold's place; large direct-lighting frames are one launch of k_batch_direct.
+// Path state, queues and accumulators are structure-of-arrays planes indexed by slot: sample in
+// flight * pixels + pixel.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -1785,7 +1790,7 @@ struct vgb_context {
     bool h_pos_stale = false;       // device positions moved by a device-side update
     uint32_t* d_vnl = nullptr;      // per-vertex corner lists of the uploaded mesh (vertex-normal updates)
     // render scratch
-    size_t cap_P = 0, cap_items = 0, cap_npix = 0;
+    size_t cap_P = 0, cap_items = 0, cap_npix = 0, cap_acc = 0;
     bool cap_fh = false;
     uint32_t cap_B = 0, cap_L = 0;
     std::vector<void*> scratch;
@@ -1889,7 +1894,7 @@ void free_bvh(vgb_context* ctx) {
 void free_scratch(vgb_context* ctx) {
     for (void* p : ctx->scratch) dfree(p);
     ctx->scratch.clear();
-    ctx->cap_P = 0; ctx->cap_items = 0; ctx->cap_npix = 0; ctx->cap_B = 0; ctx->cap_L = 0; ctx->cap_fh = false;
+    ctx->cap_P = 0; ctx->cap_items = 0; ctx->cap_npix = 0; ctx->cap_acc = 0; ctx->cap_B = 0; ctx->cap_L = 0; ctx->cap_fh = false;
 }
 void free_staging(vgb_context* ctx) {
     dfree(ctx->staging_base);
@@ -1922,13 +1927,15 @@ vgb_status ensure_staging(vgb_context* ctx, size_t bytes) {
 // bounce-0 launch covers n_items queue items (the frame rounded up to whole 8x4-pixel tiles, so
 // n_items >= P where the wavefront starts the camera rays): the hit records of bounce 0 are indexed
 // by item, the planes kept from sample to sample by pixel, every other plane by slot or by a queue
-// position below P.
-vgb_status ensure_scratch(vgb_context* ctx, size_t P, size_t n_items, size_t npix, uint32_t B, uint32_t L, bool first_hit) {
-    if (P <= ctx->cap_P && n_items <= ctx->cap_items && npix <= ctx->cap_npix && B <= ctx->cap_B && L <= ctx->cap_L &&
-        first_hit <= ctx->cap_fh)
+// position below P.  acc: floats of the sums kept between samples (the wavefront) or chunks.
+vgb_status ensure_scratch(vgb_context* ctx, size_t P, size_t n_items, size_t npix, size_t acc, uint32_t B, uint32_t L,
+                          bool first_hit) {
+    if (P <= ctx->cap_P && n_items <= ctx->cap_items && npix <= ctx->cap_npix && acc <= ctx->cap_acc && B <= ctx->cap_B &&
+        L <= ctx->cap_L && first_hit <= ctx->cap_fh)
         return VGB_OK;
     P = std::max(P, ctx->cap_P);
     npix = std::max(npix, ctx->cap_npix);
+    acc = std::max(acc, ctx->cap_acc);
     first_hit = first_hit || ctx->cap_fh;
     n_items = std::max(std::max(n_items, P), ctx->cap_items);
     B = std::max(B, ctx->cap_B);
@@ -1947,7 +1954,7 @@ vgb_status ensure_scratch(vgb_context* ctx, size_t P, size_t n_items, size_t npi
     AL(st.brad, B * P * f); AL(st.pend, P * u);
     AL(st.adir, B * P * f); AL(st.aalb, B * P * f); AL(st.anrm, 3 * P * f);
     AL(st.adep, P * f); AL(st.acnt, P * u); AL(st.atri, P * u);
-    AL(st.acc, (3 * (size_t)B + 6) * npix * f);
+    AL(st.acc, acc * f);
     st.arad = st.acc;
     st.pfh = nullptr;
     if (first_hit) AL(st.pfh, 7 * P * f);
@@ -1966,7 +1973,7 @@ vgb_status ensure_scratch(vgb_context* ctx, size_t P, size_t n_items, size_t npi
     st.counters = ctx->d_counters;
     st.stats = ctx->d_stats;
     st.P = P;
-    ctx->cap_P = P; ctx->cap_items = n_items; ctx->cap_npix = npix; ctx->cap_B = B; ctx->cap_L = L; ctx->cap_fh = first_hit;
+    ctx->cap_P = P; ctx->cap_items = n_items; ctx->cap_npix = npix; ctx->cap_acc = acc; ctx->cap_B = B; ctx->cap_L = L; ctx->cap_fh = first_hit;
     return VGB_OK;
 }
 
@@ -3704,9 +3711,11 @@ VGB_API vgb_status vgb_render(vgb_context* ctx, const vgb_camera* cam, const vgb
     vgb_status s = VGB_OK;
     if (!lean || ctx->count_pass) do {
         const size_t items = (chunk && !ctx->count_pass) ? chunk * P : tile_items(cam->width, cam->height);
-        s = ensure_scratch(ctx, std::max<size_t>(chunk, 1) * P, items, P, B, nq, chunk && first_hit);
-        if (s != VGB_ERR_OUT_OF_MEMORY || chunk <= 1) break;
-        chunk = chunk / 2;   // no memory for that many samples at a time
+        const size_t sums = chunk == 0 || ctx->count_pass ? B : 0, between = chunk && chunk < opts->samples ? 3 * (size_t)B + 6 : 0;
+        s = ensure_scratch(ctx, std::max<size_t>(chunk, 1) * P, items, P, std::max(sums, between) * P, B, nq,
+                           chunk && first_hit);
+        if (s != VGB_ERR_OUT_OF_MEMORY || chunk == 0) break;
+        chunk = chunk / 2;   // no memory for that many samples at a time; 0: the wavefront, a sample at a time
     } while (true);
     if (s != VGB_OK) return s;
     FrameParams fp;
