@@ -35,19 +35,17 @@ import numpy as np
 
 ROOT = Path(__file__).resolve().parent
 
-# ncu capture of the full path-traced frame: dram__bytes_read.sum + dram__bytes_write.sum of the
-# k_trace launches of one sample, averaged over its four bounces (one pass per launch).
-MEASURED_TRAFFIC = {
-    ("path_traced_dem4097_tex4096_2048px_64spp_3b_rr2_8band", 2): {"k_trace": 103060416.0},
-}
-# ncu counters of k_trace on the path-traced workload at scale 0.25 (1025^2 DEM, 512^2, 4 spp):
-# bounce 0 (camera rays) and bounce 1 (diffuse continuation rays).
+# DRAM bytes (read + write) per launch of a kernel family from an ncu capture of the workload, by
+# (workload, layout); none is held for the present kernels.
+MEASURED_TRAFFIC = {}
+# ncu counters of k_front on the path-traced workload at scale 0.25 (1025^2 DEM, 512^2, 4 spp).
 MEASURED_TRACE_COUNTERS = {
-    "case": "path_traced scale 0.25 (1025^2 DEM + craters, 512^2, 4 spp, 3 bounces)",
-    "issue_active_pct": {"bounce0": 56.4, "bounce1": 48.61},
-    "l1_throughput_pct": {"bounce0": 47.76, "bounce1": 31.07},
-    "threads_per_warp_inst": {"bounce0": 26.05, "bounce1": 16.06},
-    "long_scoreboard_stalls_per_issue": {"bounce0": 5.63, "bounce1": 5.59},
+    "case": "k_front, path_traced scale 0.25 (1025^2 DEM + craters, 512^2, 4 spp, 3 bounces)",
+    "issue_active_pct": 60.3,
+    "l1_throughput_pct": 56.47,
+    "threads_per_warp_inst": 23.06,
+    "long_scoreboard_stalls_per_issue": 3.69,
+    "no_instruction_stalls_per_issue": 1.69,
 }
 L2_PROBE_BYTES = 64 << 20
 sys.path.insert(0, str(ROOT))
