@@ -74,6 +74,8 @@ def _rays(mesh, rng):
             d.append(x - src)                                # not normalised
     o.append(on)                                             # from the surface, any way
     d.append(_unit(rng, 1500) * rng.choice([1e-3, 1.0, 1e3], 1500)[:, None])
+    o.append(on[:300] + 0.1 * e * _unit(rng, 300))           # a direction whose reciprocal is subnormal
+    d.append(_unit(rng, 300) * 3e38)
     o.append(v)                                              # from a vertex, in a plane of the axes
     f = _unit(rng, 1500)
     f[np.arange(1500), rng.integers(0, 3, 1500)] = 0.0

@@ -1727,7 +1727,7 @@ __global__ void __launch_bounds__(VGB_RAYS_BLOCK) k_trace_batch(const DevScene s
         WRay wr = make_wray(o, d);
         HitOut h;
         h.U = h.V = h.W = 0.f; h.det = 1.f;
-        traverse_any_layout<L, ANY, COUNT>(bvh_nodes<L>(s), s.tris, wr, tmax ? tmax[i] : __int_as_float(0x7f800000), h, err, cnt, s.iter_cap);
+        traverse_any_layout<L, ANY, COUNT, false>(bvh_nodes<L>(s), s.tris, wr, tmax ? tmax[i] : __int_as_float(0x7f800000), h, err, cnt, s.iter_cap);
         tri[i] = h.id;
         if (tout) tout[i] = h.t;
         if (bary) {

@@ -300,17 +300,23 @@ __device__ __forceinline__ void ldg32(const void* p, u64& a, u64& b, u64& c, u64
 }
 
 // 1 / d to one unit in the last place, |d| clamped away from 0: enough for the box test's margins.
+// UNIT: |d| <= 1, whose reciprocal is never subnormal; flushing one to 0 would open every box to a
+// direction of 1e38.
+template <bool UNIT>
 __device__ __forceinline__ float approx_rcp(float d) {
+    const float a = fabsf(d) < 1e-30f ? copysignf(1e-30f, d) : d;
     float r;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(fabsf(d) < 1e-30f ? copysignf(1e-30f, d) : d));
+    if (UNIT) asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
+    else asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(a));
     return r;
 }
 
 // Per-ray constants: minus the origin, 1/d and +-1/|d|, the x and y axes as a pair, z twice.
 struct WideRay { u64 noxy, nozz, ixy, izz, axy, azz, nxy, nzz; };
+template <bool UNIT = true>
 __device__ __forceinline__ WideRay make_wide(const WRay& r) {
     WideRay q;
-    const float ix = approx_rcp(r.d.x), iy = approx_rcp(r.d.y), iz = approx_rcp(r.d.z);
+    const float ix = approx_rcp<UNIT>(r.d.x), iy = approx_rcp<UNIT>(r.d.y), iz = approx_rcp<UNIT>(r.d.z);
     const float ax = fabsf(ix), ay = fabsf(iy), az = fabsf(iz);
     q.noxy = pk2(-r.o.x, -r.o.y); q.nozz = pk2(-r.o.z, -r.o.z);
     q.ixy = pk2(ix, iy); q.izz = pk2(iz, iz);
@@ -432,13 +438,13 @@ __device__ __forceinline__ bool traverse4(const uint4* __restrict__ nodes, const
     }
 }
 
-template <bool COUNT>
+template <bool COUNT, bool UNIT = true>
 __device__ __forceinline__ void traverse4_rt(const uint4* __restrict__ nodes, const float4* __restrict__ tris,
                                              const WRay& r, float tmax, const bool any, HitOut& h, uint32_t& err,
                                              Counters& cnt, uint32_t cap) {
     int stack[kStackWide];
     TravState ts = trav_start(tmax, any, h, stack);
-    traverse4<COUNT, false>(nodes, tris, r, make_wide(r), tmax, any, stack, ts, h, err, cnt, cap, 0);
+    traverse4<COUNT, false>(nodes, tris, r, make_wide<UNIT>(r), tmax, any, stack, ts, h, err, cnt, cap, 0);
 }
 
 // ------------------------------------------------------------------ compressed 8-wide traversal
@@ -583,13 +589,13 @@ __device__ __forceinline__ void traverse8(const uint4* __restrict__ nodes, const
 }
 
 // Dispatch on the node layout (2: binary, 4: wide, 8: compressed 8-wide).  `cap`: traversal steps
-// per ray before the ray gives up and sets kErrIter.
-template <int LAYOUT, bool ANY, bool COUNT>
+// per ray before the ray gives up and sets kErrIter.  UNIT: the ray's direction is normalised.
+template <int LAYOUT, bool ANY, bool COUNT, bool UNIT = true>
 __device__ __forceinline__ void traverse_any_layout(const uint4* __restrict__ nodes, const float4* __restrict__ tris,
                                                     const WRay& r, float tmax, HitOut& h, uint32_t& err, Counters& cnt,
                                                     uint32_t cap) {
     if (LAYOUT == 8) traverse8<ANY, COUNT>(nodes, tris, r, tmax, h, err, cnt, cap);
-    else if (LAYOUT == 4) traverse4_rt<COUNT>(nodes, tris, r, tmax, ANY, h, err, cnt, cap);
+    else if (LAYOUT == 4) traverse4_rt<COUNT, UNIT>(nodes, tris, r, tmax, ANY, h, err, cnt, cap);
     else traverse_rt<COUNT>(reinterpret_cast<const float4*>(nodes), tris, r, tmax, ANY, h, err, cnt, cap);
 }
 
