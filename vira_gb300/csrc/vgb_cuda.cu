@@ -182,6 +182,15 @@ using namespace vgbd;
 #ifndef VGB_ADJB_MINB
 #define VGB_ADJB_MINB 8
 #endif
+// k_trace_batch: resident blocks of 256 threads per SM for closest hits (wide nodes) and for occlusion
+// (binary nodes).  2M scattered rays over 2.1M triangles: closest 625 us left to the compiler, 596 / 598 /
+// 615 at 4 / 5 / 6; occlusion 354, 358 / 338 / 337 (30K rays: 55 us, 55 / 63 / 65; 51 throughout).
+#ifndef VGB_RAYS_MINB
+#define VGB_RAYS_MINB 4
+#endif
+#ifndef VGB_RAYS_ANY_MINB
+#define VGB_RAYS_ANY_MINB 5
+#endif
 // threads per block of k_adjoint and of k_trace_batch (vgb_trace_rays).  4.2M device-resident
 // closest-hit rays on a 2049^2 DEM: 0.954 / 0.806 ms (from one eye / scattered) at 256 threads,
 // 0.918 / 0.674 at 128, 0.913 / 0.654 at 64.
@@ -1716,7 +1725,7 @@ __global__ void k_pixel_solid_angle(const __grid_constant__ vgb_camera cam, floa
 
 // ------------------------------------------------------------------ batch trace (TLAS::intersect seam)
 template <int L, bool ANY, bool COUNT>
-__global__ void __launch_bounds__(VGB_RAYS_BLOCK) k_trace_batch(const DevScene s, const float* org, const float* dir, const float* tmax,
+__global__ void __launch_bounds__(VGB_RAYS_BLOCK, (ANY ? VGB_RAYS_ANY_MINB : VGB_RAYS_MINB) * 256 / VGB_RAYS_BLOCK) k_trace_batch(const DevScene s, const float* org, const float* dir, const float* tmax,
                                                uint32_t n, uint32_t* tri, float* tout, float* bary,
                                                uint32_t* counters, uint64_t* stats) {
     uint32_t err = 0;
