@@ -992,7 +992,7 @@ __global__ void __launch_bounds__(256, VGB_TRACEP_MINB) k_trace_p(const DevScene
                     item = it;
                     wr = make_wray(ro, rd);
                     q = make_wide(wr);
-                    ts = trav_start(0.f, false, h, stack);
+                    ts = trav_start(wr, 0.f, false, h, stack);
                     live = true;
                     nclosest++;
                 }
@@ -1052,7 +1052,7 @@ __global__ void __launch_bounds__(256, VGB_SHADOWP_MINB) k_shadow_p(const DevSce
                 tmax = st.sq_tmax[light][it];
                 wr = make_wray(o, d);
                 q = make_wide(wr);
-                ts = trav_start(tmax, true, h, stack);
+                ts = trav_start(wr, tmax, true, h, stack);
                 live = true;
                 nsh++;
             }

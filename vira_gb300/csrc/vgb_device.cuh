@@ -299,16 +299,24 @@ __device__ __forceinline__ void ldg32(const void* p, u64& a, u64& b, u64& c, u64
     asm("ld.global.nc.v4.b64 {%0, %1, %2, %3}, [%4];" : "=l"(a), "=l"(b), "=l"(c), "=l"(d) : "l"(p));
 }
 
-// 1 / d to one unit in the last place, |d| clamped away from 0: enough for the box test's margins.
-// UNIT: |d| <= 1, whose reciprocal is never subnormal; flushing one to 0 would open every box to a
-// direction of 1e38.
+// The box test runs in distances scaled by kWideTime (a power of two: nothing is rounded by it).  A
+// direction component of 0 counts as 1e-30, and in unscaled distances (c - o) / d then overflows from
+// |c - o| = 3.4e8 on: with the centre at -infinity the exit is there too, and a box that holds the ray
+// would be culled.  Scaled, that takes 6e27, beyond what the triangle test's products hold, and a
+// distance only turns subnormal below 2e-19, far under the boxes' margins.  A direction of any length
+// (UNIT false) is divided by its largest component first, |1 / Sz| of the triangle test; the rounding of
+// that is part of the margins below.
+constexpr float kWideTime = 0x1p-64f;
 template <bool UNIT>
-__device__ __forceinline__ float approx_rcp(float d) {
-    const float a = fabsf(d) < 1e-30f ? copysignf(1e-30f, d) : d;
+__device__ __forceinline__ float wide_time(const WRay& r, float t) {
+    return UNIT ? t * kWideTime : t / fabsf(r.Sz) * kWideTime;
+}
+
+// kWideTime / |d| to one unit in the last place, d clamped away from 0: enough for the box test's margins.
+__device__ __forceinline__ float wide_rcp(float d) {
     float r;
-    if (UNIT) asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
-    else asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(a));
-    return r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(fabsf(d)));
+    return fminf(r * kWideTime, 1e30f * kWideTime);
 }
 
 // Per-ray constants: minus the origin, 1/d and +-1/|d|, the x and y axes as a pair, z twice.
@@ -316,7 +324,8 @@ struct WideRay { u64 noxy, nozz, ixy, izz, axy, azz, nxy, nzz; };
 template <bool UNIT = true>
 __device__ __forceinline__ WideRay make_wide(const WRay& r) {
     WideRay q;
-    const float ix = approx_rcp<UNIT>(r.d.x), iy = approx_rcp<UNIT>(r.d.y), iz = approx_rcp<UNIT>(r.d.z);
+    const F3 d = UNIT ? r.d : r.d * fabsf(r.Sz);
+    const float ix = copysignf(wide_rcp(d.x), d.x), iy = copysignf(wide_rcp(d.y), d.y), iz = copysignf(wide_rcp(d.z), d.z);
     const float ax = fabsf(ix), ay = fabsf(iy), az = fabsf(iz);
     q.noxy = pk2(-r.o.x, -r.o.y); q.nozz = pk2(-r.o.z, -r.o.z);
     q.ixy = pk2(ix, iy); q.izz = pk2(iz, iz);
@@ -329,15 +338,16 @@ __device__ __forceinline__ WideRay make_wide(const WRay& r) {
 struct TravState {
     int node;       // next node (>= 0 inner; < 0 a leaf to test; kWideEmpty: finished)
     int sp;         // stack entries, the bottom one included
-    float best;     // closest-hit t so far (tmax for occlusion rays)
+    float best;     // closest-hit t so far (tmax for occlusion rays), in the box test's distances
     uint32_t iter;  // nodes visited
 };
 
-__device__ __forceinline__ TravState trav_start(float tmax, bool any, HitOut& h, int* stack) {
+template <bool UNIT = true>
+__device__ __forceinline__ TravState trav_start(const WRay& r, float tmax, bool any, HitOut& h, int* stack) {
     h.t = __int_as_float(0x7f800000);
     h.id = VGB_NO_HIT;
     stack[0] = kWideEmpty;
-    return TravState{0, 1, any ? tmax : __int_as_float(0x7f800000), 0u};
+    return TravState{0, 1, any ? wide_time<UNIT>(r, tmax) : __int_as_float(0x7f800000), 0u};
 }
 
 // Closest hit (any = false; ties in t go to the smaller id) or occlusion (any = true, any hit
@@ -346,7 +356,7 @@ __device__ __forceinline__ TravState trav_start(float tmax, bool any, HitOut& h,
 // off the stack, which bounds it as well: a descent between two of those is as long as the tree is deep.
 // (Testing both at every node cost 1-2 %: 512^2 x 16 spp 2.36 against 2.32 ms.)  RESUME: stops after `budget` nodes; returns true when the ray is finished (h
 // holds its answer), false when the next call is to continue from ts.
-template <bool COUNT, bool RESUME>
+template <bool COUNT, bool RESUME, bool UNIT = true>
 __device__ __forceinline__ bool traverse4(const uint4* __restrict__ nodes, const float4* __restrict__ tris,
                                           const WRay& r, const WideRay& q, float tmax, const bool any, int* stack,
                                           TravState& ts, HitOut& h, uint32_t& err, Counters& cnt, uint32_t cap,
@@ -430,7 +440,7 @@ __device__ __forceinline__ bool traverse4(const uint4* __restrict__ nodes, const
                     }
                 } else if (tt < h.t || (tt == h.t && id < h.id)) {
                     h.t = tt; h.id = id; h.U = U; h.V = V; h.W = W; h.det = det;
-                    best = tt;
+                    best = wide_time<UNIT>(r, tt);
                 }
             }
         }
@@ -443,8 +453,8 @@ __device__ __forceinline__ void traverse4_rt(const uint4* __restrict__ nodes, co
                                              const WRay& r, float tmax, const bool any, HitOut& h, uint32_t& err,
                                              Counters& cnt, uint32_t cap) {
     int stack[kStackWide];
-    TravState ts = trav_start(tmax, any, h, stack);
-    traverse4<COUNT, false>(nodes, tris, r, make_wide<UNIT>(r), tmax, any, stack, ts, h, err, cnt, cap, 0);
+    TravState ts = trav_start<UNIT>(r, tmax, any, h, stack);
+    traverse4<COUNT, false, UNIT>(nodes, tris, r, make_wide<UNIT>(r), tmax, any, stack, ts, h, err, cnt, cap, 0);
 }
 
 // ------------------------------------------------------------------ compressed 8-wide traversal
