@@ -503,7 +503,8 @@ VGB_API vgb_status vgb_texture_update(vgb_context* ctx, const float* texture, ui
 
 /* The reference's per-instance first-hit ids (passes.ipp:96-101) from a render's triangle ids, in one
  * pass over device planes of `npixels` pixels, queued on `stream` (a cudaStream_t of the context's
- * device, 0 for the default stream) without waiting for it.  tri (in: the flattened scene's triangle
+ * device, 0 for the default stream).  Up to 256 ranges travel with the launch and the call does not
+ * wait for the stream (and can be captured); with more it allocates a table and waits.  tri (in: the flattened scene's triangle
  * id + first, VGB_NO_HIT on a miss; out: the triangle within its instance + first); ranges: the
  * instances in flattening order, ascending first_triangle from 0; normal_camera ([3][npixels]):
  * `rotation` (3 x 3, row major) times normal_global, or zeros when rotation is NULL. */

@@ -3364,7 +3364,8 @@ VGB_API vgb_status vgb_first_hit_ids(vgb_context* ctx, void* stream, uint64_t np
     } else {
         vgb_status e = dalloc(ctx, &table, sizeof(vgb_instance_range) * nranges);
         if (e != VGB_OK) return e;
-        const cudaError_t ce = cudaMemcpy(table, ranges, sizeof(vgb_instance_range) * nranges, cudaMemcpyHostToDevice);
+        // on the caller's stream: one that does not wait for the default stream would start the kernel first
+        const cudaError_t ce = cudaMemcpyAsync(table, ranges, sizeof(vgb_instance_range) * nranges, cudaMemcpyHostToDevice, s);
         if (ce != cudaSuccess) { dfree(table); CK(ce); }
         q.table = table;
     }
