@@ -1827,8 +1827,7 @@ struct vgb_context {
     uint64_t tuned_key = 0;                  // the work they were tuned for
     uint32_t bvh_serial = 0;                 // trees built in this context
     cudaGraphExec_t graph_exec = nullptr;
-    uint64_t graph_key = 0;
-    unsigned char graph_params_probe[1024] = {0};   // kernel parameters the graph was captured with
+    std::vector<unsigned char> graph_launch; // the BatchLaunch that graph_exec holds
     // adjoint
     float* d_adj = nullptr;                  // [nverts][3] vertex-normal gradients, [nverts][3] normal sums,
     size_t cap_adj = 0;                      //   [nverts][3] position gradients (z-only callers)
@@ -1988,6 +1987,7 @@ vgb_status ensure_scratch(vgb_context* ctx, size_t P, size_t n_items, size_t npi
 
 DevScene dev_scene(const vgb_context* ctx) {
     DevScene s;
+    std::memset(&s, 0, sizeof(s));   // padding included: BatchLaunch is compared by its bytes
     s.nodes = ctx->d_nodes; s.wide = ctx->d_wide; s.tris = ctx->d_tris; s.idx = ctx->d_idx; s.vpos = ctx->d_vpos; s.vnrm = ctx->d_vnrm;
     s.vuv = ctx->d_vuv; s.valb = ctx->d_valb; s.tex = ctx->d_tex; s.tw = ctx->tw; s.th = ctx->th;
     s.nmap = ctx->d_nmap; s.nw = ctx->nw; s.nh = ctx->nh;
@@ -4153,6 +4153,14 @@ struct BatchParams {
     uint32_t sums;   // some frame requests a direct, indirect, albedo or normal plane
 };
 
+// What a captured batch launch holds: kernel parameters (the scene's buffers among them), frame table, shape.
+struct BatchLaunch {
+    DevScene scene;
+    BatchParams bp;
+    const DevFrame* frames;
+    uint32_t threads, bps, layout;
+};
+
 __device__ __forceinline__ uint32_t find_frame(const DevFrame* __restrict__ frames, uint32_t n, uint32_t t) {
     uint32_t lo = 0, hi = n - 1;
     while (lo < hi) {
@@ -4794,13 +4802,16 @@ extern "C" VGB_API vgb_status vgb_render_batch(vgb_context* ctx, const vgb_frame
     bp.tile_stride = 1;
     CK(cudaEventRecord(ctx->ev0, ctx->stream));
     if (bo && bo->use_graph) {
-        const uint64_t key = ((uint64_t)nframes << 40) ^ ((uint64_t)total_tiles << 8) ^ ((uint64_t)threads << 4) ^ bps ^
-                             ((uint64_t)grab << 56) ^ ((uint64_t)ctx->nbands << 60) ^ ((uint64_t)ctx->bvh_layout << 20) ^
-                             ((uint64_t)opts->bounces << 24) ^ ((uint64_t)opts->samples << 28);
+        // the graph holds the launch with all of this by value; it is captured again when any of it changes
+        BatchLaunch now;
+        std::memset(&now, 0, sizeof(now));
+        now.scene = dev_scene(ctx);
+        now.bp = bp;
+        now.frames = dfr;
+        now.threads = threads; now.bps = bps; now.layout = ctx->bvh_layout;
         static_assert(sizeof(BatchParams) < 4096, "kernel parameters");
-        // the graph holds the launch with these parameters; rebuild it when they change
-        if (!ctx->graph_exec || ctx->graph_key != key ||
-            std::memcmp(&ctx->graph_params_probe, &bp, sizeof(bp)) != 0) {
+        if (!ctx->graph_exec || ctx->graph_launch.size() != sizeof(now) ||
+            std::memcmp(ctx->graph_launch.data(), &now, sizeof(now)) != 0) {
             if (ctx->graph_exec) { cudaGraphExecDestroy(ctx->graph_exec); ctx->graph_exec = nullptr; }
             cudaGraph_t g = nullptr;
             CK(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
@@ -4811,8 +4822,8 @@ extern "C" VGB_API vgb_status vgb_render_batch(vgb_context* ctx, const vgb_frame
             cudaError_t ie = cudaGraphInstantiate(&ctx->graph_exec, g, 0);
             cudaGraphDestroy(g);
             CK(ie);
-            ctx->graph_key = key;
-            std::memcpy(&ctx->graph_params_probe, &bp, sizeof(bp));
+            const unsigned char* bytes = reinterpret_cast<const unsigned char*>(&now);
+            ctx->graph_launch.assign(bytes, bytes + sizeof(now));
         }
         CK(cudaGraphLaunch(ctx->graph_exec, ctx->stream));
     } else {
