@@ -207,6 +207,7 @@ SIGNATURES = {
     "vgb_get_stats": (C.c_int, [_P, C.POINTER(Stats)]),
     "vgb_set_count_pass": (C.c_int, [_P, C.c_int]),
     "vgb_set_profiling": (C.c_int, [_P, C.c_int]),
+    "vgb_set_scratch_limit": (C.c_int, [_P, C.c_uint64]),
     "vgb_set_traversal_limit": (C.c_int, [_P, C.c_uint32]),
     "vgb_sensor_simulate_rgb": (C.c_int, [_P, _P, _U32, _U32, _U32, _P, _P, _P, C.c_int]),
     "vgb_set_wavefront_tuning": (C.c_int, [_P, C.c_uint32, C.c_uint32, C.c_uint32]),

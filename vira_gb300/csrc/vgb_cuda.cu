@@ -229,6 +229,13 @@ struct DevScene {
 template <int L>
 __device__ __forceinline__ const uint4* bvh_nodes(const DevScene& s) { return L == 4 ? s.wide : s.nodes; }
 
+// Planes of the render scratch (ensure_scratch).
+enum {
+    S_ORG, S_DIR, S_THR, S_PRAD, S_BRAD, S_PEND, S_ADIR, S_AALB, S_ANRM, S_ADEP, S_ACNT, S_ATRI, S_ACC, S_PFH, S_PQ0,
+    S_PQ1, S_HIT, S_AS1, S_AS2, S_ANUM, S_SQ, S_SQ_PLANES = 5
+};
+constexpr int kScratchPlanes = S_SQ + S_SQ_PLANES * VGB_MAX_LIGHTS;
+
 struct DevState {
     // per-pixel path state
     float* org;    // [3][P]
@@ -1799,10 +1806,10 @@ struct vgb_context {
     bool h_pos_stale = false;       // device positions moved by a device-side update
     uint32_t* d_vnl = nullptr;      // per-vertex corner lists of the uploaded mesh (vertex-normal updates)
     // render scratch
-    size_t cap_P = 0, cap_items = 0, cap_npix = 0, cap_acc = 0;
-    bool cap_fh = false;
-    uint32_t cap_B = 0, cap_L = 0;
-    std::vector<void*> scratch;
+    struct Plane { void* p; size_t bytes; };
+    Plane scratch[kScratchPlanes] = {};
+    size_t scratch_limit = 0;                // bytes the planes may take together (vgb_set_scratch_limit), or 0
+    size_t refused_bytes = 0, refused_free = 0;   // the last refused total, and the device's free bytes then
     DevState st{};
     uint32_t* d_counters = nullptr;
     uint64_t* d_stats = nullptr;      // 8 statistics; d_counters follows, the error word first
@@ -1865,6 +1872,7 @@ vgb_status fail(vgb_context* c, vgb_status s, const std::string& msg) {
     do {                                                                                          \
         cudaError_t e_ = (call);                                                                  \
         if (e_ != cudaSuccess) {                                                                  \
+            cudaGetLastError(); /* reported by this call, not by the next */                      \
             return fail(ctx, e_ == cudaErrorMemoryAllocation ? VGB_ERR_OUT_OF_MEMORY : VGB_ERR_CUDA, \
                         std::string(#call) + ": " + cudaGetErrorString(e_));                     \
         }                                                                                         \
@@ -1875,7 +1883,11 @@ vgb_status dalloc(vgb_context* ctx, T** p, size_t bytes) {
     *p = nullptr;
     if (bytes == 0) bytes = 16;
     cudaError_t e = cudaMalloc((void**)p, bytes);
-    if (e != cudaSuccess) return fail(ctx, VGB_ERR_OUT_OF_MEMORY, std::string("cudaMalloc: ") + cudaGetErrorString(e));
+    if (e != cudaSuccess) {
+        cudaGetLastError();   // reported here: a caller that goes on with less must not meet it at its next launch
+        *p = nullptr;
+        return fail(ctx, VGB_ERR_OUT_OF_MEMORY, std::string("cudaMalloc: ") + cudaGetErrorString(e));
+    }
     return VGB_OK;
 }
 
@@ -1900,9 +1912,10 @@ void free_bvh(vgb_context* ctx) {
     ctx->bvh_serial++;
 }
 void free_scratch(vgb_context* ctx) {
-    for (void* p : ctx->scratch) dfree(p);
-    ctx->scratch.clear();
-    ctx->cap_P = 0; ctx->cap_items = 0; ctx->cap_npix = 0; ctx->cap_acc = 0; ctx->cap_B = 0; ctx->cap_L = 0; ctx->cap_fh = false;
+    for (vgb_context::Plane& q : ctx->scratch) {
+        dfree(q.p);
+        q = {nullptr, 0};
+    }
 }
 void free_staging(vgb_context* ctx) {
     dfree(ctx->staging_base);
@@ -1931,57 +1944,97 @@ vgb_status ensure_staging(vgb_context* ctx, size_t bytes) {
     return VGB_OK;
 }
 
+// Grows the planes of `want` (bytes) that are smaller; the others keep their size.  On failure every
+// plane is given back.
+vgb_status grow_scratch(vgb_context* ctx, const size_t* want) {
+    size_t total = 0;
+    for (int i = 0; i < kScratchPlanes; ++i) total += std::max(want[i], ctx->scratch[i].bytes);
+    // A limit is a device that has no more: the allocator itself is made to refuse.
+    const bool over = ctx->scratch_limit && total > ctx->scratch_limit;
+    for (int i = 0; i < kScratchPlanes; ++i) {
+        vgb_context::Plane& q = ctx->scratch[i];
+        if (want[i] <= q.bytes) continue;
+        dfree(q.p);
+        q = {nullptr, 0};
+        const vgb_status s = dalloc(ctx, &q.p, over ? SIZE_MAX >> 1 : want[i]);
+        if (s != VGB_OK) {
+            free_scratch(ctx);
+            size_t free_bytes = 0, all = 0;
+            if (cudaMemGetInfo(&free_bytes, &all) != cudaSuccess) cudaGetLastError();
+            ctx->refused_bytes = total;
+            ctx->refused_free = free_bytes;
+            return s;
+        }
+        q.bytes = want[i];
+    }
+    return VGB_OK;
+}
+
+// Whether `total` bytes of scratch were refused before and the device's free memory has not grown by an
+// eighth of that since: then the render goes on with less without giving back what it holds.
+bool scratch_refused(vgb_context* ctx, size_t total, size_t held) {
+    if (!ctx->refused_bytes || total < ctx->refused_bytes) return false;
+    size_t free_bytes = 0, all = 0;
+    if (cudaMemGetInfo(&free_bytes, &all) != cudaSuccess) { cudaGetLastError(); return false; }
+    return free_bytes + held < ctx->refused_free + ctx->refused_bytes / 8;
+}
+
 // Scratch for P state slots (pixels times samples in flight) of a frame of npix pixels whose
 // bounce-0 launch covers n_items queue items (the frame rounded up to whole 8x4-pixel tiles, so
 // n_items >= P where the wavefront starts the camera rays): the hit records of bounce 0 are indexed
 // by item, the planes kept from sample to sample by pixel, every other plane by slot or by a queue
 // position below P.  acc: floats of the sums kept between samples (the wavefront) or chunks.
+// last: there is no way to render with less, so what was refused before is asked for again.
 vgb_status ensure_scratch(vgb_context* ctx, size_t P, size_t n_items, size_t npix, size_t acc, uint32_t B, uint32_t L,
-                          bool first_hit) {
-    if (P <= ctx->cap_P && n_items <= ctx->cap_items && npix <= ctx->cap_npix && acc <= ctx->cap_acc && B <= ctx->cap_B &&
-        L <= ctx->cap_L && first_hit <= ctx->cap_fh)
-        return VGB_OK;
-    P = std::max(P, ctx->cap_P);
-    npix = std::max(npix, ctx->cap_npix);
-    acc = std::max(acc, ctx->cap_acc);
-    first_hit = first_hit || ctx->cap_fh;
-    n_items = std::max(std::max(n_items, P), ctx->cap_items);
-    B = std::max(B, ctx->cap_B);
-    L = std::max(L, ctx->cap_L);
-    free_scratch(ctx);
-    DevState& st = ctx->st;
-    auto A = [&](auto** p, size_t n) -> vgb_status {
-        vgb_status s = dalloc(ctx, p, n);
-        if (s == VGB_OK) ctx->scratch.push_back((void*)*p);
-        return s;
-    };
-    vgb_status s = VGB_OK;
-    const size_t f = sizeof(float), u = sizeof(uint32_t);
-#define AL(ptr, n) do { s = A(&(ptr), (n)); if (s != VGB_OK) { free_scratch(ctx); return s; } } while (0)
-    AL(st.org, 3 * P * f); AL(st.dir, 3 * P * f); AL(st.thr, B * P * f); AL(st.prad, B * P * f);
-    AL(st.brad, B * P * f); AL(st.pend, P * u);
-    AL(st.adir, B * P * f); AL(st.aalb, B * P * f); AL(st.anrm, 3 * P * f);
-    AL(st.adep, P * f); AL(st.acnt, P * u); AL(st.atri, P * u);
-    AL(st.acc, acc * f);
-    st.arad = st.acc;
-    st.pfh = nullptr;
-    if (first_hit) AL(st.pfh, 7 * P * f);
-    AL(st.pq[0], P * u); AL(st.pq[1], P * u);
-    AL(st.hit, n_items * sizeof(float4));
-    AL(st.as1, npix * f); AL(st.as2, npix * f); AL(st.anum, npix * u);
-    for (uint32_t l = 0; l < VGB_MAX_LIGHTS; ++l) {
-        if (l < L) {
-            AL(st.sq_org[l], 3 * P * f); AL(st.sq_dir[l], 3 * P * f); AL(st.sq_tmax[l], P * f);
-            AL(st.sq_slot[l], P * u); AL(st.sq_con[l], B * P * f);
-        } else {
-            st.sq_org[l] = st.sq_dir[l] = st.sq_tmax[l] = st.sq_con[l] = nullptr; st.sq_slot[l] = nullptr;
-        }
+                          bool first_hit, bool last) {
+    const size_t w = 4;   // bytes of a float or an index
+    size_t want[kScratchPlanes] = {0};
+    want[S_ORG] = want[S_DIR] = want[S_ANRM] = 3 * P * w;
+    want[S_THR] = want[S_PRAD] = want[S_BRAD] = want[S_ADIR] = want[S_AALB] = B * P * w;
+    want[S_PEND] = want[S_ADEP] = want[S_ACNT] = want[S_ATRI] = want[S_PQ0] = want[S_PQ1] = P * w;
+    want[S_ACC] = acc * w;
+    if (first_hit) want[S_PFH] = 7 * P * w;
+    want[S_HIT] = std::max(n_items, P) * sizeof(float4);
+    want[S_AS1] = want[S_AS2] = want[S_ANUM] = npix * w;
+    for (uint32_t l = 0; l < L; ++l) {
+        size_t* q = want + S_SQ + S_SQ_PLANES * l;   // origin, direction, length, slot, contribution
+        q[0] = q[1] = 3 * P * w;
+        q[2] = q[3] = P * w;
+        q[4] = B * P * w;
     }
-#undef AL
+    bool grow = false;
+    size_t held = 0, total = 0, alone = 0;
+    for (int i = 0; i < kScratchPlanes; ++i) {
+        grow |= want[i] > ctx->scratch[i].bytes;
+        held += ctx->scratch[i].bytes;
+        total += std::max(want[i], ctx->scratch[i].bytes);
+        alone += want[i];
+    }
+    if (grow) {
+        vgb_status s = VGB_ERR_OUT_OF_MEMORY;
+        if (last || !scratch_refused(ctx, total, held)) s = grow_scratch(ctx, want);
+        // once more without what earlier calls needed
+        if (s == VGB_ERR_OUT_OF_MEMORY && alone < total && (last || !scratch_refused(ctx, alone, held))) {
+            free_scratch(ctx);
+            s = grow_scratch(ctx, want);
+        }
+        if (s != VGB_OK) return s;
+    }
+    DevState& st = ctx->st;
+    auto F = [&](int i) { return static_cast<float*>(ctx->scratch[i].p); };
+    auto U = [&](int i) { return static_cast<uint32_t*>(ctx->scratch[i].p); };
+    st.org = F(S_ORG); st.dir = F(S_DIR); st.thr = F(S_THR); st.prad = F(S_PRAD); st.brad = F(S_BRAD); st.pend = U(S_PEND);
+    st.adir = F(S_ADIR); st.aalb = F(S_AALB); st.anrm = F(S_ANRM); st.adep = F(S_ADEP); st.acnt = U(S_ACNT);
+    st.atri = U(S_ATRI); st.arad = st.acc = F(S_ACC); st.pfh = F(S_PFH);
+    st.pq[0] = U(S_PQ0); st.pq[1] = U(S_PQ1); st.hit = static_cast<float4*>(ctx->scratch[S_HIT].p);
+    st.as1 = F(S_AS1); st.as2 = F(S_AS2); st.anum = U(S_ANUM);
+    for (uint32_t l = 0; l < VGB_MAX_LIGHTS; ++l) {
+        const int q = S_SQ + S_SQ_PLANES * (int)l;
+        st.sq_org[l] = F(q); st.sq_dir[l] = F(q + 1); st.sq_tmax[l] = F(q + 2); st.sq_slot[l] = U(q + 3); st.sq_con[l] = F(q + 4);
+    }
     st.counters = ctx->d_counters;
     st.stats = ctx->d_stats;
     st.P = P;
-    ctx->cap_P = P; ctx->cap_items = n_items; ctx->cap_npix = npix; ctx->cap_acc = acc; ctx->cap_B = B; ctx->cap_L = L; ctx->cap_fh = first_hit;
     return VGB_OK;
 }
 
@@ -2798,6 +2851,20 @@ VGB_API vgb_status vgb_set_wavefront_tuning(vgb_context* ctx, uint32_t persisten
     ctx->trav_persistent = persistent ? 1u : 0u;
     ctx->trav_budget = budget ? budget : VGB_TRAV_BUDGET;
     ctx->trav_refill = refill ? refill : VGB_TRAV_REFILL;
+    return VGB_OK;
+} catch (...) {
+    return vgb::status_of_exception(ctx ? &ctx->err : nullptr);
+}
+
+VGB_API vgb_status vgb_set_scratch_limit(vgb_context* ctx, uint64_t bytes) try {
+    if (!ctx) return VGB_ERR_INVALID_ARGUMENT;
+    cudaSetDevice(ctx->device);
+    CK(cudaStreamSynchronize(ctx->stream));
+    ctx->scratch_limit = (size_t)bytes;
+    ctx->refused_bytes = 0;
+    size_t held = 0;
+    for (const vgb_context::Plane& q : ctx->scratch) held += q.bytes;
+    if (bytes && held > bytes) free_scratch(ctx);
     return VGB_OK;
 } catch (...) {
     return vgb::status_of_exception(ctx ? &ctx->err : nullptr);
@@ -3723,7 +3790,7 @@ VGB_API vgb_status vgb_render(vgb_context* ctx, const vgb_camera* cam, const vgb
         const size_t items = (chunk && !ctx->count_pass) ? chunk * P : tile_items(cam->width, cam->height);
         const size_t sums = chunk == 0 || ctx->count_pass ? B : 0, between = chunk && chunk < opts->samples ? 3 * (size_t)B + 6 : 0;
         s = ensure_scratch(ctx, std::max<size_t>(chunk, 1) * P, items, P, std::max(sums, between) * P, B, nq,
-                           chunk && first_hit);
+                           chunk && first_hit, chunk == 0);
         if (s != VGB_ERR_OUT_OF_MEMORY || chunk == 0) break;
         chunk = chunk / 2;   // no memory for that many samples at a time; 0: the wavefront, a sample at a time
     } while (true);
