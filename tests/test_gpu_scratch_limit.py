@@ -65,3 +65,22 @@ def test_a_refused_allocation_does_not_fail_the_next_call(gpu):
     _limit(s, 0)
     _render(s, cam)
     s.close()
+
+
+@pytest.mark.parametrize("w,h,samples,bounces,limits", [(1025, 1023, 1, 0, (1,)), (96, 64, 4, 1, (1.7e6, 2e6, 4e6))],
+                         ids=["one_launch", "chunks"])
+def test_no_memory_for_the_direction_table(gpu, w, h, samples, bounces, limits):
+    """A camera with a lens distortion renders the same without its table of directions (one launch less
+    where only the table was refused)."""
+    s, cam = _scene(w, h, bands=3, lights=1)
+    s[cam].set_brown_distortion_coefficients(k1=-0.05, k2=0.01, p1=1e-4, p2=-2e-4)
+    s.pathtracer.options.samples, s.pathtracer.options.bounces = samples, bounces
+    want, launches = _render(s, cam)
+    for limit in limits:
+        _limit(s, limit)
+        for _ in range(2):
+            got, n = _render(s, cam)
+            for k in want:
+                assert np.array_equal(got[k].view(np.uint32), want[k].view(np.uint32)), (limit, k)
+            assert bounces or n == launches - 1
+    s.close()

@@ -1849,9 +1849,9 @@ struct vgb_context {
     // pinned host staging of file payloads (Quipu LoDs)
     void* h_pin = nullptr;
     size_t cap_pin = 0;
-    // integer-pixel ray directions of the render in hand (cameras with a lens distortion)
+    // integer-pixel ray directions of the render in hand (cameras with a lens distortion), part of the scratch
     float4* d_dirs = nullptr;
-    size_t cap_dirs = 0;
+    size_t cap_dirs = 0;                     // bytes
     // device address of vgb_render_noalloc's fixed array, looked up by its first call
     unsigned char* noalloc_base = nullptr;
     // traversal steps per ray before the ray gives up (vgb_set_traversal_limit)
@@ -1916,6 +1916,9 @@ void free_scratch(vgb_context* ctx) {
         dfree(q.p);
         q = {nullptr, 0};
     }
+    dfree(ctx->d_dirs);
+    ctx->d_dirs = nullptr;
+    ctx->cap_dirs = 0;
 }
 void free_staging(vgb_context* ctx) {
     dfree(ctx->staging_base);
@@ -1944,10 +1947,33 @@ vgb_status ensure_staging(vgb_context* ctx, size_t bytes) {
     return VGB_OK;
 }
 
-// Grows the planes of `want` (bytes) that are smaller; the others keep their size.  On failure every
-// plane is given back.
+size_t scratch_held(const vgb_context* ctx) {
+    size_t n = ctx->cap_dirs;
+    for (const vgb_context::Plane& q : ctx->scratch) n += q.bytes;
+    return n;
+}
+
+// Notes that `total` bytes of scratch did not fit.
+void note_refused(vgb_context* ctx, size_t total) {
+    size_t free_bytes = 0, all = 0;
+    if (cudaMemGetInfo(&free_bytes, &all) != cudaSuccess) cudaGetLastError();
+    ctx->refused_bytes = total;
+    ctx->refused_free = free_bytes + scratch_held(ctx);
+}
+
+// Whether `total` bytes of scratch were refused before and the device's free memory has not grown by an
+// eighth of that since: then the render goes on with less without giving back what it holds.
+bool scratch_refused(vgb_context* ctx, size_t total) {
+    if (!ctx->refused_bytes || total < ctx->refused_bytes) return false;
+    size_t free_bytes = 0, all = 0;
+    if (cudaMemGetInfo(&free_bytes, &all) != cudaSuccess) { cudaGetLastError(); return false; }
+    return free_bytes + scratch_held(ctx) < ctx->refused_free + ctx->refused_bytes / 8;
+}
+
+// Grows the planes of `want` (bytes) that are smaller; the others keep their size.  On failure the whole
+// scratch is given back.
 vgb_status grow_scratch(vgb_context* ctx, const size_t* want) {
-    size_t total = 0;
+    size_t total = ctx->cap_dirs;
     for (int i = 0; i < kScratchPlanes; ++i) total += std::max(want[i], ctx->scratch[i].bytes);
     // A limit is a device that has no more: the allocator itself is made to refuse.
     const bool over = ctx->scratch_limit && total > ctx->scratch_limit;
@@ -1959,10 +1985,7 @@ vgb_status grow_scratch(vgb_context* ctx, const size_t* want) {
         const vgb_status s = dalloc(ctx, &q.p, over ? SIZE_MAX >> 1 : want[i]);
         if (s != VGB_OK) {
             free_scratch(ctx);
-            size_t free_bytes = 0, all = 0;
-            if (cudaMemGetInfo(&free_bytes, &all) != cudaSuccess) cudaGetLastError();
-            ctx->refused_bytes = total;
-            ctx->refused_free = free_bytes;
+            note_refused(ctx, total);
             return s;
         }
         q.bytes = want[i];
@@ -1970,13 +1993,19 @@ vgb_status grow_scratch(vgb_context* ctx, const size_t* want) {
     return VGB_OK;
 }
 
-// Whether `total` bytes of scratch were refused before and the device's free memory has not grown by an
-// eighth of that since: then the render goes on with less without giving back what it holds.
-bool scratch_refused(vgb_context* ctx, size_t total, size_t held) {
-    if (!ctx->refused_bytes || total < ctx->refused_bytes) return false;
-    size_t free_bytes = 0, all = 0;
-    if (cudaMemGetInfo(&free_bytes, &all) != cudaSuccess) { cudaGetLastError(); return false; }
-    return free_bytes + held < ctx->refused_free + ctx->refused_bytes / 8;
+// The table of integer-pixel directions of a frame of n pixels, or null where there is no memory for it:
+// then every ray computes the directions around it.
+float4* ensure_directions(vgb_context* ctx, size_t n) {
+    const size_t need = n * sizeof(float4);
+    if (need <= ctx->cap_dirs) return ctx->d_dirs;
+    const size_t total = scratch_held(ctx) - ctx->cap_dirs + need;
+    if (scratch_refused(ctx, total)) return nullptr;
+    dfree(ctx->d_dirs);
+    ctx->cap_dirs = 0;
+    const bool over = ctx->scratch_limit && total > ctx->scratch_limit;
+    if (dalloc(ctx, &ctx->d_dirs, over ? SIZE_MAX >> 1 : need) != VGB_OK) note_refused(ctx, total);
+    else ctx->cap_dirs = need;
+    return ctx->d_dirs;
 }
 
 // Scratch for P state slots (pixels times samples in flight) of a frame of npix pixels whose
@@ -2003,18 +2032,17 @@ vgb_status ensure_scratch(vgb_context* ctx, size_t P, size_t n_items, size_t npi
         q[4] = B * P * w;
     }
     bool grow = false;
-    size_t held = 0, total = 0, alone = 0;
+    size_t total = ctx->cap_dirs, alone = 0;
     for (int i = 0; i < kScratchPlanes; ++i) {
         grow |= want[i] > ctx->scratch[i].bytes;
-        held += ctx->scratch[i].bytes;
         total += std::max(want[i], ctx->scratch[i].bytes);
         alone += want[i];
     }
     if (grow) {
         vgb_status s = VGB_ERR_OUT_OF_MEMORY;
-        if (last || !scratch_refused(ctx, total, held)) s = grow_scratch(ctx, want);
+        if (last || !scratch_refused(ctx, total)) s = grow_scratch(ctx, want);
         // once more without what earlier calls needed
-        if (s == VGB_ERR_OUT_OF_MEMORY && alone < total && (last || !scratch_refused(ctx, alone, held))) {
+        if (s == VGB_ERR_OUT_OF_MEMORY && alone < total && (last || !scratch_refused(ctx, alone))) {
             free_scratch(ctx);
             s = grow_scratch(ctx, want);
         }
@@ -2507,7 +2535,6 @@ VGB_API vgb_status vgb_context_destroy(vgb_context* ctx) try {
     if (ctx->h_frames) cudaFreeHost(ctx->h_frames);
     dfree(ctx->d_adj); dfree(ctx->d_views); dfree(ctx->d_loss); dfree(ctx->d_rec); dfree(ctx->d_dn);
     if (ctx->h_pin) cudaFreeHost(ctx->h_pin);
-    dfree(ctx->d_dirs);
     if (ctx->ev0) cudaEventDestroy(ctx->ev0);
     if (ctx->ev1) cudaEventDestroy(ctx->ev1);
     if (ctx->own_stream && ctx->stream) cudaStreamDestroy(ctx->stream);
@@ -2862,9 +2889,7 @@ VGB_API vgb_status vgb_set_scratch_limit(vgb_context* ctx, uint64_t bytes) try {
     CK(cudaStreamSynchronize(ctx->stream));
     ctx->scratch_limit = (size_t)bytes;
     ctx->refused_bytes = 0;
-    size_t held = 0;
-    for (const vgb_context::Plane& q : ctx->scratch) held += q.bytes;
-    if (bytes && held > bytes) free_scratch(ctx);
+    if (bytes && scratch_held(ctx) > bytes) free_scratch(ctx);
     return VGB_OK;
 } catch (...) {
     return vgb::status_of_exception(ctx ? &ctx->err : nullptr);
@@ -3880,14 +3905,7 @@ VGB_API vgb_status vgb_render(vgb_context* ctx, const vgb_camera* cam, const vgb
     uint32_t launches = 0;
     ctx->prof_used = 0;
     if (cam->distortion && cam->interpolate_directions) {
-        if (P > ctx->cap_dirs) {
-            dfree(ctx->d_dirs);
-            ctx->d_dirs = nullptr;
-            ctx->cap_dirs = 0;
-            if ((s = dalloc(ctx, &ctx->d_dirs, P * sizeof(float4))) != VGB_OK) return s;
-            ctx->cap_dirs = P;
-        }
-        fp.dirs = ctx->d_dirs;
+        fp.dirs = ensure_directions(ctx, P);
     }
     CK(cudaEventRecord(ctx->ev0, ctx->stream));
     if (fp.dirs) {
