@@ -550,8 +550,9 @@ VGB_API vgb_status vgb_measure_l2_read(vgb_context* ctx, uint64_t bytes, uint32_
 VGB_API vgb_status vgb_set_wavefront_tuning(vgb_context* ctx, uint32_t persistent, uint32_t budget, uint32_t refill);
 /* Device memory that the context may keep as vgb_render's scratch, in bytes; 0 (the default) sets no
  * limit.  vgb_render keeps the state of the samples in flight, up to 2^24 of them or one of every pixel,
- * from call to call until the context is destroyed: about 300 bytes each at 8 bands and one light, so up
- * to 5 GB.  With a limit, or on a device without that much memory, a frame renders fewer samples at a
+ * from call to call until the context is destroyed (or another of its allocations needs the memory):
+ * at 8 bands up to 120 bytes each without bounces (the fewer planes the film asks for, the fewer), up to
+ * 296 with bounces and one light, and 64 more for each further light, so up to 5 GB.  With a limit, or on a device without that much memory, a frame renders fewer samples at a
  * time, down to one; less than that needs fails with VGB_ERR_OUT_OF_MEMORY.  The planes are the same
  * whatever the limit.  Scratch above a new limit is given back at once. */
 VGB_API vgb_status vgb_set_scratch_limit(vgb_context* ctx, uint64_t bytes);

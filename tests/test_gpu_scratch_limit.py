@@ -84,3 +84,38 @@ def test_no_memory_for_the_direction_table(gpu, w, h, samples, bounces, limits):
                 assert np.array_equal(got[k].view(np.uint32), want[k].view(np.uint32)), (limit, k)
             assert bounces or n == launches - 1
     s.close()
+
+
+def test_a_direct_frame_asks_for_no_path_state(gpu):
+    """Without bounces a slot holds what the film asks for: at 3 bands 60 bytes with every sum of the
+    path tracer's passes (radiance 12, state 4, direct 12, albedo 12, normal 12, depth 4, triangle 4)."""
+    s, cam = _scene(128, 96, bands=3, lights=4)
+    s.pathtracer.options.samples = 32
+    _limit(s, 128 * 96 * 32 * 60)
+    want, launches = _render(s, cam)
+    assert launches == 2             # one chunk: k_front and k_fold
+    _limit(s, 128 * 96 * 32 * 60 - 1)
+    got, launches = _render(s, cam)
+    assert launches > 2
+    for k in want:
+        assert np.array_equal(got[k].view(np.uint32), want[k].view(np.uint32)), k
+    s.close()
+
+
+def test_scratch_makes_room_for_other_allocations(gpu):
+    """An allocation of another call that the device refuses gives the render scratch back before it fails."""
+    import torch
+
+    s, cam = _scene(512, 511, bands=3, lights=1)
+    s.pathtracer.options.samples, s.pathtracer.options.bounces = 16, 1
+    want, _ = _render(s, cam)        # 4.2M slots of 176 bytes: 740 MB
+    before = torch.cuda.mem_get_info()[0]
+    one = torch.zeros(8, device="cuda")
+    lib, ctx = capi.load(), s.context()
+    # 2.9 TB of planes: refused before any of them is touched
+    assert lib.vgb_psf_convolve(ctx, one.data_ptr(), 300000, 300000, 8, one.data_ptr(), 1, 1, 1) == 3
+    assert torch.cuda.mem_get_info()[0] - before > 500e6
+    got, _ = _render(s, cam)
+    for k in want:
+        assert np.array_equal(got[k].view(np.uint32), want[k].view(np.uint32)), k
+    s.close()

@@ -1878,11 +1878,20 @@ vgb_status fail(vgb_context* c, vgb_status s, const std::string& msg) {
         }                                                                                         \
     } while (0)
 
+void free_scratch(vgb_context* ctx);
+size_t scratch_held(const vgb_context* ctx);
+
+// keep_scratch: the caller is using the render scratch; otherwise that is given back before a refusal.
 template <typename T>
-vgb_status dalloc(vgb_context* ctx, T** p, size_t bytes) {
+vgb_status dalloc(vgb_context* ctx, T** p, size_t bytes, bool keep_scratch = false) {
     *p = nullptr;
     if (bytes == 0) bytes = 16;
     cudaError_t e = cudaMalloc((void**)p, bytes);
+    if (e != cudaSuccess && !keep_scratch && scratch_held(ctx)) {
+        cudaGetLastError();
+        free_scratch(ctx);
+        e = cudaMalloc((void**)p, bytes);
+    }
     if (e != cudaSuccess) {
         cudaGetLastError();   // reported here: a caller that goes on with less must not meet it at its next launch
         *p = nullptr;
@@ -1982,7 +1991,7 @@ vgb_status grow_scratch(vgb_context* ctx, const size_t* want) {
         if (want[i] <= q.bytes) continue;
         dfree(q.p);
         q = {nullptr, 0};
-        const vgb_status s = dalloc(ctx, &q.p, over ? SIZE_MAX >> 1 : want[i]);
+        const vgb_status s = dalloc(ctx, &q.p, over ? SIZE_MAX >> 1 : want[i], true);
         if (s != VGB_OK) {
             free_scratch(ctx);
             note_refused(ctx, total);
@@ -2003,34 +2012,58 @@ float4* ensure_directions(vgb_context* ctx, size_t n) {
     dfree(ctx->d_dirs);
     ctx->cap_dirs = 0;
     const bool over = ctx->scratch_limit && total > ctx->scratch_limit;
-    if (dalloc(ctx, &ctx->d_dirs, over ? SIZE_MAX >> 1 : need) != VGB_OK) note_refused(ctx, total);
+    if (dalloc(ctx, &ctx->d_dirs, over ? SIZE_MAX >> 1 : need, true) != VGB_OK) note_refused(ctx, total);
     else ctx->cap_dirs = need;
     return ctx->d_dirs;
 }
 
-// Scratch for P state slots (pixels times samples in flight) of a frame of npix pixels whose
-// bounce-0 launch covers n_items queue items (the frame rounded up to whole 8x4-pixel tiles, so
-// n_items >= P where the wavefront starts the camera rays): the hit records of bounce 0 are indexed
-// by item, the planes kept from sample to sample by pixel, every other plane by slot or by a queue
-// position below P.  acc: floats of the sums kept between samples (the wavefront) or chunks.
-// last: there is no way to render with less, so what was refused before is asked for again.
-vgb_status ensure_scratch(vgb_context* ctx, size_t P, size_t n_items, size_t npix, size_t acc, uint32_t B, uint32_t L,
-                          bool first_hit, bool last) {
+// What the wavefront kernels need for a frame of P pixels, a sample at a time.  n_items: the queue items
+// of the bounce-0 launch (the frame rounded up to whole 8x4-pixel tiles), by which that launch's hit
+// records are indexed; every other plane is indexed by pixel or by a queue position below P.
+void want_wavefront(size_t* want, size_t P, size_t n_items, uint32_t B, uint32_t lights) {
     const size_t w = 4;   // bytes of a float or an index
-    size_t want[kScratchPlanes] = {0};
-    want[S_ORG] = want[S_DIR] = want[S_ANRM] = 3 * P * w;
-    want[S_THR] = want[S_PRAD] = want[S_BRAD] = want[S_ADIR] = want[S_AALB] = B * P * w;
-    want[S_PEND] = want[S_ADEP] = want[S_ACNT] = want[S_ATRI] = want[S_PQ0] = want[S_PQ1] = P * w;
-    want[S_ACC] = acc * w;
-    if (first_hit) want[S_PFH] = 7 * P * w;
-    want[S_HIT] = std::max(n_items, P) * sizeof(float4);
-    want[S_AS1] = want[S_AS2] = want[S_ANUM] = npix * w;
-    for (uint32_t l = 0; l < L; ++l) {
-        size_t* q = want + S_SQ + S_SQ_PLANES * l;   // origin, direction, length, slot, contribution
-        q[0] = q[1] = 3 * P * w;
-        q[2] = q[3] = P * w;
-        q[4] = B * P * w;
+    auto need = [&](int i, size_t bytes) { want[i] = std::max(want[i], bytes); };
+    for (int i : {S_ORG, S_DIR, S_ANRM}) need(i, 3 * P * w);
+    for (int i : {S_THR, S_PRAD, S_BRAD, S_ADIR, S_AALB, S_ACC}) need(i, B * P * w);
+    for (int i : {S_PEND, S_ADEP, S_ACNT, S_ATRI, S_PQ0, S_PQ1, S_AS1, S_AS2, S_ANUM}) need(i, P * w);
+    need(S_HIT, n_items * sizeof(float4));
+    for (uint32_t l = 0; l < std::max<uint32_t>(1, lights); ++l) {
+        const int q = S_SQ + S_SQ_PLANES * (int)l;   // origin, direction, length, slot, contribution
+        need(q, 3 * P * w); need(q + 1, 3 * P * w); need(q + 2, P * w); need(q + 3, P * w); need(q + 4, B * P * w);
     }
+}
+
+// What k_front, the bounces after it and k_fold need for P state slots (the frame's pixels times the
+// samples in flight): only the sums that the film asks for (aux), and path state and queues, indexed by
+// slot or by a queue position below P, only for a frame with bounces.  acc: floats of the sums kept
+// between chunks of samples.
+void want_chunks(size_t* want, size_t P, size_t acc, uint32_t B, uint32_t lights, uint32_t bounces, uint32_t aux,
+                 bool first_hit) {
+    const size_t w = 4;
+    auto need = [&](int i, size_t bytes) { want[i] = std::max(want[i], bytes); };
+    need(S_PRAD, B * P * w);
+    need(S_PEND, P * w);
+    need(S_ACC, acc * w);
+    if (aux & AUX_DIR) need(S_ADIR, B * P * w);
+    if (aux & AUX_ALB) need(S_AALB, B * P * w);
+    if (aux & AUX_NRM) need(S_ANRM, 3 * P * w);
+    if (aux & AUX_DEP) need(S_ADEP, P * w);
+    if (aux & AUX_TRI) need(S_ATRI, P * w);
+    if (first_hit) need(S_PFH, 7 * P * w);
+    if (bounces == 0) return;
+    need(S_ORG, 3 * P * w); need(S_DIR, 3 * P * w);
+    need(S_THR, B * P * w); need(S_BRAD, B * P * w);
+    need(S_PQ0, P * w); need(S_PQ1, P * w);
+    need(S_HIT, P * sizeof(float4));
+    for (uint32_t l = 0; l < lights; ++l) {
+        const int q = S_SQ + S_SQ_PLANES * (int)l;
+        need(q, 3 * P * w); need(q + 1, 3 * P * w); need(q + 2, P * w); need(q + 3, P * w); need(q + 4, B * P * w);
+    }
+}
+
+// The scratch planes of at least `want` bytes, and ctx->st pointing at them.
+// last: there is no way to render with less, so what was refused before is asked for again.
+vgb_status ensure_scratch(vgb_context* ctx, const size_t* want, bool last) {
     bool grow = false;
     size_t total = ctx->cap_dirs, alone = 0;
     for (int i = 0; i < kScratchPlanes; ++i) {
@@ -2062,7 +2095,6 @@ vgb_status ensure_scratch(vgb_context* ctx, size_t P, size_t n_items, size_t npi
     }
     st.counters = ctx->d_counters;
     st.stats = ctx->d_stats;
-    st.P = P;
     return VGB_OK;
 }
 
@@ -3799,27 +3831,16 @@ VGB_API vgb_status vgb_render(vgb_context* ctx, const vgb_camera* cam, const vgb
     // sampling, whose next sample depends on the last, the 8-wide layout, the persistent traversal
     // and the counting pass, which needs counted traversals.
     const bool fused = !opts->adaptive_sampling && ctx->bvh_layout == 2 && !ctx->trav_persistent;
-    const uint32_t nq = std::max<uint32_t>(1, nlights);
     // Without bounces a pixel's samples are summed in one thread's registers (k_batch_direct, one launch,
     // no planes between launches) where the pixels alone fill the GPU several times over, or once with one
     // sample: k_front and k_fold / k_batch_direct took 325 / 297 us at 1024^2 x 1 spp, 3.84 / 3.53 ms at
     // 1024^2 x 16, 554 / 576 us at 512^2 x 8, 316 / 567 us at 256^2 x 16, 35 / 41 us at 96^2 x 1 (4 bands;
     // the frame table's upload is 5 us of it).
     // Its film stores are 8-pixel rows of a tile: films across the host link keep k_fold's whole lines.
-    const bool lean = fused && film->on_device && opts->bounces == 0 && 
+    const bool lean = fused && film->on_device && opts->bounces == 0 &&
                       P >= (opts->samples == 1 ? size_t(1) << 18 : size_t(1) << 20);
     const bool first_hit = film->velocity_global || film->velocity_camera || film->triangle_size;
-    uint32_t chunk = fused && !lean ? chunk_samples(P, opts->samples) : 0u;
     vgb_status s = VGB_OK;
-    if (!lean || ctx->count_pass) do {
-        const size_t items = (chunk && !ctx->count_pass) ? chunk * P : tile_items(cam->width, cam->height);
-        const size_t sums = chunk == 0 || ctx->count_pass ? B : 0, between = chunk && chunk < opts->samples ? 3 * (size_t)B + 6 : 0;
-        s = ensure_scratch(ctx, std::max<size_t>(chunk, 1) * P, items, P, std::max(sums, between) * P, B, nq,
-                           chunk && first_hit, chunk == 0);
-        if (s != VGB_ERR_OUT_OF_MEMORY || chunk == 0) break;
-        chunk = chunk / 2;   // no memory for that many samples at a time; 0: the wavefront, a sample at a time
-    } while (true);
-    if (s != VGB_OK) return s;
     FrameParams fp;
     std::memset(&fp, 0, sizeof(fp));
     fp.cam = *cam;
@@ -3830,7 +3851,6 @@ VGB_API vgb_status vgb_render(vgb_context* ctx, const vgb_camera* cam, const vgb
     fp.tiles_x = (cam->width + 7) / 8;
     fp.tiles_y = (cam->height + 3) / 4;
     fp.npix = (uint32_t)P;
-    DevState st = ctx->st;
     // film planes: device pointers as given, or staging buffers for host films
     FilmOut f{};
     struct Plane { float** host_f; uint32_t** host_u; size_t n; };
@@ -3901,12 +3921,23 @@ VGB_API vgb_status vgb_render(vgb_context* ctx, const vgb_camera* cam, const vgb
     }
     fp.aux = aux_for(fr) | (opts->adaptive_sampling ? AUX_DEP : 0u);  // the miss test reads the depth sum
     fp.vel_g = fr.vel_g; fp.vel_c = fr.vel_c; fp.tsz = fr.tsz;
+    // Last of all allocations, as it can do with less.
+    uint32_t chunk = fused && !lean ? chunk_samples(P, opts->samples) : 0u;
+    if (!lean || ctx->count_pass) do {
+        size_t want[kScratchPlanes] = {0};
+        if (chunk) want_chunks(want, chunk * P, chunk < opts->samples ? (3 * (size_t)B + 6) * P : 0, B, nlights,
+                               opts->bounces, fp.aux, first_hit);
+        if (!chunk || ctx->count_pass) want_wavefront(want, P, tile_items(cam->width, cam->height), B, nlights);
+        s = ensure_scratch(ctx, want, chunk == 0);
+        if (s != VGB_ERR_OUT_OF_MEMORY || chunk == 0) break;
+        chunk = chunk / 2;   // no memory for that many samples at a time; 0: the wavefront, a sample at a time
+    } while (true);
+    if (s != VGB_OK) return s;
+    DevState st = ctx->st;
     CK(cudaMemsetAsync(ctx->d_stats, 0, sizeof(uint64_t) * 8, ctx->stream));
     uint32_t launches = 0;
     ctx->prof_used = 0;
-    if (cam->distortion && cam->interpolate_directions) {
-        fp.dirs = ensure_directions(ctx, P);
-    }
+    if (cam->distortion && cam->interpolate_directions) fp.dirs = ensure_directions(ctx, P);
     CK(cudaEventRecord(ctx->ev0, ctx->stream));
     if (fp.dirs) {
         k_direction_table<<<grid_for(ctx, P, 16), 256, 0, ctx->stream>>>(fp.cam, ctx->d_dirs);
@@ -4736,7 +4767,7 @@ static vgb_status ensure_frames(vgb_context* ctx, uint32_t n) {
     dfree(ctx->d_frames);
     if (ctx->h_frames) cudaFreeHost(ctx->h_frames);
     ctx->d_frames = nullptr; ctx->h_frames = nullptr; ctx->cap_frames = 0;
-    vgb_status s = dalloc(ctx, &ctx->d_frames, sizeof(DevFrame) * n);
+    vgb_status s = dalloc(ctx, &ctx->d_frames, sizeof(DevFrame) * n, true);   // also within a render
     if (s != VGB_OK) return s;
     CK(cudaMallocHost(&ctx->h_frames, sizeof(DevFrame) * n));
     ctx->cap_frames = n;
