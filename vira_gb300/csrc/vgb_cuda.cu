@@ -2718,24 +2718,33 @@ VGB_API vgb_status vgb_scene_upload(vgb_context* ctx, const float* pos, uint32_t
     return vgb::status_of_exception(ctx ? &ctx->err : nullptr);
 }
 
-// The wide nodes of the context's binary BVH.  too_deep: the tree has more levels than the traversal's
-// stack holds (a binary tree of more than 63 levels, and skewed so that folding does not shorten it).
+// The wide nodes of the context's binary BVH.  Folded by surface a chain of nodes keeps its length where
+// every sibling is larger than the rest of the chain and has nodes of its own; a tree that is then deeper
+// than the traversal's stack is folded by height, to at most half its levels.  too_deep: that was not enough
+// either (a binary tree of more than 126 levels).
 static vgb_status build_wide(vgb_context* ctx, bool& too_deep) {
-    uint32_t* work = nullptr;
+    uint32_t *work = nullptr, *heights = nullptr;
     uint32_t levels = 0;
     vgb_status s = dalloc(ctx, &work, vgb::wide_work_words(ctx->nnodes) * sizeof(uint32_t));
     if (s != VGB_OK) return s;
     const uint32_t* nodes = reinterpret_cast<const uint32_t*>(ctx->d_nodes);
-    cudaError_t e = (cudaError_t)vgb::launch_wide_fold(ctx->stream, ctx->num_sms, nodes, ctx->nnodes, work, &ctx->nwide, &levels);
-    if (e == cudaSuccess) s = dalloc(ctx, &ctx->d_wide, (size_t)ctx->nwide * 128);
-    if (e == cudaSuccess && s == VGB_OK)
+    cudaError_t e = (cudaError_t)vgb::launch_wide_fold(ctx->stream, ctx->num_sms, nodes, ctx->nnodes, work, nullptr, &ctx->nwide, &levels);
+    if (e == cudaSuccess && levels > vgb::kWideLevels) {
+        s = dalloc(ctx, &heights, (size_t)ctx->nnodes * sizeof(uint32_t));
+        if (s == VGB_OK) e = (cudaError_t)vgb::launch_node_heights(ctx->stream, ctx->num_sms, nodes, ctx->nnodes, ctx->d_parent, ctx->d_refit, heights);
+        if (s == VGB_OK && e == cudaSuccess)
+            e = (cudaError_t)vgb::launch_wide_fold(ctx->stream, ctx->num_sms, nodes, ctx->nnodes, work, heights, &ctx->nwide, &levels);
+    }
+    too_deep = levels > vgb::kWideLevels;
+    if (e == cudaSuccess && s == VGB_OK && !too_deep) s = dalloc(ctx, &ctx->d_wide, (size_t)ctx->nwide * 128);
+    if (e == cudaSuccess && s == VGB_OK && !too_deep)
         e = (cudaError_t)vgb::launch_wide_emit(ctx->stream, ctx->num_sms, nodes, ctx->nnodes, work, ctx->nwide, ctx->d_wide);
     const cudaError_t e2 = cudaStreamSynchronize(ctx->stream);
     dfree(work);
+    dfree(heights);
     if (s != VGB_OK) return s;
     CK(e);
     CK(e2);
-    too_deep = levels > (uint32_t)vgb::kWideLevels;
     ctx->stats.bvh_nodes = ctx->nwide;
     ctx->stats.bvh_node_bytes = 128;
     return VGB_OK;
@@ -2782,7 +2791,8 @@ VGB_API vgb_status vgb_bvh_build(vgb_context* ctx, const vgb_bvh_options* opts) 
         ctx->bvh_leaf = leaf; ctx->bvh_threads = 0;
         bool deep = false;
         if ((s = build_wide(ctx, deep)) != VGB_OK) return s;
-        if (deep) return fail(ctx, VGB_ERR_INVALID_ARGUMENT, "bvh_build: the tree is too deep to traverse");
+        // cannot be: 63 key bits and 32 of the position split at most 95 times
+        if (deep) return fail(ctx, VGB_ERR_INTERNAL, "bvh_build: the tree is too deep to traverse");
         ctx->bvh_ready = true;
         ctx->stats.tri_record_bytes = 48;
         return VGB_OK;
@@ -2824,7 +2834,7 @@ VGB_API vgb_status vgb_bvh_build(vgb_context* ctx, const vgb_bvh_options* opts) 
     if (layout == 2) {
         bool deep = false;
         if ((s = build_wide(ctx, deep)) != VGB_OK) return s;
-        if (deep) {   // Morton order splits at most 63 + 32 times, whatever the triangles
+        if (deep) {   // Morton order splits at most 95 times, whatever the triangles
             const vgb_bvh_options o{leaf, 1u, threads, 2u};
             return vgb_bvh_build(ctx, &o);
         }

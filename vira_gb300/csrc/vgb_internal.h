@@ -202,10 +202,14 @@ int launch_refit(void* stream, int sms, const void* vpos /* float4 */, const uin
 // (wide_work_words) and returns the number of wide nodes; emit writes them (128 bytes each);
 // refit rewrites the boxes of emitted nodes from the binary ones.  Return a CUDA error or 0.
 size_t wide_work_words(uint32_t nnodes);
-// levels_out: the wide tree's depth, which the traversal's stack limits to kWideLevels.
-constexpr int kWideLevels = 63, kStackWide = 3 * kWideLevels + 3;
-int launch_wide_fold(void* stream, int sms, const uint32_t* nodes, uint32_t nnodes, uint32_t* work, uint32_t* nwide_out,
-                     uint32_t* levels_out);
+// levels_out: the wide tree's depth, which the traversal's stack limits to kWideLevels (the fold stops
+// beyond).  heights (or null): fold by the binary nodes' heights, for trees that are too deep folded by
+// surface.  counts: nnodes words of scratch.
+constexpr uint32_t kWideLevels = 63, kStackWide = 3 * kWideLevels + 3;
+int launch_node_heights(void* stream, int sms, const uint32_t* nodes, uint32_t nnodes, const uint32_t* parent,
+                        uint32_t* counts, uint32_t* heights);
+int launch_wide_fold(void* stream, int sms, const uint32_t* nodes, uint32_t nnodes, uint32_t* work, const uint32_t* heights,
+                     uint32_t* nwide_out, uint32_t* levels_out);
 int launch_wide_emit(void* stream, int sms, const uint32_t* nodes, uint32_t nnodes, const uint32_t* work,
                      uint32_t nwide, void* wide);
 int launch_wide_refit(void* stream, int sms, const uint32_t* nodes, uint32_t nwide, void* wide);

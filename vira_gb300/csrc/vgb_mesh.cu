@@ -506,10 +506,33 @@ __device__ __forceinline__ void put_wide_child(float* w, int k, const RBox& b) {
     w[20 + k] = ok ? wide_half_extent(b.lz, b.hz, cz, slack) : 3e38f;
 }
 
+// Levels of inner nodes from each binary node down: one thread per (node, side) whose child is a leaf
+// walks up, and the second of a node's two sides to finish goes on (as in k_refit_nodes).
+__global__ void k_node_heights(const uint32_t* __restrict__ nodes, uint32_t nnodes, const uint32_t* __restrict__ parent,
+                               uint32_t* counts, uint32_t* heights) {
+    for (size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x; q < 2 * (size_t)nnodes;
+         q += (size_t)gridDim.x * blockDim.x) {
+        uint32_t node = (uint32_t)(q >> 1);
+        if ((int32_t)nodes[16 * (size_t)node + 12 + (q & 1)] >= 0) continue;
+        uint32_t h = 1;
+        for (uint32_t step = 0; step < nnodes; ++step) {
+            atomicMax(&heights[node], h);
+            if (atomic_add_acq_rel(&counts[node], 1u) == 0u) break;   // the other side is not done yet
+            h = __ldcg(&heights[node]) + 1u;
+            const uint32_t pr = parent[node];
+            if (pr == vgb::kNoParent) break;
+            node = pr >> 1;
+        }
+    }
+}
+
 // One level of the fold: the roots queue[begin, end) each open the inner child of the largest
-// surface until they have four children or only leaves, and queue the inner children as roots.
+// surface (with `heights`, the tallest) until they have four children or only leaves, and queue the
+// inner children as roots.  Opening the tallest leaves no inner child above the root's height less 2,
+// so that fold has at most half the binary tree's levels.
 __global__ void k_wide_fold(const uint32_t* __restrict__ nodes, uint32_t* queue, uint32_t begin, uint32_t end,
-                            uint4* __restrict__ src, uint32_t* __restrict__ is_root, uint32_t* tail) {
+                            uint4* __restrict__ src, uint32_t* __restrict__ is_root, uint32_t* tail,
+                            const uint32_t* __restrict__ heights) {
     for (uint32_t i = begin + blockIdx.x * blockDim.x + threadIdx.x; i < end; i += gridDim.x * blockDim.x) {
         const uint32_t root = queue[i];
         is_root[root] = 1u;
@@ -519,10 +542,11 @@ __global__ void k_wide_fold(const uint32_t* __restrict__ nodes, uint32_t* queue,
             int best = -1;
             float area = -1.f;
             for (int k = 0; k < n; ++k) {
-                if ((int32_t)nodes[16 * (size_t)(e[k] >> 1) + 12 + (e[k] & 1u)] < 0) continue;
+                const int32_t link = (int32_t)nodes[16 * (size_t)(e[k] >> 1) + 12 + (e[k] & 1u)];
+                if (link < 0) continue;
                 const RBox b = get_box(nodes, e[k] >> 1, (int)(e[k] & 1u));
                 const float x = b.hx - b.lx, y = b.hy - b.ly, z = b.hz - b.lz;
-                const float a = x * y + y * z + z * x;
+                const float a = heights ? (float)heights[link] : x * y + y * z + z * x;
                 if (best < 0 || a > area) { area = a; best = k; }
             }
             if (best < 0) break;
@@ -606,8 +630,17 @@ WideWork wide_work(uint32_t* work, uint32_t nnodes) {
 }
 }  // namespace
 
-int launch_wide_fold(void* stream, int sms, const uint32_t* nodes, uint32_t nnodes, uint32_t* work, uint32_t* nwide_out,
-                     uint32_t* levels_out) {
+int launch_node_heights(void* stream, int sms, const uint32_t* nodes, uint32_t nnodes, const uint32_t* parent,
+                        uint32_t* counts, uint32_t* heights) {
+    cudaStream_t s = (cudaStream_t)stream;
+    cudaMemsetAsync(counts, 0, (size_t)nnodes * sizeof(uint32_t), s);
+    cudaMemsetAsync(heights, 0, (size_t)nnodes * sizeof(uint32_t), s);
+    k_node_heights<<<grid(2 * (size_t)nnodes, sms), 256, 0, s>>>(nodes, nnodes, parent, counts, heights);
+    return (int)cudaGetLastError();
+}
+
+int launch_wide_fold(void* stream, int sms, const uint32_t* nodes, uint32_t nnodes, uint32_t* work, const uint32_t* heights,
+                     uint32_t* nwide_out, uint32_t* levels_out) {
     cudaStream_t s = (cudaStream_t)stream;
     const WideWork w = wide_work(work, nnodes);
     const uint32_t one = 1;
@@ -616,8 +649,8 @@ int launch_wide_fold(void* stream, int sms, const uint32_t* nodes, uint32_t nnod
     cudaMemcpyAsync(w.tail, &one, sizeof(uint32_t), cudaMemcpyHostToDevice, s);
     uint32_t begin = 0, end = 1;
     *levels_out = 0;
-    while (begin < end) {   // one level of wide nodes per pass; every binary node is a root at most once
-        k_wide_fold<<<grid(end - begin, sms), 256, 0, s>>>(nodes, w.queue, begin, end, w.src, w.flag, w.tail);
+    while (begin < end && *levels_out <= kWideLevels) {   // one level of wide nodes per pass; every binary node is a root at most once
+        k_wide_fold<<<grid(end - begin, sms), 256, 0, s>>>(nodes, w.queue, begin, end, w.src, w.flag, w.tail, heights);
         uint32_t tail = 0;
         cudaMemcpyAsync(&tail, w.tail, sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
         const cudaError_t e = cudaStreamSynchronize(s);
