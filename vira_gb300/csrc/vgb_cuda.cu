@@ -1802,6 +1802,7 @@ struct vgb_context {
     bool bvh_ready = false;
     uint32_t* d_parent = nullptr;   // binary layout: (parent << 1 | side) per node, for refits
     uint32_t* d_refit = nullptr;    // nnodes + 1 words: arrival counters and the walk-bound flag
+    size_t cap_nodes = 0, cap_wide = 0, cap_tris = 0, cap_parent = 0, cap_refit = 0;   // bytes of these, kept over rebuilds
     uint32_t bvh_leaf = 0, bvh_threads = 0;
     bool h_pos_stale = false;       // device positions moved by a device-side update
     uint32_t* d_vnl = nullptr;      // per-vertex corner lists of the uploaded mesh (vertex-normal updates)
@@ -1914,11 +1915,18 @@ void free_scene(vgb_context* ctx) {
     ctx->d_motion = nullptr;
     ctx->nmotion = 0;
 }
+// The tree is gone, its buffers stay for the next one of the scene: freeing and allocating five of them was
+// a third of a GPU build's time (0.5M triangles 960 -> 614 us).
+void retire_bvh(vgb_context* ctx) {
+    ctx->bvh_ready = false;
+    ctx->nnodes = ctx->nwide = 0;
+    ctx->bvh_serial++;
+}
 void free_bvh(vgb_context* ctx) {
     dfree(ctx->d_nodes); dfree(ctx->d_wide); dfree(ctx->d_tris); dfree(ctx->d_parent); dfree(ctx->d_refit);
-    ctx->d_nodes = ctx->d_wide = nullptr; ctx->nwide = 0; ctx->d_tris = nullptr; ctx->d_parent = nullptr; ctx->d_refit = nullptr;
-    ctx->bvh_ready = false; ctx->nnodes = 0;
-    ctx->bvh_serial++;
+    ctx->d_nodes = ctx->d_wide = nullptr; ctx->d_tris = nullptr; ctx->d_parent = nullptr; ctx->d_refit = nullptr;
+    ctx->cap_nodes = ctx->cap_wide = ctx->cap_tris = ctx->cap_parent = ctx->cap_refit = 0;
+    retire_bvh(ctx);
 }
 void free_scratch(vgb_context* ctx) {
     for (vgb_context::Plane& q : ctx->scratch) {
@@ -1945,6 +1953,17 @@ void* mapped_host(const void* p) {
         return nullptr;
     }
     return (a.type == cudaMemoryTypeHost && a.devicePointer) ? a.devicePointer : nullptr;
+}
+
+template <typename T>
+vgb_status grow_buffer(vgb_context* ctx, T** p, size_t& cap, size_t bytes) {
+    if (*p && bytes <= cap) return VGB_OK;
+    dfree(*p);
+    *p = nullptr;
+    cap = 0;
+    const vgb_status s = dalloc(ctx, p, bytes);
+    if (s == VGB_OK) cap = bytes;
+    return s;
 }
 
 vgb_status ensure_staging(vgb_context* ctx, size_t bytes) {
@@ -2723,10 +2742,13 @@ VGB_API vgb_status vgb_scene_upload(vgb_context* ctx, const float* pos, uint32_t
 // than the traversal's stack is folded by height, to at most half its levels.  too_deep: that was not enough
 // either (a binary tree of more than 126 levels).
 static vgb_status build_wide(vgb_context* ctx, bool& too_deep) {
-    uint32_t *work = nullptr, *heights = nullptr;
+    uint32_t *own = nullptr, *heights = nullptr;
     uint32_t levels = 0;
-    vgb_status s = dalloc(ctx, &work, vgb::wide_work_words(ctx->nnodes) * sizeof(uint32_t));
-    if (s != VGB_OK) return s;
+    vgb_status s = VGB_OK;
+    // the GPU builder leaves its larger work area, which is free by now
+    const size_t need = vgb::wide_work_words(ctx->nnodes) * sizeof(uint32_t);
+    if (need > ctx->cap_dn && (s = dalloc(ctx, &own, need)) != VGB_OK) return s;
+    uint32_t* work = own ? own : reinterpret_cast<uint32_t*>(ctx->d_dn);
     const uint32_t* nodes = reinterpret_cast<const uint32_t*>(ctx->d_nodes);
     cudaError_t e = (cudaError_t)vgb::launch_wide_fold(ctx->stream, ctx->num_sms, nodes, ctx->nnodes, work, nullptr, &ctx->nwide, &levels);
     if (e == cudaSuccess && levels > vgb::kWideLevels) {
@@ -2736,11 +2758,11 @@ static vgb_status build_wide(vgb_context* ctx, bool& too_deep) {
             e = (cudaError_t)vgb::launch_wide_fold(ctx->stream, ctx->num_sms, nodes, ctx->nnodes, work, heights, &ctx->nwide, &levels);
     }
     too_deep = levels > vgb::kWideLevels;
-    if (e == cudaSuccess && s == VGB_OK && !too_deep) s = dalloc(ctx, &ctx->d_wide, (size_t)ctx->nwide * 128);
+    if (e == cudaSuccess && s == VGB_OK && !too_deep) s = grow_buffer(ctx, &ctx->d_wide, ctx->cap_wide, (size_t)ctx->nwide * 128);
     if (e == cudaSuccess && s == VGB_OK && !too_deep)
         e = (cudaError_t)vgb::launch_wide_emit(ctx->stream, ctx->num_sms, nodes, ctx->nnodes, work, ctx->nwide, ctx->d_wide);
     const cudaError_t e2 = cudaStreamSynchronize(ctx->stream);
-    dfree(work);
+    dfree(own);
     dfree(heights);
     if (s != VGB_OK) return s;
     CK(e);
@@ -2770,16 +2792,16 @@ VGB_API vgb_status vgb_bvh_build(vgb_context* ctx, const vgb_bvh_options* opts) 
             return fail(ctx, VGB_ERR_INVALID_ARGUMENT, "bvh_build: too many triangles for the leaf encoding");
         cudaSetDevice(ctx->device);
         CK(cudaStreamSynchronize(ctx->stream));
-        free_bvh(ctx);
+        retire_bvh(ctx);
         vgb_status s;
         uint32_t nn = 0;
         if ((s = ensure_dn_scratch(ctx, vgb::lbvh_work_words(n))) != VGB_OK) return s;
         CK((cudaError_t)vgb::launch_lbvh_sort_and_link(ctx->stream, ctx->num_sms, ctx->d_vpos, ctx->d_idx, n, leaf,
                                                        reinterpret_cast<uint32_t*>(ctx->d_dn), &nn));
-        if ((s = dalloc(ctx, &ctx->d_nodes, (size_t)nn * 64)) != VGB_OK) return s;
-        if ((s = dalloc(ctx, &ctx->d_tris, (size_t)n * 48)) != VGB_OK) return s;
-        if ((s = dalloc(ctx, &ctx->d_parent, (size_t)nn * 4)) != VGB_OK) return s;
-        if ((s = dalloc(ctx, &ctx->d_refit, ((size_t)nn + 1) * 4)) != VGB_OK) return s;
+        if ((s = grow_buffer(ctx, &ctx->d_nodes, ctx->cap_nodes, (size_t)nn * 64)) != VGB_OK) return s;
+        if ((s = grow_buffer(ctx, &ctx->d_tris, ctx->cap_tris, (size_t)n * 48)) != VGB_OK) return s;
+        if ((s = grow_buffer(ctx, &ctx->d_parent, ctx->cap_parent, (size_t)nn * 4)) != VGB_OK) return s;
+        if ((s = grow_buffer(ctx, &ctx->d_refit, ctx->cap_refit, ((size_t)nn + 1) * 4)) != VGB_OK) return s;
         const int rc = vgb::launch_lbvh_emit(ctx->stream, ctx->num_sms, ctx->d_vpos, ctx->d_idx, n, leaf,
                                              reinterpret_cast<const uint32_t*>(ctx->d_dn),
                                              reinterpret_cast<uint32_t*>(ctx->d_nodes), nn, ctx->d_tris, ctx->d_parent,
@@ -2815,15 +2837,16 @@ VGB_API vgb_status vgb_bvh_build(vgb_context* ctx, const vgb_bvh_options* opts) 
     if (!vgb::build_bvh(ctx->h_pos.data(), ctx->nverts, ctx->h_idx.data(), ctx->ntris, leaf, threads, layout, bvh, &why))
         return fail(ctx, VGB_ERR_INVALID_ARGUMENT, std::string("bvh_build: ") + why);
     CK(cudaStreamSynchronize(ctx->stream));
-    free_bvh(ctx);
+    if (layout == 8) free_bvh(ctx);   // which has no wide nodes, parents and counters
+    else retire_bvh(ctx);
     vgb_status s;
-    if ((s = dalloc(ctx, &ctx->d_nodes, bvh.nodes.size() * sizeof(uint32_t))) != VGB_OK) return s;
-    if ((s = dalloc(ctx, &ctx->d_tris, bvh.tris.size() * sizeof(float))) != VGB_OK) return s;
+    if ((s = grow_buffer(ctx, &ctx->d_nodes, ctx->cap_nodes, bvh.nodes.size() * sizeof(uint32_t))) != VGB_OK) return s;
+    if ((s = grow_buffer(ctx, &ctx->d_tris, ctx->cap_tris, bvh.tris.size() * sizeof(float))) != VGB_OK) return s;
     CK(cudaMemcpy(ctx->d_nodes, bvh.nodes.data(), bvh.nodes.size() * sizeof(uint32_t), cudaMemcpyHostToDevice));
     CK(cudaMemcpy(ctx->d_tris, bvh.tris.data(), bvh.tris.size() * sizeof(float), cudaMemcpyHostToDevice));
     if (layout == 2) {
-        if ((s = dalloc(ctx, &ctx->d_parent, bvh.parent.size() * sizeof(uint32_t))) != VGB_OK) return s;
-        if ((s = dalloc(ctx, &ctx->d_refit, (bvh.parent.size() + 1) * sizeof(uint32_t))) != VGB_OK) return s;
+        if ((s = grow_buffer(ctx, &ctx->d_parent, ctx->cap_parent, bvh.parent.size() * sizeof(uint32_t))) != VGB_OK) return s;
+        if ((s = grow_buffer(ctx, &ctx->d_refit, ctx->cap_refit, (bvh.parent.size() + 1) * sizeof(uint32_t))) != VGB_OK) return s;
         CK(cudaMemcpy(ctx->d_parent, bvh.parent.data(), bvh.parent.size() * sizeof(uint32_t), cudaMemcpyHostToDevice));
     }
     ctx->nnodes = bvh.num_nodes;
@@ -3073,11 +3096,9 @@ VGB_API vgb_status vgb_scene_update_positions(vgb_context* ctx, const float* pos
         if (ctx->bvh_layout == 2) {
             const int rc = vgb::launch_refit(ctx->stream, ctx->num_sms, ctx->d_vpos, ctx->d_idx, (uint32_t)nt, ctx->d_tris,
                                              reinterpret_cast<uint32_t*>(ctx->d_nodes), ctx->nnodes, ctx->d_parent,
-                                             ctx->d_refit);
+                                             ctx->d_refit, ctx->nwide, ctx->d_wide);
             if (rc == -2) return fail(ctx, VGB_ERR_CUDA, "scene_update_positions: refit walk exceeded the tree depth");
             CK((cudaError_t)rc);
-            CK((cudaError_t)vgb::launch_wide_refit(ctx->stream, ctx->num_sms, reinterpret_cast<const uint32_t*>(ctx->d_nodes),
-                                                   ctx->nwide, ctx->d_wide));
         } else {
             vgb_bvh_options o{};
             o.max_leaf_size = ctx->bvh_leaf; o.threads = ctx->bvh_threads; o.layout = ctx->bvh_layout;

@@ -197,10 +197,11 @@ int launch_lbvh_emit(void* stream, int sms, const void* vpos, const uint32_t* id
 // from vpos, then every child box recomputed bottom up.  counts: nnodes words of scratch.
 // Returns nonzero on a CUDA error, -2 when an upward walk exceeded its bound.
 int launch_refit(void* stream, int sms, const void* vpos /* float4 */, const uint32_t* idx, uint32_t ntris,
-                 void* tris /* float4 */, uint32_t* nodes, uint32_t nnodes, const uint32_t* parent, uint32_t* counts);
+                 void* tris /* float4 */, uint32_t* nodes, uint32_t nnodes, const uint32_t* parent, uint32_t* counts,
+                 uint32_t nwide, void* wide /* the wide nodes, whose boxes follow */);
 // The wide nodes of a binary BVH: fold writes the node roots and their children into `work`
-// (wide_work_words) and returns the number of wide nodes; emit writes them (128 bytes each);
-// refit rewrites the boxes of emitted nodes from the binary ones.  Return a CUDA error or 0.
+// (wide_work_words) and returns the number of wide nodes; emit writes them (128 bytes each).
+// Return a CUDA error or 0.
 size_t wide_work_words(uint32_t nnodes);
 // levels_out: the wide tree's depth, which the traversal's stack limits to kWideLevels (the fold stops
 // beyond).  heights (or null): fold by the binary nodes' heights, for trees that are too deep folded by
@@ -212,7 +213,6 @@ int launch_wide_fold(void* stream, int sms, const uint32_t* nodes, uint32_t nnod
                      uint32_t* nwide_out, uint32_t* levels_out);
 int launch_wide_emit(void* stream, int sms, const uint32_t* nodes, uint32_t nnodes, const uint32_t* work,
                      uint32_t nwide, void* wide);
-int launch_wide_refit(void* stream, int sms, const uint32_t* nodes, uint32_t nwide, void* wide);
 
 
 // ---- DEM Quipu (vgb_quipu.cpp host side, vgb_mesh.cu device decode)

@@ -526,13 +526,15 @@ __global__ void k_node_heights(const uint32_t* __restrict__ nodes, uint32_t nnod
     }
 }
 
-// One level of the fold: the roots queue[begin, end) each open the inner child of the largest
-// surface (with `heights`, the tallest) until they have four children or only leaves, and queue the
+// One level of the fold: the level's roots (counts[level] of them in the queue, after those of the levels
+// above) each open the inner child of the largest surface (with `heights`, the tallest) until they have four children or only leaves, and queue the
 // inner children as roots.  Opening the tallest leaves no inner child above the root's height less 2,
 // so that fold has at most half the binary tree's levels.
-__global__ void k_wide_fold(const uint32_t* __restrict__ nodes, uint32_t* queue, uint32_t begin, uint32_t end,
-                            uint4* __restrict__ src, uint32_t* __restrict__ is_root, uint32_t* tail,
+__global__ void k_wide_fold(const uint32_t* __restrict__ nodes, uint32_t* queue, uint32_t level, uint32_t* counts,
+                            uint4* __restrict__ src, uint32_t* __restrict__ is_root,
                             const uint32_t* __restrict__ heights) {
+    uint32_t begin = 0, end = 1;   // level 0: the binary root
+    for (uint32_t l = 1; l <= level; ++l) { begin = end; end += counts[l]; }
     for (uint32_t i = begin + blockIdx.x * blockDim.x + threadIdx.x; i < end; i += gridDim.x * blockDim.x) {
         const uint32_t root = queue[i];
         is_root[root] = 1u;
@@ -564,7 +566,7 @@ __global__ void k_wide_fold(const uint32_t* __restrict__ nodes, uint32_t* queue,
             if (link >= 0) inner[c++] = (uint32_t)link;
         }
         if (c) {
-            const uint32_t at = atomicAdd(tail, (uint32_t)c);
+            const uint32_t at = end + atomicAdd(&counts[level + 1], (uint32_t)c);
             for (int k = 0; k < c; ++k) queue[at + k] = inner[k];
         }
     }
@@ -609,23 +611,24 @@ __global__ void k_wide_refit(const uint32_t* __restrict__ nodes, uint32_t nwide,
 
 namespace vgb {
 
-// work: queue of roots [nnodes], sources [4 nnodes], root flags and their scan [nnodes + 1 each],
-// the queue's tail, scan scratch
+// work: sources [4 nnodes], queue of roots [nnodes], root flags [nnodes + 1], the roots of each level, the
+// flags' scan [nnodes + 1], scan scratch
+constexpr uint32_t kFoldCounts = kWideLevels + 2;
 size_t wide_work_words(uint32_t nnodes) {
-    return 7 * (size_t)nnodes + 8 + scan_temp_words((size_t)nnodes + 1);
+    return 7 * (size_t)nnodes + 2 + kFoldCounts + scan_temp_words((size_t)nnodes + 1);
 }
 
 namespace {
-struct WideWork { uint4* src; uint32_t *queue, *flag, *rank, *tail, *tmp; };
+struct WideWork { uint4* src; uint32_t *queue, *flag, *rank, *counts, *tmp; };
 WideWork wide_work(uint32_t* work, uint32_t nnodes) {
     WideWork w;
     const size_t n = nnodes;
     w.src = reinterpret_cast<uint4*>(work);
     w.queue = work + 4 * n;
     w.flag = w.queue + n;
-    w.rank = w.flag + n + 1;
-    w.tail = w.rank + n + 1;
-    w.tmp = w.tail + 1;
+    w.counts = w.flag + n + 1;
+    w.rank = w.counts + kFoldCounts;
+    w.tmp = w.rank + n + 1;
     return w;
 }
 }  // namespace
@@ -643,24 +646,30 @@ int launch_wide_fold(void* stream, int sms, const uint32_t* nodes, uint32_t nnod
                      uint32_t* nwide_out, uint32_t* levels_out) {
     cudaStream_t s = (cudaStream_t)stream;
     const WideWork w = wide_work(work, nnodes);
-    const uint32_t one = 1;
-    cudaMemsetAsync(w.queue, 0, sizeof(uint32_t), s);   // the binary root
-    cudaMemsetAsync(w.flag, 0, ((size_t)nnodes + 1) * sizeof(uint32_t), s);
-    cudaMemcpyAsync(w.tail, &one, sizeof(uint32_t), cudaMemcpyHostToDevice, s);
-    uint32_t begin = 0, end = 1;
-    *levels_out = 0;
-    while (begin < end && *levels_out <= kWideLevels) {   // one level of wide nodes per pass; every binary node is a root at most once
-        k_wide_fold<<<grid(end - begin, sms), 256, 0, s>>>(nodes, w.queue, begin, end, w.src, w.flag, w.tail, heights);
-        uint32_t tail = 0;
-        cudaMemcpyAsync(&tail, w.tail, sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
+    // queue (its first entry is the binary root), flags and counts
+    cudaMemsetAsync(w.queue, 0, (size_t)(w.rank - w.queue) * sizeof(uint32_t), s);
+    // Every binary node is a root at most once.  The levels are queued without a wait between them (level l
+    // has at most 4^l roots): three more than a full tree has, then eight at a time.
+    uint32_t counts[kFoldCounts], level = 0, batch = 3;
+    while (((size_t)1 << 2 * (batch - 3)) < nnodes) ++batch;
+    do {
+        const uint32_t stop = std::min(level + batch, kWideLevels + 1);
+        batch = 8;
+        for (; level < stop; ++level) {
+            const size_t most = level < 16 ? std::min<size_t>(nnodes, (size_t)1 << 2 * level) : nnodes;
+            k_wide_fold<<<grid(most, sms), 256, 0, s>>>(nodes, w.queue, level, w.counts, w.src, w.flag, heights);
+        }
+        scan(s, w.flag, w.rank, (size_t)nnodes + 1, w.tmp);
+        cudaMemcpyAsync(counts, w.counts, sizeof(counts), cudaMemcpyDeviceToHost, s);
         const cudaError_t e = cudaStreamSynchronize(s);
         if (e != cudaSuccess) return (int)e;
-        begin = end;
-        end = tail;
+    } while (counts[level] && level <= kWideLevels);
+    counts[0] = 1;
+    *levels_out = *nwide_out = 0;
+    for (uint32_t l = 0; l <= kWideLevels && counts[l]; ++l) {
         ++*levels_out;
+        *nwide_out += counts[l];
     }
-    scan(s, w.flag, w.rank, (size_t)nnodes + 1, w.tmp);
-    *nwide_out = end;
     return (int)cudaGetLastError();
 }
 
@@ -671,19 +680,15 @@ int launch_wide_emit(void* stream, int sms, const uint32_t* nodes, uint32_t nnod
     return (int)cudaGetLastError();
 }
 
-int launch_wide_refit(void* stream, int sms, const uint32_t* nodes, uint32_t nwide, void* wide) {
-    k_wide_refit<<<grid(4 * (size_t)nwide, sms), 256, 0, (cudaStream_t)stream>>>(nodes, nwide, (float*)wide);
-    return (int)cudaGetLastError();
-}
-
 int launch_refit(void* stream, int sms, const void* vpos, const uint32_t* idx, uint32_t ntris, void* tris,
-                 uint32_t* nodes, uint32_t nnodes, const uint32_t* parent, uint32_t* counts) {
+                 uint32_t* nodes, uint32_t nnodes, const uint32_t* parent, uint32_t* counts, uint32_t nwide, void* wide) {
     cudaStream_t s = (cudaStream_t)stream;
     uint32_t* flag = counts + nnodes;
     cudaMemsetAsync(counts, 0, ((size_t)nnodes + 1) * sizeof(uint32_t), s);
     k_refit_tris<<<grid(ntris, sms), 256, 0, s>>>((const float4*)vpos, idx, ntris, (float4*)tris);
     k_refit_nodes<<<grid(2 * (size_t)nnodes, sms), 256, 0, s>>>((const float4*)tris, nodes, nnodes, parent, counts,
                                                                  4096u, flag);
+    k_wide_refit<<<grid(4 * (size_t)nwide, sms), 256, 0, s>>>(nodes, nwide, (float*)wide);
     uint32_t bad = 0;
     cudaMemcpyAsync(&bad, flag, sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
     cudaError_t e = cudaStreamSynchronize(s);
