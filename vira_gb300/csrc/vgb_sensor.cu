@@ -208,7 +208,10 @@ __host__ __device__ constexpr int round4(int v) { return (v + 3) & ~3; }
 // summed over ky outer, kx inner, as the reference's loop.  Bound by the FP32 pipes, as a product and a sum
 // are separate operations (reference rounding): 81^2 taps on 1024^2 x 4 bands 2.7 -> 1.8 ms, 76 % of
 // their rate, with the test for the row's padded taps out of the inner loop.  Packed f32x2 operations on
-// pairs of bands took the same time.
+// pairs of bands took the same time.  REST: kw % 4.  FULL: kw / 4 up to 1, else -1.  Both known to the
+// compiler, as the tests of a row's end and the set-up of its unrolled loop cost small kernels more than
+// the loop gains (512^2 x 4 bands, 5^2 / 6^2 taps 29.5 / 30.8 -> 31.0 / 31.9 us).
+template <int REST, int FULL>
 __global__ void __launch_bounds__(256) k_psf(const float* __restrict__ in, float* __restrict__ out, uint32_t W,
                                              uint32_t H, const float* __restrict__ kernel, int kw, int kh) {
     extern __shared__ float4 sm4[];
@@ -241,7 +244,7 @@ __global__ void __launch_bounds__(256) k_psf(const float* __restrict__ in, float
         const float4* krow = reinterpret_cast<const float4*>(ks + ky * kwp);
         float4 a = row[0];
 #pragma unroll 4
-        for (int c = 0; c < kw / 4; ++c) {
+        for (int c = 0; c < (FULL < 0 ? kw / 4 : FULL); ++c) {
             const float4 b = row[c + 1];
             const float4 k = krow[c];
             const float in[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
@@ -255,14 +258,14 @@ __global__ void __launch_bounds__(256) k_psf(const float* __restrict__ in, float
             }
             a = b;
         }
-        if (kw & 3) {   // the last 1..3 taps of the row; its padded taps are not summed
-            const float4 b = row[kw / 4 + 1];
-            const float4 k = krow[kw / 4];
+        if (REST != 0) {   // the last 1..3 taps of the row; its padded taps are not summed
+            const int c = FULL < 0 ? kw / 4 : FULL;
+            const float4 b = row[c + 1];
+            const float4 k = krow[c];
             const float in[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
             const float kk[4] = {k.x, k.y, k.z, k.w};
 #pragma unroll
-            for (int t = 0; t < 3; ++t) {
-                if (t >= (kw & 3)) break;
+            for (int t = 0; t < REST; ++t) {
                 s0 += in[t] * kk[t];
                 s1 += in[t + 1] * kk[t];
                 s2 += in[t + 2] * kk[t];
@@ -305,14 +308,19 @@ int launch_sensor_rgb(void* stream, const float* power, uint32_t width, uint32_t
 
 int launch_psf(void* stream, const float* in, float* out, uint32_t width, uint32_t height, uint32_t nbands,
                const float* kernel, uint32_t kw, uint32_t kh) {
-    if (kw > (uint32_t)kMaxKernel || kh > (uint32_t)kMaxKernel) return (int)cudaErrorInvalidValue;
+    if (kw == 0 || kw > (uint32_t)kMaxKernel || kh > (uint32_t)kMaxKernel) return (int)cudaErrorInvalidValue;
     const int kwp = round4((int)kw);
     const size_t tw = round4(kTileW + kwp + 3), th = kTileH + kh - 1;
     const size_t smem = (tw * th + (size_t)kwp * kh) * sizeof(float);
-    cudaError_t e = cudaFuncSetAttribute(k_psf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    using Kernel = void (*)(const float*, float*, uint32_t, uint32_t, const float*, int, int);
+    static constexpr Kernel kSmall[8] = {nullptr,     k_psf<1, 0>, k_psf<2, 0>, k_psf<3, 0>,
+                                         k_psf<0, 1>, k_psf<1, 1>, k_psf<2, 1>, k_psf<3, 1>};
+    static constexpr Kernel kLarge[4] = {k_psf<0, -1>, k_psf<1, -1>, k_psf<2, -1>, k_psf<3, -1>};
+    const Kernel k = kw < 8 ? kSmall[kw] : kLarge[kw & 3];
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
     const dim3 grid((width + kTileW - 1) / kTileW, (height + kTileH - 1) / kTileH, nbands);
-    k_psf<<<grid, dim3(32, kTileH), smem, (cudaStream_t)stream>>>(in, out, width, height, kernel, (int)kw, (int)kh);
+    k<<<grid, dim3(32, kTileH), smem, (cudaStream_t)stream>>>(in, out, width, height, kernel, (int)kw, (int)kh);
     return (int)cudaGetLastError();
 }
 
