@@ -346,7 +346,10 @@ typedef struct vgb_frame {
 } vgb_frame;
 
 typedef struct vgb_batch_options {
-    uint32_t autotune;         /* 1: time launch shapes on a 1/16 sample of the tiles, keep the best */
+    uint32_t autotune;         /* 1: time launch shapes on a 1/16 sample of the tiles and keep the best, which
+                                  later calls use as long as the kernel variant (bands, planes, bounces,
+                                  sampling, lens, lights), the tree and the work's size (tiles and samples, to
+                                  a factor of two) are the same */
     uint32_t use_graph;        /* 1: replay the batch from a captured CUDA graph */
     uint32_t block_threads;    /* 0: default or tuned (64, 128 or 256) */
     uint32_t blocks_per_sm;    /* 0: default or tuned */
@@ -357,6 +360,8 @@ typedef struct vgb_batch_options {
  * vgb_frame).  Frames' film planes are written as by vgb_render. */
 VGB_API vgb_status vgb_render_batch(vgb_context* ctx, const vgb_frame* frames, uint32_t nframes,
                                     const vgb_pt_options* opts, const vgb_batch_options* bopts);
+/* Launches that the autotuner has timed in this context so far. */
+VGB_API vgb_status vgb_batch_probes(vgb_context* ctx, uint64_t* probes);
 /* The launch shape chosen by the last autotuned batch (0s before the first one). */
 VGB_API vgb_status vgb_batch_tuning(vgb_context* ctx, uint32_t* block_threads, uint32_t* blocks_per_sm,
                                     uint32_t* tiles_per_grab);

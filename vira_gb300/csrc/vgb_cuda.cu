@@ -1832,7 +1832,14 @@ struct vgb_context {
     size_t cap_frames = 0;
     void* h_frames = nullptr;                // pinned staging of the table
     uint32_t tuned_threads = 0, tuned_bps = 0, tuned_grab = 0;
-    uint64_t tuned_key = 0;                  // the work they were tuned for
+    struct TunedFor {                        // the work they were tuned for
+        uint32_t bands, sums, bounces, adaptive, lens, lights, tiles, rays, tree;
+        bool operator==(const TunedFor& o) const {
+            return bands == o.bands && sums == o.sums && bounces == o.bounces && adaptive == o.adaptive && lens == o.lens &&
+                   lights == o.lights && tiles == o.tiles && rays == o.rays && tree == o.tree;
+        }
+    } tuned_for{};
+    uint64_t tuning_probes = 0;              // launches timed by the autotuner since the context was made
     uint32_t bvh_serial = 0;                 // trees built in this context
     cudaGraphExec_t graph_exec = nullptr;
     std::vector<unsigned char> graph_launch; // the BatchLaunch that graph_exec holds
@@ -4833,6 +4840,14 @@ static vgb_status launch_direct_frame(vgb_context* ctx, const FrameParams& fp, c
     return VGB_OK;
 }
 
+extern "C" VGB_API vgb_status vgb_batch_probes(vgb_context* ctx, uint64_t* probes) try {
+    if (!ctx || !probes) return VGB_ERR_INVALID_ARGUMENT;
+    *probes = ctx->tuning_probes;
+    return VGB_OK;
+} catch (...) {
+    return vgb::status_of_exception(ctx ? &ctx->err : nullptr);
+}
+
 extern "C" VGB_API vgb_status vgb_batch_tuning(vgb_context* ctx, uint32_t* threads, uint32_t* bps, uint32_t* grab) try {
     if (!ctx) return VGB_ERR_INVALID_ARGUMENT;
     if (threads) *threads = ctx->tuned_threads;
@@ -4908,14 +4923,21 @@ extern "C" VGB_API vgb_status vgb_render_batch(vgb_context* ctx, const vgb_frame
     if (threads != 64 && threads != 128 && threads != 256)
         return fail(ctx, VGB_ERR_INVALID_ARGUMENT, "render_batch: block_threads must be 64, 128 or 256");
     CK(cudaMemsetAsync(ctx->d_stats, 0, sizeof(uint64_t) * 8, ctx->stream));
-    // The shape tuned for this kernel (bands, lean or general, sums, bounces), this tree and this
-    // magnitude of work; a call that asks for tuning again with the same uses it as it is.
-    uint32_t mag = 0;
-    while ((bp.total_tiles >> mag) > 1u) ++mag;
-    const uint64_t tune_key = 1ull | ((uint64_t)ctx->nbands << 1) | ((uint64_t)bp.sums << 5) |
-                              ((uint64_t)(opts->bounces != 0) << 6) | ((uint64_t)(opts->adaptive_sampling != 0) << 7) |
-                              ((uint64_t)mag << 8) | ((uint64_t)ctx->bvh_serial << 16);
-    if (bo && bo->autotune && ctx->tuned_key != tune_key) {
+    // The shape tuned for this kernel (bands, sums, bounces, sampling, lens, lights), this tree and work of
+    // this size (tiles, and tiles times samples, by powers of two); a call that asks for tuning again with
+    // the same uses it as it is.
+    auto magnitude = [](uint64_t n) { uint32_t m = 0; while (n >>= 1) ++m; return m; };
+    vgb_context::TunedFor tune_for{ctx->nbands, bp.sums, opts->bounces, opts->adaptive_sampling != 0 ? 1u : 0u, 0, 0,
+                                   magnitude(total_tiles), 0, ctx->bvh_serial + 1};
+    uint64_t tile_samples = 0;
+    for (uint32_t f = 0; f < nframes; ++f) {
+        const vgb_frame& fr = frames[f];
+        tile_samples += (uint64_t)((fr.camera.width + 7) / 8) * ((fr.camera.height + 3) / 4) * fr.samples;
+        tune_for.lights = std::max(tune_for.lights, fr.nlights);
+        tune_for.lens |= (fr.camera.distortion ? 1u : 0u) | (fr.camera.depth_of_field ? 2u : 0u);
+    }
+    tune_for.rays = magnitude(tile_samples);
+    if (bo && bo->autotune && !(ctx->tuned_for == tune_for)) {
         // Autotuner: time candidate launch shapes on every 16th tile, keep the fastest.  Every
         // candidate fills the SMs (the launch clamps the blocks to what is resident): with the 24
         // shapes of 2-16 blocks per SM tried on every call, most of them duplicates or a fraction of
@@ -4934,14 +4956,15 @@ extern "C" VGB_API vgb_status vgb_render_batch(vgb_context* ctx, const vgb_frame
                 CK(cudaEventSynchronize(ctx->ev1));
                 float ms = 0.f;
                 cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
+                ctx->tuning_probes++;
                 if (ms < best) { best = ms; threads = ct; bps = 16; grab = cg; }
             }
-        ctx->tuned_threads = threads; ctx->tuned_bps = bps; ctx->tuned_grab = grab;
-        ctx->tuned_key = tune_key;
         CK(read_back(ctx));
         CK(cudaMemsetAsync(ctx->d_stats, 0, sizeof(uint64_t) * 8, ctx->stream));
         vgb_status es = check_device_error(ctx);
-        if (es != VGB_OK) return es;
+        if (es != VGB_OK) return es;   // probes that gave up say nothing of the shapes: nothing is kept
+        ctx->tuned_threads = threads; ctx->tuned_bps = bps; ctx->tuned_grab = grab;
+        ctx->tuned_for = tune_for;
     } else if (bo && bo->autotune) {
         threads = ctx->tuned_threads; bps = ctx->tuned_bps; grab = ctx->tuned_grab;
     }
