@@ -156,10 +156,6 @@ using namespace vgbd;
 #ifndef VGB_TRAV_REFILL
 #define VGB_TRAV_REFILL 8
 #endif
-// k_adjoint: blocks per SM, and blocks resident per SM (2 / 3 blocks of 256 threads, 4 blocks of 64 at
-// the same registers: within 2 % of each other on 4 views of 256^2 x 16 spp); k_adjoint_batch: 128-thread
-// blocks resident per SM (2 / 3 / 4 / 5 / 6 / 8 / 10 / 12: 5.6 / 4.7 / 4.4 / 4.25 / 4.1 / 4.0 / 4.1 / 4.2
-// ms for 12 asteroid views; the spills of 64 registers cost less than the idle issue slots).
 // k_raster_cover and k_raster_resolve: 64-thread blocks, blocks per SM as above, and k_raster_resolve's
 // resident blocks (64 registers).  Triangles and pixels cost unevenly, and 8 blocks of 256 threads per SM
 // left two thirds of the warp slots idle behind the slowest: 2.1M triangles at 1024^2, 8 bands 152 -> 126
@@ -173,18 +169,29 @@ using namespace vgbd;
 #ifndef VGB_RESOLVE_MINB
 #define VGB_RESOLVE_MINB 4
 #endif
+// k_adjoint: blocks per SM, and the register budget as resident blocks of 256 threads per SM.  At 3 (80
+// registers) one band on either layout and four on wide nodes are fastest; what more bands and the 8-wide
+// traversal spill there costs more than the warps gain.  1024^2 x 4 spp at 3 / 2 blocks, 0 and 2 bounces, ms:
+// wide, 1 band 1.20 / 1.30, 4.15 / 4.43; 4 bands 1.69 / 1.76, 5.71 / 5.81; 8 bands 2.76 / 2.77, 8.45 / 7.81;
+// 8-wide, 1 band 1.82 / 1.88, 7.27 / 7.17; 4 bands 2.33 / 2.22, 10.2 / 9.15; 8 bands 3.28 / 2.99, 14.9 / 12.2.
 #ifndef VGB_ADJOINT_GRID
 #define VGB_ADJOINT_GRID 64
 #endif
 #ifndef VGB_ADJOINT_MINB
-#define VGB_ADJOINT_MINB 3
+#define VGB_ADJOINT_MINB(NB, L) ((NB) == 1 || ((NB) == 4 && (L) == 4) ? 3 : 2)
 #endif
+// k_adjoint_batch: 128-thread blocks resident per SM (2 / 3 / 4 / 5 / 6 / 8 / 10 / 12: 5.6 / 4.7 / 4.4 / 4.25 /
+// 4.1 / 4.0 / 4.1 / 4.2 ms for 12 asteroid views; the spills of 64 registers cost less than the idle issue
+// slots).  The same for 1, 4 and 8 bands, both layouts, 0 and 2 bounces at 1024^2 x 4 spp (4 / 6 / 8 blocks
+// at 8 bands, 2 bounces: 19.8 / 17.0 / 15.1 ms wide, 28.5 / 26.7 / 24.1 8-wide); two views of 192^2, which do
+// not fill the GPU, would rather have 4 (8 bands: 2.66 / 2.93 / 3.02 ms).
 #ifndef VGB_ADJB_MINB
 #define VGB_ADJB_MINB 8
 #endif
-// k_trace_batch: resident blocks of 256 threads per SM for closest hits (wide nodes) and for occlusion
-// (binary nodes).  2M scattered rays over 2.1M triangles: closest 625 us left to the compiler, 596 / 598 /
-// 615 at 4 / 5 / 6; occlusion 354, 358 / 338 / 337 (30K rays: 55 us, 55 / 63 / 65; 51 throughout).
+// k_trace_batch: resident blocks of 256 threads per SM for closest hits and for occlusion on the binary nodes;
+// occlusion on 8-wide nodes, which spills at 5, has the first.  2M scattered rays over 2.1M triangles: closest
+// (wide nodes) 625 us left to the compiler, 596 / 598 / 615 at 4 / 5 / 6; occlusion 354, 358 / 338 / 337 (30K
+// rays: 55 us, 55 / 63 / 65; 51 throughout); 8-wide occlusion 434 us left to the compiler, 420 / 443 at 4 / 5.
 #ifndef VGB_RAYS_MINB
 #define VGB_RAYS_MINB 4
 #endif
@@ -1732,7 +1739,7 @@ __global__ void k_pixel_solid_angle(const __grid_constant__ vgb_camera cam, floa
 
 // ------------------------------------------------------------------ batch trace (TLAS::intersect seam)
 template <int L, bool ANY, bool COUNT>
-__global__ void __launch_bounds__(VGB_RAYS_BLOCK, (ANY ? VGB_RAYS_ANY_MINB : VGB_RAYS_MINB) * 256 / VGB_RAYS_BLOCK) k_trace_batch(const DevScene s, const float* org, const float* dir, const float* tmax,
+__global__ void __launch_bounds__(VGB_RAYS_BLOCK, (ANY && L != 8 ? VGB_RAYS_ANY_MINB : VGB_RAYS_MINB) * 256 / VGB_RAYS_BLOCK) k_trace_batch(const DevScene s, const float* org, const float* dir, const float* tmax,
                                                uint32_t n, uint32_t* tri, float* tout, float* bary,
                                                uint32_t* counters, uint64_t* stats) {
     uint32_t err = 0;
@@ -5330,7 +5337,7 @@ __device__ __forceinline__ void adj_scatter(const DevScene& s, uint32_t nb, bool
 // view of 256^2 pixels alone is a sixth of the threads the GPU holds.  4 views of 256^2 x 16 spp, 2
 // bounces: 14.9 -> 6.4 ms of backward pass against a thread per pixel.
 template <int NB, int L>
-__global__ void __launch_bounds__(VGB_ADJOINT_BLOCK, VGB_ADJOINT_MINB) k_adjoint(const DevScene s, const __grid_constant__ FrameParams fp,
+__global__ void __launch_bounds__(VGB_ADJOINT_BLOCK, VGB_ADJOINT_MINB(NB, L)) k_adjoint(const DevScene s, const __grid_constant__ FrameParams fp,
                                                  const float* __restrict__ dldi, const AdjOut out, uint32_t* errw,
                                                  uint64_t* stats) {
     const uint32_t nb = fp.nb;
