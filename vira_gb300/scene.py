@@ -222,7 +222,7 @@ class Camera:
         c.width, c.height = self.resolution
         c.origin[:] = (self.position - scene_origin).astype(f32).tolist()    # FP64 rebasing, then FP32
         c.rotation[:] = self.rotation.astype(f32).T.ravel().tolist()         # column major
-        c.kinv[:] = self._kinv_c() if kinv is None else np.asarray(kinv, f32).tolist()
+        c.kinv[:] = self._kinv_c() if kinv is None else np.asarray(kinv, f32)[:6].tolist()
         c.z_dir = float(self.z_dir)
         area = self.aperture_area()
         if isinstance(self.optical_efficiency, (int, float)):
@@ -232,15 +232,15 @@ class Camera:
             c.power_scale[:nbands] = (eff * area).astype(f32).tolist()
         if self.distortion is not None:
             c.distortion = int(self.distortion[0])
-            c.distortion_coeffs[:len(self.distortion[1])] = self.distortion[1].tolist()
+            c.distortion_coeffs[:len(self.distortion[1])] = [float(v) for v in self.distortion[1]]
         c.interpolate_directions = int(bool(self.interpolate_distortion_directions))
         c.depth_of_field = int(bool(self.depth_of_field))
         c.aperture_radius = float(self.aperture_radius())
         c.focal_length = float(self.focal_length)
         c.focus_distance = float(self.focus_distance)
         c.sensor_size[:] = [float(self.sensor_size[0]), float(self.sensor_size[1])]
-        c.velocity[:] = np.asarray(self.velocity, np.float64).astype(f32).tolist()
-        c.angular_rate[:] = np.asarray(self.angular_rate, np.float64).astype(f32).tolist()
+        c.velocity[:] = np.asarray(self.velocity[:3], np.float64).astype(f32).tolist()
+        c.angular_rate[:] = np.asarray(self.angular_rate[:3], np.float64).astype(f32).tolist()
         c.rot_origin[:] = (self.rotation @ np.asarray(scene_origin, np.float64)).astype(f32).tolist()
         return c
 
@@ -909,7 +909,7 @@ class Scene:
         out.position[:] = (np.asarray(position, np.float64) - self.origin).astype(np.float32).tolist()
         out.radius = float(light.radius)
         n = self.bands.size
-        out.radiance[:n] = np.asarray(light.radiance[:n], np.float32).tolist()
+        out.radiance[:n] = [float(x) for x in light.radiance[:n]]
 
     def pixel_solid_angle(self, camera: Camera, cam_c: capi.Camera):
         """Camera::initializePixelSolidAngle (camera.ipp:1622-1666) on the device, FP64, cached."""
