@@ -182,17 +182,16 @@ __device__ __forceinline__ void slab(const SlabRay& q, float lox, float hix, flo
     tf = fmin3(fmaxf(a0, a1), fmaxf(b0, b1), fminf(fmaxf(c0, c1), tfar)) * widen;
 }
 
-// Closest hit (any = false; ties in t go to the smaller id) or occlusion (any = true, any
-// hit with t <= tmax).  Box tests are conservative (make_slab).
-// One body for both kinds of ray; the templated wrapper below passes `any` as a constant.
+// Occlusion on the binary nodes: the first triangle met with t <= tmax.  vgb_trace_rays reports that
+// triangle, so its walk keeps this tree's order; every other ray walks the wide nodes below.  Box tests
+// are conservative (make_slab).
 template <bool COUNT>
-__device__ __forceinline__ void traverse_rt(const float4* __restrict__ nodes, const float4* __restrict__ tris,
-                                            const WRay& r, float tmax, const bool any, HitOut& h, uint32_t& err,
-                                            Counters& cnt, uint32_t cap) {
+__device__ __forceinline__ void occluded2(const float4* __restrict__ nodes, const float4* __restrict__ tris,
+                                          const WRay& r, float tmax, HitOut& h, uint32_t& err, Counters& cnt,
+                                          uint32_t cap) {
     int stack[kStackSize];
     int sp = 0;
     int node = 0;
-    float best = any ? tmax : __int_as_float(0x7f800000);
     h.t = __int_as_float(0x7f800000);
     h.id = VGB_NO_HIT;
     uint32_t iter = 0;
@@ -206,8 +205,8 @@ __device__ __forceinline__ void traverse_rt(const float4* __restrict__ nodes, co
             const float4 n3 = __ldg(&nodes[4 * node + 3]);
             if (COUNT) cnt.nodes++;
             float tn0, tf0, tn1, tf1;
-            slab(q, n0.x, n0.y, n0.z, n0.w, n2.x, n2.y, best, tn0, tf0);
-            slab(q, n1.x, n1.y, n1.z, n1.w, n2.z, n2.w, best, tn1, tf1);
+            slab(q, n0.x, n0.y, n0.z, n0.w, n2.x, n2.y, tmax, tn0, tf0);
+            slab(q, n1.x, n1.y, n1.z, n1.w, n2.z, n2.w, tmax, tn1, tf1);
             const bool h0 = tn0 <= tf0, h1 = tn1 <= tf1;
             const int ch0 = __float_as_int(n3.x), ch1 = __float_as_int(n3.y);
             if (h0 && h1) {
@@ -234,14 +233,10 @@ __device__ __forceinline__ void traverse_rt(const float4* __restrict__ nodes, co
             const float4 t2 = __ldg(&tris[3 * (start + k) + 2]);
             if (COUNT) cnt.tris++;
             float tt, U, V, W, det;
-            if (wt_test(r, ld3(t0), ld3(t1), ld3(t2), tt, U, V, W, det)) {
-                const uint32_t id = __float_as_uint(t0.w);
-                if (any) {
-                    if (tt <= tmax) { h.t = tt; h.id = id; return; }
-                } else if (tt < h.t || (tt == h.t && id < h.id)) {
-                    h.t = tt; h.id = id; h.U = U; h.V = V; h.W = W; h.det = det;
-                    best = tt;
-                }
+            if (wt_test(r, ld3(t0), ld3(t1), ld3(t2), tt, U, V, W, det) && tt <= tmax) {
+                h.t = tt;
+                h.id = __float_as_uint(t0.w);
+                return;
             }
         }
         if (sp == 0) return;
@@ -598,15 +593,16 @@ __device__ __forceinline__ void traverse8(const uint4* __restrict__ nodes, const
     traverse8_rt<COUNT>(nodes, tris, r, tmax, ANY, h, err, cnt, cap);
 }
 
-// Dispatch on the node layout (2: binary, 4: wide, 8: compressed 8-wide).  `cap`: traversal steps
+// Dispatch on the node layout (2: binary, occlusion only; 4: wide; 8: compressed 8-wide).  `cap`: traversal steps
 // per ray before the ray gives up and sets kErrIter.  UNIT: the ray's direction is normalised.
 template <int LAYOUT, bool ANY, bool COUNT, bool UNIT = true>
 __device__ __forceinline__ void traverse_any_layout(const uint4* __restrict__ nodes, const float4* __restrict__ tris,
                                                     const WRay& r, float tmax, HitOut& h, uint32_t& err, Counters& cnt,
                                                     uint32_t cap) {
+    static_assert(LAYOUT != 2 || ANY, "closest hits walk the wide nodes");
     if (LAYOUT == 8) traverse8<ANY, COUNT>(nodes, tris, r, tmax, h, err, cnt, cap);
     else if (LAYOUT == 4) traverse4_rt<COUNT, UNIT>(nodes, tris, r, tmax, ANY, h, err, cnt, cap);
-    else traverse_rt<COUNT>(reinterpret_cast<const float4*>(nodes), tris, r, tmax, ANY, h, err, cnt, cap);
+    else occluded2<COUNT>(reinterpret_cast<const float4*>(nodes), tris, r, tmax, h, err, cnt, cap);
 }
 
 }  // namespace vgbd
