@@ -36,16 +36,18 @@ import numpy as np
 ROOT = Path(__file__).resolve().parent
 
 # DRAM bytes (read + write) per launch of a kernel family from an ncu capture of the workload, by
-# (workload, layout); none is held for the present kernels.
-MEASURED_TRAFFIC = {}
+# (workload, layout): the mean over the launches of a render.
+MEASURED_TRAFFIC = {
+    ("path_traced_dem4097_tex4096_2048px_64spp_3b_rr2_8band", 2): {"k_front + k_trace + k_shadow": 564435016.0},
+}
 # ncu counters of k_front on the path-traced workload at scale 0.25 (1025^2 DEM, 512^2, 4 spp).
 MEASURED_TRACE_COUNTERS = {
     "case": "k_front, path_traced scale 0.25 (1025^2 DEM + craters, 512^2, 4 spp, 3 bounces)",
-    "issue_active_pct": 60.3,
-    "l1_throughput_pct": 56.47,
-    "threads_per_warp_inst": 23.06,
-    "long_scoreboard_stalls_per_issue": 3.69,
-    "no_instruction_stalls_per_issue": 1.69,
+    "issue_active_pct": 62.08,
+    "l1_throughput_pct": 58.44,
+    "threads_per_warp_inst": 23.07,
+    "long_scoreboard_stalls_per_issue": 3.64,
+    "no_instruction_stalls_per_issue": 1.10,
 }
 L2_PROBE_BYTES = 64 << 20
 sys.path.insert(0, str(ROOT))

@@ -212,8 +212,9 @@ typedef struct vgb_stats {
     uint32_t kernel_launches;  /* kernels launched by the last render */
     uint32_t device_error;     /* last device error word (0 = none) */
     float ms_last;             /* device time of the last render, or of the device phase of the last vgb_quipu_read_mesh (CUDA events) */
-    /* profiling mode only (vgb_set_profiling): device time and launches per kernel family:
-     * closest-hit traversal, shading, shadow traversal, film */
+    /* profiling mode only (vgb_set_profiling): device time and launches per kernel family: trace (closest-hit
+     * traversal; also the kernel that takes camera rays to their second hit, shading and shadow rays
+     * included, and the one launch of a large direct-lighting frame), shading, shadow traversal, film */
     float ms_trace, ms_shade, ms_shadow, ms_film;
     uint32_t launches_trace, launches_shade, launches_shadow, launches_film;
 } vgb_stats;
@@ -546,11 +547,11 @@ VGB_API vgb_status vgb_set_profiling(vgb_context* ctx, int enable);
  * larger one HBM.  The buffer is freed before return. */
 VGB_API vgb_status vgb_measure_l2_read(vgb_context* ctx, uint64_t bytes, uint32_t passes, uint32_t repeats,
                                        double* gbps);
-/* How vgb_render and vgb_render_noalloc traverse the binary BVH (no counterpart in the
+/* How vgb_render and vgb_render_noalloc traverse the folded nodes of layout 2 (no counterpart in the
  * reference; results do not depend on it).  persistent = 0 (default): one thread per ray in
- * grid-stride loops of many short blocks; persistent = 1: one resident wave of closest-hit and
+ * many short blocks; persistent = 1: one resident wave of closest-hit and
  * occlusion kernels whose warps hand queue rays to lanes as lanes finish, each ray advancing at
- * most `budget` inner-node visits between hand-outs, a hand-out happening once `refill` lanes of
+ * most `budget` node visits between hand-outs, a hand-out happening once `refill` lanes of
  * a warp are free (0: the defaults, 32 and 8). */
 VGB_API vgb_status vgb_set_wavefront_tuning(vgb_context* ctx, uint32_t persistent, uint32_t budget, uint32_t refill);
 /* Device memory that the context may keep as vgb_render's scratch, in bytes; 0 (the default) sets no
@@ -561,8 +562,9 @@ VGB_API vgb_status vgb_set_wavefront_tuning(vgb_context* ctx, uint32_t persisten
  * time, down to one; less than that needs fails with VGB_ERR_OUT_OF_MEMORY.  The planes are the same
  * whatever the limit.  Scratch above a new limit is given back at once. */
 VGB_API vgb_status vgb_set_scratch_limit(vgb_context* ctx, uint64_t bytes);
-/* Traversal steps (node visits) one ray may take before it gives up; 0 restores the default
- * of 2^22.  A ray past the limit stops, the call returns VGB_ERR_DEVICE_LIMIT with a message
+/* Traversal steps (visits of the nodes that its traversal walks, vgb_stats.bvh_nodes) one ray may take before
+ * it gives up; 0 restores the default of 2^22.  On folded nodes the limit is looked at where the ray goes on to
+ * its next subtree, so it may be passed by the tree's depth, at most 63.  A ray past the limit stops, the call returns VGB_ERR_DEVICE_LIMIT with a message
  * and the context stays usable.  The limit exists so that no kernel can run unbounded on a
  * corrupt tree; a small value exercises that path on a healthy scene.  No counterpart in the
  * reference (Embree has no such limit). */

@@ -88,7 +88,7 @@ using namespace vgbd;
 #define VGB_FRONT_MINB 8
 #endif
 // Grids of the wavefront kernels after k_front, in 256-thread blocks per SM: their queues hold the
-// few paths that hit a second time (8 / 20 / 60: 2.756 / 2.760 / 2.791 ms at 512^2 x 16 spp).
+// few paths that hit a second time (8 / 20 / 60: within 1.3 % of each other at 512^2 x 16 spp).
 #ifndef VGB_LATE_GRID
 #define VGB_LATE_GRID 20
 #endif
@@ -1459,14 +1459,16 @@ __global__ void __launch_bounds__(256) k_end_sample(DevState st, const __grid_co
 // Against starting the path with k_trace, k_shade, k_shadow and k_trace a sample at a time this moves
 // no ray, hit or shadow queue through memory for the camera rays (all of them) and the paths that
 // leave the terrain after one bounce (most), and a launch covers enough samples to fill the GPU
-// whatever the frame's size.  Device time against the wavefront alone: 301 x 203 x 16 spp 4.09 -> 0.75
-// ms, 512^2 x 16 spp 7.38 -> 2.76 ms, 2048^2 x 4 spp 13.15 -> 11.5 ms, 1024^2 direct 0.355 -> 0.331 ms.
-// Bound by instruction issue and fetch (56 % of the issue slots, 20 of 32 threads an instruction).
+// whatever the frame's size.  Device time of a frame against the wavefront kernels alone, both on wide
+// nodes: 301 x 203 x 16 spp 3.33 -> 0.66 ms, 512^2 x 16 spp 7.08 -> 2.42 ms, 2048^2 x 4 spp 12.8 -> 8.93 ms,
+// 96^2 x 1 spp without bounces 51 -> 33 us.  Bound by instruction issue (62 % of the slots, 23 of 32 threads
+// an instruction; 512^2 x 4 spp, 8 bands).
 template <int NB>
 __global__ void __launch_bounds__(VGB_FRONT_BLOCK, VGB_FRONT_MINB) k_front(const DevScene s, DevState st, const __grid_constant__ FrameParams fp,
                                                   uint32_t sample0, uint32_t nsamples) {
     // Band loops rolled, the bands in local memory (they wait there through each traversal anyway): the
-    // kernel is bound by instruction fetch as much as by issue.  2048^2 x 4 spp 8.96 -> 8.70 ms.
+    // kernel was bound by instruction fetch as much as by issue.  With sine and cosine, the lens and the
+    // texture wrap out of line 2048^2 x 4 spp 10.3 -> 10.0 ms.
     constexpr bool ROLL = NB > 1;
     constexpr int U = ROLL ? 1 : NB;
     const uint32_t nb = fp.nb;

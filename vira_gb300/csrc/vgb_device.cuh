@@ -349,8 +349,9 @@ __device__ __forceinline__ TravState trav_start(const WRay& r, float tmax, bool 
 // with t <= tmax).  The stack holds any walk of a tree that the build accepts (kWideLevels levels, three
 // pushes each), so pushes need no test; a ray over its step cap is stopped where it next takes a node
 // off the stack, which bounds it as well: a descent between two of those is as long as the tree is deep.
-// (Testing both at every node cost 1-2 %: 512^2 x 16 spp 2.36 against 2.32 ms.)  RESUME: stops after `budget` nodes; returns true when the ray is finished (h
-// holds its answer), false when the next call is to continue from ts.
+// (Testing both at every node cost 1-2 %: 512^2 x 16 spp 2.36 against 2.32 ms.)  RESUME: stops after
+// `budget` nodes; returns true when the ray is finished (h holds its answer), false when the next call is to
+// continue from ts.
 template <bool COUNT, bool RESUME, bool UNIT = true>
 __device__ __forceinline__ bool traverse4(const uint4* __restrict__ nodes, const float4* __restrict__ tris,
                                           const WRay& r, const WideRay& q, float tmax, const bool any, int* stack,
