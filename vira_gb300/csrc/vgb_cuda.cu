@@ -2788,8 +2788,7 @@ static vgb_status build_wide(vgb_context* ctx, bool& too_deep) {
     return VGB_OK;
 }
 
-VGB_API vgb_status vgb_bvh_build(vgb_context* ctx, const vgb_bvh_options* opts) try {
-    if (!ctx) return VGB_ERR_INVALID_ARGUMENT;
+static vgb_status build_bvh_once(vgb_context* ctx, const vgb_bvh_options* opts) {
     if (ctx->ntris == 0) return fail(ctx, VGB_ERR_NOT_READY, "bvh_build: no scene uploaded");
     uint32_t leaf = opts ? opts->max_leaf_size : 0, threads = opts ? opts->threads : 0;
     uint32_t layout = (opts && opts->layout) ? opts->layout : 2;
@@ -2875,12 +2874,21 @@ VGB_API vgb_status vgb_bvh_build(vgb_context* ctx, const vgb_bvh_options* opts) 
         if ((s = build_wide(ctx, deep)) != VGB_OK) return s;
         if (deep) {   // Morton order splits at most 95 times, whatever the triangles
             const vgb_bvh_options o{leaf, 1u, threads, 2u};
-            return vgb_bvh_build(ctx, &o);
+            return build_bvh_once(ctx, &o);
         }
     }
     ctx->bvh_ready = true;
     ctx->stats.tri_record_bytes = 48;
     return VGB_OK;
+}
+
+VGB_API vgb_status vgb_bvh_build(vgb_context* ctx, const vgb_bvh_options* opts) try {
+    if (!ctx) return VGB_ERR_INVALID_ARGUMENT;
+    const bool kept = ctx->d_nodes != nullptr;
+    const vgb_status s = build_bvh_once(ctx, opts);
+    if (s != VGB_ERR_OUT_OF_MEMORY || !kept) return s;
+    free_bvh(ctx);   // once more without the buffers of the tree before
+    return build_bvh_once(ctx, opts);
 } catch (...) {
     return vgb::status_of_exception(ctx ? &ctx->err : nullptr);
 }
